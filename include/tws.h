@@ -191,9 +191,11 @@ TWS_API int tws_variant_info(int variant, int* steps_per_launch, int* tile_x, in
 /* The kind of kernel variant i, or TWS_ERR_INVALID past the last one:
  * TWS_VARIANT_TILE (TMA-staged tiles: tile_x x tile_y output cells per CTA),
  * TWS_VARIANT_STREAM (register streaming, one step: tile_x columns per warp
- * walking tile_y rows) or TWS_VARIANT_SWEEP (a warp sweeps a strip of tile_x
- * output columns down a band of tile_y rows, the steps' time levels in
- * registers).  Only the tile variants wait on barriers that
+ * walking tile_y rows) or TWS_VARIANT_SWEEP (a warp sweeps a strip of columns
+ * down a band of tile_y rows, the steps' time levels on chip; without a tail
+ * the bands are taller where every resident warp still gets one, and idle warps
+ * take over rows of others' bands.  tile_x = 64 - 4K names the column unit; a
+ * strip is two of them side by side, 128 columns less their common halo).  Only the tile variants wait on barriers that
  * tws_set_wait_limit bounds. */
 #define TWS_VARIANT_TILE 0
 #define TWS_VARIANT_STREAM 1

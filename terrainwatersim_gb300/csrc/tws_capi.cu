@@ -58,6 +58,7 @@ struct tws_grid {
   double vol_host[1] = {0.0};
   int* err = nullptr;     // device error word
   int* queue = nullptr;   // the sweep kernel's work queue (two ints, zero between launches)
+  unsigned long long* ranges = nullptr;  // and its warps' unclaimed rows (empty between launches)
   int err_host[1] = {0};
   CUtensorMap* desc = nullptr;  // device copies of the maps, 5 per variant (batched kernel)
   long long wait_cycles = kDefaultWaitCycles;  // SM clocks a tile-load wait may take
@@ -137,6 +138,9 @@ float pick_flux_scale(float d_max, float c) {
   const int e = (int)std::floor(std::log2(8192.0 / fmax));
   return std::ldexp(1.0f, std::max(-24, std::min(24, e)));
 }
+
+// The error word, the sweep kernel's queue (at byte 16) and its ranges (at 64).
+constexpr size_t kSweepScratch = 64 + sizeof(unsigned long long) * kSweepMaxWarps;
 
 VariantMaps* maps_for(tws_grid* g, int variant, std::string* why) {
   if ((int)g->maps.size() < step_variant_count()) g->maps.resize(step_variant_count());
@@ -231,8 +235,10 @@ StepArgs make_step_args(const tws_grid* g) {
   a.v_out = g->v;
   a.flux_scale = g->flux_scale;
   a.flux_inv_scale = 1.0f / g->flux_scale;
+  a.neg_zero = -0.0f;
   a.err = g->err;
   a.queue = g->queue;
+  a.ranges = g->ranges;
   a.wait_cycles = g->wait_cycles;
   a.drop_loads = g->drop_loads;
   return a;
@@ -391,7 +397,7 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   const size_t ob = take(n * 4), od0 = take(n * 4), od1 = take(n * 4), of0 = take(n * fb),
                of1 = take(n * fb), ov = take(n * 8),
                op = take(sizeof(double) * volume_partials_needed()), oo = take(sizeof(double)),
-               oe = take(64), ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
+               oe = take(kSweepScratch), ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
   cudaMemPool_t pool = library_pool(g->device);
   if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&g->slab), off, pool, g->stream) !=
                    cudaSuccess) {
@@ -408,6 +414,7 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   g->vol_out = reinterpret_cast<double*>(g->slab + oo);
   g->err = reinterpret_cast<int*>(g->slab + oe);
   g->queue = reinterpret_cast<int*>(g->slab + oe + 16);
+  g->ranges = reinterpret_cast<unsigned long long*>(g->slab + oe + 64);
   g->desc = reinterpret_cast<CUtensorMap*>(g->slab + ot);
   // Zero everything, padding included (the F16 flux map reads the padding
   // cell of odd-width rows and relies on it staying zero).
@@ -417,7 +424,7 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   cudaMemsetAsync(g->f[0], 0, n * fb, g->stream);
   cudaMemsetAsync(g->f[1], 0, n * fb, g->stream);
   cudaMemsetAsync(g->v, 0, n * 8, g->stream);
-  cudaMemsetAsync(g->err, 0, 64, g->stream);  // the error word and the sweep queue
+  cudaMemsetAsync(g->err, 0, kSweepScratch, g->stream);  // error word, sweep queue and ranges
   if (cudaStreamSynchronize(g->stream) != cudaSuccess) return bail(TWS_ERR_CUDA);
   *out = g;
   return TWS_OK;

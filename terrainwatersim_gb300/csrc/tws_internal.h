@@ -34,11 +34,15 @@ struct StepArgs {
   float2* v_out;
   float flux_scale;      // F16 storage: stored = f * flux_scale
   float flux_inv_scale;  // F16 storage: f = stored * flux_inv_scale
+  float neg_zero;        // -0.0f, as data: a product formed as a * b + (-0) keeps its own
+                         // rounding whatever the assembler does with a sum it feeds
   int* err;              // device error word (bounded-wait time-outs)
   long long wait_cycles; // bounded waits give up after this many SM clocks
   int drop_loads;        // test hook: tile loads arm their barrier but issue no copy
   int* queue;            // the sweep kernel's work queue: next unit, warps done (zero
                          // between launches; the last warp of a launch resets it)
+  unsigned long long* ranges;  // the sweep kernel's unclaimed rows, one word per resident
+                         // warp (empty between launches)
 };
 
 // Kernel variants (temporal block depth K x tile).
@@ -54,7 +58,6 @@ struct StepVariant {
   int fw, fh; // flux box
   int sw;     // F16 staging width in cells (whole pairs)
   int uni;    // unified layout: the flux box is the b/d box
-  int ring;   // kKindSweep: rows in each lane's load ring
   int ry_tail; // kKindSweep: rows of the short bands that end the work queue (0: none)
   size_t smem;
 };
@@ -121,15 +124,17 @@ int step_variant_large_grid(int flux_storage, int W, int H);
 cudaError_t launch_step(int variant, int flux_storage, const CUtensorMap* tm_b,
                         const CUtensorMap* tm_d, const CUtensorMap* tm_f, const float* b,
                         const float* d, const void* f, const StepArgs& a, cudaStream_t s);
-// tws_sweep.cu: K = 2..4 steps per launch, `rows` rows per warp band (the
-// last bands `tail_rows` rows when it is above 0), a ring of `ring` rows per
-// lane (4)
-cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int ring, int flux_storage,
-                              const float* b,
+// tws_sweep.cu: K = 2..4 steps per launch, bands of `rows` rows (the last bands
+// `tail_rows` rows when it is above 0; with none, taller where every resident
+// warp still gets a band)
+cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, const float* b,
                               const float* d, const void* f, const StepArgs& a, cudaStream_t s);
 constexpr int kSweepCtaThreads = 128;  // four warps, each its own sweep
-size_t sweep_smem_bytes(int k, int flux_storage, int ring);
-int sweep_valid_columns(int k);
+constexpr int kSweepMaxWarps = 4096;   // warps of a sweep launch (words of StepArgs::ranges)
+size_t sweep_smem_bytes(int k, int flux_storage);
+// The column unit that the variant table names a sweep by: 64 columns less their
+// halo.  A warp sweeps two such halves side by side (128 columns).
+constexpr int sweep_column_unit(int k) { return 64 - 4 * k; }
 // tws_stream.cu
 cudaError_t launch_stream_step(int ry, int flux_storage, const float* b, const float* d,
                                const void* f, const StepArgs& a, cudaStream_t s);

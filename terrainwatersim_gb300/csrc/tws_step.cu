@@ -898,39 +898,32 @@ struct VariantTable {
     add<4, 32, 32, 1, true>();  // 20
     add<4, 64, 16, 1, true>();  // 21
     add<3, 64, 32, 1, true>();  // 22
-    // row sweeps: 64-column warp strips, K time levels on chip.  4096^2 FP32
-    // (Gcell-steps/s): K = 3 with 32-row bands 211.9, 40 211.6, 48 205.2, 64
-    // 184.4; K = 2 171-173; K = 4 173 with 64-row bands.  A ring of 4 rows is
-    // 0.3-1.5% faster than 3, one of 8 no faster than 4.
-    add_sweep(2, 32, 4);   // 23
-    add_sweep(2, 48, 4);   // 24
-    add_sweep(3, 32, 4);   // 25
-    add_sweep(3, 40, 4);   // 26  the default for large FP32 grids
-    add_sweep(3, 48, 4);   // 27
-    add_sweep(3, 64, 4);   // 28
-    add_sweep(4, 64, 4);   // 29
+    // row sweeps: 128-column warp strips, K time levels on chip, the rows
+    // of a band.  4096^2 FP32 (Gcell-steps/s): K = 3 256, K = 2 200, K = 4 196.
+    add_sweep(2, 32);  // 23
+    add_sweep(2, 48);  // 24
+    add_sweep(3, 32);  // 25
+    add_sweep(3, 40);  // 26  the default for large FP32 grids
+    add_sweep(3, 48);  // 27
+    add_sweep(3, 64);  // 28
+    add_sweep(4, 64);  // 29
     // Taller bands, the last ones short (the tail: about one short unit per
-    // resident warp ends the work queue).  Tall bands recompute fewer halo
-    // rows per output row, and the tail keeps the launch's end short.
-    // K = 3 (Gcell-steps/s, FP32 / FP16 flux): 6144^2 80/32 234.5 / 219.4;
-    // 8192^2 192/48 253.1 / 237.6; 16384^2 128/48 272.0 / 268.8, 192/48
-    // 276.8 / 275.4, 256/64 272.6 / 275.3 (64 rows: 258.8 / 251.4).
-    add_sweep(3, 80, 4, 32);   // 30
-    add_sweep(3, 128, 4, 48);  // 31
-    add_sweep(3, 192, 4, 48);  // 32
-    add_sweep(3, 256, 4, 64);  // 33
+    // resident warp ends the work queue): 2-5% on 16384^2 over uniform bands.
+    add_sweep(3, 80, 32);   // 30
+    add_sweep(3, 128, 48);  // 31
+    add_sweep(3, 192, 48);  // 32
+    add_sweep(3, 256, 64);  // 33
   }
-  void add_sweep(int k, int rows, int ring, int tail_rows = 0) {
+  void add_sweep(int k, int rows, int tail_rows = 0) {
     VariantEntry s{};
     s.v.ry_tail = tail_rows;
     s.v.k = k;
-    s.v.tx = sweep_valid_columns(k);
+    s.v.tx = sweep_column_unit(k);
     s.v.ty = rows;
     s.v.stages = 1;
     s.v.kind = kKindSweep;
     s.v.ry = rows;
-    s.v.ring = ring;
-    s.v.smem = sweep_smem_bytes(k, TWS_FLUX_F32, ring);
+    s.v.smem = sweep_smem_bytes(k, TWS_FLUX_F32);
     e[n] = s;
     if (n < kMax) ++n;
   }
@@ -981,13 +974,12 @@ int step_variant_count() { return table().n; }
 const StepVariant& step_variant(int i) { return table().e[i].v; }
 
 int step_variant_large_grid(int flux_storage, int W, int H) {
-  // The three-step row sweep: FP32 flux from kLargeGridCells on (4096^2:
-  // 40-row bands, 202.8 Gcell-steps/s against 193.4 for the two-step tiles),
-  // FP16 flux from kLargeF16Cells on (6144^2: 219.4 against 209.0 for the
-  // FP16 tiles; below it the tiles are as fast or faster: 4096^2 203.7
-  // against 184.9).  The band height is the tallest rung of a
-  // ladder that leaves at least 2.5 units per resident warp (four CTAs of four
-  // warps per SM), measured on 4096^2 to 16384^2.
+  // The three-step row sweep: FP32 flux from kLargeGridCells on (4096^2: 256
+  // Gcell-steps/s against 192 for the two-step tiles), FP16 flux from
+  // kLargeF16Cells on.  The band height is the tallest rung of a ladder that
+  // leaves at least 2.5 column-unit bands per resident warp of a 16-warp SM
+  // (8192^2: 310 with 192/48 rows, 305 with uniform bands of 64 to 192;
+  // 16384^2: 337 with 256/64, 320 uniform).
   const long long cells = (long long)W * H;
   if (cells < kLargeGridCells) return -1;
   if (flux_storage != TWS_FLUX_F32 && cells < kLargeF16Cells) return -1;
@@ -1000,7 +992,7 @@ int step_variant_large_grid(int flux_storage, int W, int H) {
                : 1;
   }();
   const double warps = (double)sms * 4 * (kSweepCtaThreads / 32);
-  const long long strips = (W + sweep_valid_columns(3) - 1) / sweep_valid_columns(3);
+  const long long strips = (W + sweep_column_unit(3) - 1) / sweep_column_unit(3);
   int pick = -1;
   for (int r = 0; r < (int)(sizeof(kLadder) / sizeof(kLadder[0])); ++r) {
     const long long units = strips * ((H + kLadder[r][0] - 1) / kLadder[r][0]);
@@ -1094,7 +1086,7 @@ cudaError_t launch_step(int variant, int flux_storage, const CUtensorMap* tm_b,
   VariantEntry& e = t.e[variant];
   if (e.v.kind == kKindStream) return launch_stream_step(e.v.ry, fs, b, d, f, a, s);
   if (e.v.kind == kKindSweep)
-    return launch_sweep_step(e.v.k, e.v.ry, e.v.ry_tail, e.v.ring, fs, b, d, f, a, s);
+    return launch_sweep_step(e.v.k, e.v.ry, e.v.ry_tail, fs, b, d, f, a, s);
   if (!tm_b || !tm_d || !tm_f) return cudaErrorInvalidValue;
   const void* fn = e.fn[fs];
   const size_t smem = e.smem[fs];

@@ -2,41 +2,55 @@
 //
 // Same arithmetic as the tiled kernels (flowUpdate.comp:34-62 then
 // flowApply.comp:32-52, K steps per launch, bit-identical to the FP32
-// transcription of the shaders), organised so that no halo is recomputed in y:
+// transcription of the shaders), organised so that no halo is recomputed in y
+// within a band:
 //
-// * A warp owns a strip of 64 columns (two per lane) and sweeps it down a
-//   band of R rows; the warps are persistent and take (strip, band) units
-//   from a per-grid queue, border units first, short bands last.  Each lane
-//   keeps, per time level s = 0..K-1, a rolling window of the rows that level
-//   needs: surface heights h of three rows, depths and terrain of two rows in
-//   registers, the new outflows of two rows in shared memory (the registers
-//   they would take cost a CTA per SM).
-//   Row by row, level s computes the outflow of one row and the depth of the
-//   row above, which is the input row of level s + 1 two rows further up; the
-//   last level writes its depth, flux and flow map.  The y neighbours come
-//   from the window, the x neighbours from the lane itself or its neighbour
-//   lanes (warp shuffles).  Values of the two outermost columns of the strip
-//   go stale one more column per phase, so a strip yields 64 - 4K output
-//   columns; neighbouring strips overlap by 4K columns (their loads are L2
-//   hits).  A band also loads 2K rows above and below it, whose results are
-//   not written.
-// * The two columns of a lane are one packed f32x2 operand
-//   (add/sub/mul.rn.f32x2): each lane of it is the IEEE round-to-nearest
-//   result of its own operands.  A packed product never feeds a packed sum
-//   (the assembler would contract the pair into a fused multiply-add); those
-//   sums are scalar.
-// * Loads: each lane copies its own two cells of a row (b, d, the flux
-//   records) into a private ring of P rows in shared memory with cp.async,
-//   P - 1 rows ahead of the row it computes.  Cells off the grid are
+// * A warp owns a strip of 128 columns, four per lane, and sweeps it down a
+//   band of rows.  Row by row, time level s = 0..K-1 computes the outflow of
+//   one row and the depth of the row above, which is the input row of level
+//   s + 1 two rows further up; the last level writes its depth, flux and flow
+//   map.  The y neighbours come from what the level keeps of its previous
+//   rows, the x neighbours from the lane itself or its neighbour lanes (warp
+//   shuffles).  Values of the outermost columns of the strip go stale one
+//   more column per phase, so a strip yields 112 (K = 3, 4) or 120 (K = 2)
+//   output columns; neighbouring strips overlap by the rest (their loads are
+//   mostly L2 hits).  A band also loads 2K rows above and below it, whose
+//   results are not written.
+// * What bounds it: instruction issue, and on the largest grids HBM.  Four
+//   cells a lane halve the shuffles, branches and address arithmetic per cell
+//   against two, and the strip overlap falls from 23% to 14%.  What a level
+//   keeps between rows is split so that three CTAs of four warps fit an SM
+//   (168 registers a thread, 18 KB of shared memory a warp at K = 3): depths
+//   and outflows that are read once, two rows later, wait in shared memory
+//   (which also saves the moves that shift a register window); the slope
+//   term of the last row pair, the x inflow and the outflow sum stay in
+//   registers.  The loop over rows is not unrolled: two rows per trip double
+//   the code and run 15-30% slower (instruction fetch).
+// * Neighbouring cells share the slope term ka * (h - h_n) of their common
+//   edge up to its sign, so each is computed once.
+// * The columns of a lane are two packed f32x2 operands: each half is the
+//   IEEE round-to-nearest result of its own operands.  A packed product that
+//   feeds a packed sum is formed as a fused multiply-add of -0 (prod2), which
+//   has the product's own bits and which the assembler cannot contract
+//   further.
+// * Loads: cp.async into shared memory, one row ahead of the row computed
+//   (12 warps of 3 KB in flight cover the latency).  Cells off the grid are
 //   zero-filled by the copy itself (the shaders' out-of-range image loads
-//   read zero).  A lane reads back only what it copied, so no barrier is
-//   needed; cp.async.wait_group is the hardware's wait, and a slot is
-//   refilled only in the iteration after the one that read it into
-//   registers and used those values.
+//   read zero).  cp.async.wait_group and a warp barrier hand a row over.
+// * The warps are persistent and take (strip, band) units from a per-grid
+//   queue, border units first.  A warp that finds the queue empty takes over
+//   half of the rows that another has not begun (range_pack below), so units
+//   under rain, at the border or on shores, which take longer, do not hold
+//   the launch up.
 //
 // HBM traffic per launch: the state once in, once out (52 B per cell for FP32
-// flux, 36 B for FP16), plus the re-read of the strip and band overlaps,
-// which L2 serves when neighbouring strips run together.
+// flux, 36 B for FP16), plus what L2 does not catch of the overlaps.
+//
+// Measured (CUDA events, Gcell-steps/s on moving water with a rain disk, K = 3;
+// in brackets the two-columns-a-lane kernel with static bands that this
+// replaced): 4096^2 256 (209), 8192^2 311 (250), 16384^2 337 (260), FP16 flux
+// 312 (253).  16384^2 at 337 moves 5.8 TB/s of compulsory bytes, 0.86 of the
+// copy rate.
 
 #include <algorithm>
 #include <map>
@@ -50,7 +64,10 @@ namespace {
 
 constexpr int kSweepThreads = kSweepCtaThreads;
 constexpr int kSweepWarps = kSweepThreads / 32;
-constexpr int kSweepCols = 64;  // columns a warp loads
+constexpr int kSweepCols = 128;  // columns a warp loads: four per lane
+// columns at either end of a strip that are not written: the 2K that go stale,
+// in whole lanes
+__host__ __device__ constexpr int kSweepHaloX(int k) { return (2 * k + 3) / 4 * 4; }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -72,121 +89,275 @@ __device__ __forceinline__ void copy_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// The four outflow channels (+x, -x, +y, -y) of a lane's two cells: .x of
-// each float2 is the lane's first column, .y its second.
-struct Flux2 {
-  float2 x, y, z, w;
-};
-__device__ __forceinline__ Flux2 zero_flux() {
-  const float2 z = make_float2(0.0f, 0.0f);
-  return Flux2{z, z, z, z};
+// A lane's two cells as one packed f32x2 operand, kept in a 64-bit register (its
+// low half is the lane's first column): values that stay packed from one row to
+// the next then cost no moves to line their halves up.
+typedef unsigned long long pair_t;
+__device__ __forceinline__ pair_t pk(float x, float y) {
+  pair_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 un(pair_t p) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ pair_t add2(pair_t a, pair_t b) {
+  pair_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ pair_t sub2(pair_t a, pair_t b) {
+  pair_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// a * b rounded, with -0 added: the product's own bits (x + -0 = x for every x,
+// -0 included), as a fused multiply-add that no later sum can be contracted
+// with.  `nz` must reach the kernel as data (StepArgs::neg_zero).
+__device__ __forceinline__ pair_t prod2(pair_t a, pair_t b, pair_t nz) {
+  pair_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+  return r;
+}
+__device__ __forceinline__ pair_t max0p(pair_t v) {
+  const float2 f = un(v);
+  return pk(max0_fast(f.x), max0_fast(f.y));
 }
 
-__device__ __forceinline__ float2 max0x2(float2 v) {
-  return make_float2(max0_fast(v.x), max0_fast(v.y));
+// d / t per half, rounded to nearest, for t up to kDivMaxT and d in
+// [kDivMinD, t): nothing on the way then overflows or leaves the normal range.
+// Markstein's division (IBM J. Res. Dev. 34, 1990): a reciprocal refined to
+// its correct rounding with one Newton step in fused arithmetic, a quotient
+// within an ulp, and the exact remainder's correction.  Against the
+// correctly rounded quotient: no difference in 1e11 random and structured
+// pairs of that range, nor in the pairs closest to a rounding boundary.
+// `nt` is -t.
+constexpr float kDivMinD = 0x1p-100f, kDivMaxT = 0x1p20f;
+__device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
+  pair_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
 }
-// p + q per column, with p and q packed products: scalar sums (never fadd2
-// of an fmul2 result, see the file comment)
-__device__ __forceinline__ float2 sum_products(float2 p, float2 q) {
-  return make_float2(fadd(p.x, q.x), fadd(p.y, q.y));
+__device__ __forceinline__ pair_t div2(pair_t d, pair_t t, pair_t nt) {
+  const float2 tv = un(t);
+  float y0, y1;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(tv.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(tv.y));
+  pair_t y = pk(y0, y1);
+  y = fma2(fma2(nt, y, pk(1.0f, 1.0f)), y, y);
+  pair_t q;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(d), "l"(y));
+  return fma2(fma2(nt, q, d), y, q);
 }
+
+// A lane's four cells: columns 0, 1 and 2, 3.
+struct Quad {
+  pair_t p[2];
+};
+#define TWS_QUAD_OP(name, op)                                     \
+  __device__ __forceinline__ Quad name(const Quad& a, const Quad& b) { \
+    return Quad{{op(a.p[0], b.p[0]), op(a.p[1], b.p[1])}};          \
+  }
+TWS_QUAD_OP(add4, add2)
+TWS_QUAD_OP(sub4, sub2)
+#undef TWS_QUAD_OP
+__device__ __forceinline__ Quad prod4(const Quad& a, pair_t b, pair_t nz) {
+  return Quad{{prod2(a.p[0], b, nz), prod2(a.p[1], b, nz)}};
+}
+__device__ __forceinline__ Quad prod4(const Quad& a, const Quad& b, pair_t nz) {
+  return Quad{{prod2(a.p[0], b.p[0], nz), prod2(a.p[1], b.p[1], nz)}};
+}
+__device__ __forceinline__ Quad max0q(const Quad& v) {
+  return Quad{{max0p(v.p[0]), max0p(v.p[1])}};
+}
+__device__ __forceinline__ float4 un4(const Quad& v) {
+  const float2 l = un(v.p[0]), h = un(v.p[1]);
+  return make_float4(l.x, l.y, h.x, h.y);
+}
+__device__ __forceinline__ Quad pk4(float x, float y, float z, float w) {
+  return Quad{{pk(x, y), pk(z, w)}};
+}
+__device__ __forceinline__ Quad load_quad(const unsigned char* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return Quad{{v.x, v.y}};
+}
+__device__ __forceinline__ void store_quad(unsigned char* p, const Quad& v) {
+  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.p[0], v.p[1]);
+}
+// One 32-byte store (whole sectors; the address is a multiple of 32).
+__device__ __forceinline__ void store32(void* p, float a, float b, float c, float d, float e,
+                                        float f, float g, float h) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b),
+               "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h)
+               : "memory");
+}
+
+// The four outflow channels (+x, -x, +y, -y) of a lane's four cells.
+struct Flux4 {
+  Quad x, y, z, w;
+};
 
 // Shared memory of one warp, in bytes.
-constexpr int sweep_row_bytes(bool f16) { return 512 + (f16 ? 512 : 1024); }
-constexpr int kSweepSlotBytes = 1024;
-constexpr int sweep_warp_bytes(int k, bool f16, int ring) {
-  return sweep_row_bytes(f16) * ring + k * 2 * kSweepSlotBytes;
+constexpr int kSweepRow = kSweepCols * 4;  // one float per column
+constexpr int sweep_flux_row_bytes(bool f16) { return kSweepCols * (f16 ? 8 : 16); }
+constexpr int kSweepSlotBytes = kSweepCols * 16;
+// rows of the terrain ring: the row in flight, the current one and those the
+// deeper levels still form h from (row r - 2(K - 1)): 2K, in a power of two
+constexpr int sweep_b_rows(int k) { return k <= 2 ? 4 : 8; }
+constexpr int kSweepDRows = 4;  // depth ring: the row in flight, rows r, r - 1 and r - 2
+constexpr int sweep_warp_bytes(int k, bool f16) {
+  return kSweepRow * (sweep_b_rows(k) + kSweepDRows + 2 * (k - 1)) + sweep_flux_row_bytes(f16) +
+         (k - 1) * 2 * kSweepSlotBytes;
 }
 
-template <int K, bool F16, int P>
+template <int K, bool F16>
 struct SweepRing {
-  // one row of a lane's ring: b and d of its two cells, then the flux records
-  // (FP32: the first cells of all lanes, then the second cells, so that a
-  // warp's 16-byte reads are conflict-free; FP16: both cells' 8 halves)
-  static constexpr int B = 0;    // 64 floats
-  static constexpr int D = 256;  // 64 floats
-  static constexpr int F = 512;  // FP32: 2 x 32 float4; FP16: 32 x 16 bytes
-  static constexpr int ROW = sweep_row_bytes(F16);
-  static constexpr int RING = ROW * P;  // P rows: P - 1 in flight
-  // The new outflows of each level's two previous rows, one 1 KB slot per
-  // row (the row computed in an iteration takes the slot of the older one
-  // once it has been read): each lane's (+x, -x) pairs at 16 * lane, its
-  // (+y, -y) pairs at 512 + 16 * lane.
+  static constexpr int PB = sweep_b_rows(K);
+  static constexpr int B = 0;
+  static constexpr int D = B + kSweepRow * PB;
+  // depths of the two previous input rows of levels 1 .. K - 1
+  static constexpr int DS = D + kSweepRow * kSweepDRows;
+  static constexpr int F = DS + kSweepRow * 2 * (K - 1);
+  // The new outflows of each level's two previous rows (all levels but the
+  // last), one slot per row (the row computed in an iteration takes the slot
+  // of the older one once it has been read): four channel planes.
+  static constexpr int N = F + sweep_flux_row_bytes(F16);
   static constexpr int NSLOT = kSweepSlotBytes;
-  static constexpr int WARP = sweep_warp_bytes(K, F16, P);
+  static constexpr int WARP = sweep_warp_bytes(K, F16);
+  static_assert(WARP == N + (K - 1) * 2 * NSLOT && PB >= 2 * K, "ring sizes");
 };
 
-template <int K, bool F16, bool INTERIOR, int P>
+// The rows of a warp's unit that nobody has claimed yet, one word per resident
+// warp: [cur, end) of strip `strip`.  The owner claims kSweepClaim rows at a
+// time from the front (one atomic add); a warp that finds the queue empty takes
+// the back half of another's range (one compare-and-swap).  Equal words mean
+// equal unclaimed rows, so a swap that succeeds is right whatever happened in
+// between.  Nothing waits on anything.
+constexpr int kSweepClaim = 8;     // rows of one claim
+constexpr int kSweepStealTries = 6;
+constexpr int kSweepMinSteal = 8; // unclaimed rows worth halving: a new unit computes
+                                   // about six rows' worth of halo
+__device__ __forceinline__ unsigned long long range_pack(int strip, int cur, int end) {
+  return (unsigned long long)(unsigned)strip << 42 | (unsigned long long)(unsigned)end << 21 |
+         (unsigned long long)(unsigned)cur;
+}
+__device__ __forceinline__ int range_cur(unsigned long long w) { return (int)(w & 0x1fffff); }
+__device__ __forceinline__ int range_end(unsigned long long w) { return (int)(w >> 21 & 0x1fffff); }
+__device__ __forceinline__ int range_strip(unsigned long long w) { return (int)(w >> 42); }
+
+template <int K, bool F16, bool INTERIOR>
 __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __restrict__ gb,
                                            const float* __restrict__ gd,
                                            const void* __restrict__ gf,
                                            float* __restrict__ d_out, void* __restrict__ f_out,
                                            float2* __restrict__ v_out, unsigned char* ring,
-                                           int xs, int y0, int R, uint32_t mask) {
-  using RG = SweepRing<K, F16, P>;
+                                           int xs, int y0, int R, uint32_t mask,
+                                           unsigned long long* word) {
+  using RG = SweepRing<K, F16>;
   constexpr int HALO = 2 * K;
   const int lane = threadIdx.x & 31;
   const int W = a.W, H = a.H;
   const size_t pitch = (size_t)a.pitch;
-  const float2 kf2 = make_float2(a.kf, a.kf), ka2 = make_float2(a.ka, a.ka);
-  const float2 cc2 = make_float2(a.c, a.c);
-  const float fscale = a.flux_scale, finv = a.flux_inv_scale;
-  const float2 fscale2 = make_float2(fscale, fscale), finv2 = make_float2(finv, finv);
+  const pair_t kf2 = pk(a.kf, a.kf), ka2 = pk(a.ka, a.ka), cc2 = pk(a.c, a.c);
+  const pair_t ncc2 = pk(-a.c, -a.c), nz2 = pk(a.neg_zero, a.neg_zero);
+  const float2 fscale2 = make_float2(a.flux_scale, a.flux_scale);
+  const float2 finv2 = make_float2(a.flux_inv_scale, a.flux_inv_scale);
   const bool closed = a.closed != 0;
 
-  // this lane's columns
-  const int gx0 = xs + 2 * lane, gx1 = gx0 + 1;
-  const bool in0 = INTERIOR || (gx0 >= 0 && gx0 < W);
-  const bool in1 = INTERIOR || (gx1 >= 0 && gx1 < W);
-  const bool out_lane = lane >= K && lane < 32 - K;  // columns HALO .. 63 - HALO
+  // this lane's columns gx .. gx + 3 (xs is a multiple of 4); `cols` of them
+  // are on the grid, all on one side
+  const int gx = xs + 4 * lane;
+  const int cols = INTERIOR ? 4 : (gx < 0 ? 0 : min(4, max(0, W - gx)));
+  const bool out_lane =
+      lane >= kSweepHaloX(K) / 4 && lane < 32 - kSweepHaloX(K) / 4 && (INTERIOR || cols > 0);
   const int first_row = y0 - HALO;
-  const int rows = R + 2 * HALO;  // rows loaded
 
-  // ---- the copies of row r into ring slot `slot`
-  auto issue_row = [&](int r, int slot) {
-    unsigned char* st = ring + slot * RG::ROW;
-    const bool row_in = INTERIOR || (r >= 0 && r < H);
-    const int nb = (row_in && in0) ? (in1 ? 8 : 4) : 0;
-    const size_t g = row_in ? (size_t)r * pitch + (size_t)(in0 ? gx0 : 0) : 0;
-    copy8(st + RG::B + 8 * lane, gb + g, nb);
-    copy8(st + RG::D + 8 * lane, gd + g, nb);
-    if constexpr (F16) {
-      copy16(st + RG::F + 16 * lane, reinterpret_cast<const uint2*>(gf) + g, nb * 2);
+  unsigned char* const lane16 = ring + 16 * lane;
+  // ---- the copies of load step i: b and d of row first_row + i, the flux of
+  // the row above it (which level 0 updates in the same iteration).  The
+  // flux of the first two steps is never used.
+  // Flux records go to shared memory in 16-byte chunks, lane l copying chunks
+  // l, l + 32, ... of the row (whole sectors), chunk j at position j with its
+  // low bits exchanged so that a lane's own chunks (4 in a row; FP16: 2) are
+  // read back without bank conflicts.
+  auto chunk = [](int j) { return F16 ? j ^ ((j >> 3) & 1) : j ^ ((j >> 3) & 3); };
+  constexpr int CH = F16 ? 2 : 4;  // chunks of a lane
+  // element index of row first_row + i (advanced with i), column xs or, at the
+  // grid's edge, column 0
+  long long g_in = (long long)first_row * (long long)pitch + (INTERIOR ? xs : 0);
+  const int gx_in = max(0, gx), nb = 4 * cols;
+  auto issue_row = [&](int i) {
+    unsigned char* const sb = lane16 + RG::B + ((unsigned)i % RG::PB) * kSweepRow;
+    unsigned char* const sd = lane16 + RG::D + ((unsigned)i % kSweepDRows) * kSweepRow;
+    unsigned char* const sf = ring + RG::F;
+    const unsigned char* const fb = reinterpret_cast<const unsigned char*>(gf);
+    if constexpr (INTERIOR) {
+      copy16(sb, gb + g_in + 4 * lane, 16);
+      copy16(sd, gd + g_in + 4 * lane, 16);
+      if (i >= 2) {
+        const unsigned char* f = fb + (g_in - (long long)pitch) * (F16 ? 8 : 16) + 16 * lane;
+#pragma unroll
+        for (int k = 0; k < CH; ++k) copy16(sf + 16 * chunk(32 * k + lane), f + 512 * k, 16);
+      }
     } else {
-      const float4* f4 = reinterpret_cast<const float4*>(gf);
-      copy16(st + RG::F + 16 * lane, f4 + g, (row_in && in0) ? 16 : 0);
-      copy16(st + RG::F + 512 + 16 * lane, f4 + g + ((row_in && in1) ? 1 : 0),
-             (row_in && in1) ? 16 : 0);
+      // cells off the grid are cleared: a copy of n bytes zero-fills the rest
+      // of its 16 (of no bytes: it reads nothing)
+      const unsigned r = (unsigned)(first_row + i);  // rows above the grid wrap around
+      const int n = r < (unsigned)H ? nb : 0;
+      const long long g = n ? g_in + gx_in : 0;
+      copy16(sb, gb + g, n);
+      copy16(sd, gd + g, n);
+      if (i >= 2) {
+        const bool row_in = r - 1 < (unsigned)H;
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
+          const int j = 32 * k + lane;
+          const int c = xs + (F16 ? 2 * j : j);  // the chunk's first column
+          const int m = row_in && c >= 0 ? min(F16 ? 2 : 1, max(0, W - c)) : 0;
+          const long long h = m ? g_in - (long long)pitch + c : 0;
+          copy16(sf + 16 * chunk(j), fb + h * (F16 ? 8 : 16), m * (F16 ? 8 : 16));
+        }
+      }
     }
+    g_in += (long long)pitch;
   };
-  auto read_bd = [&](int slot, float2& b, float2& d) {
-    const unsigned char* st = ring + slot * RG::ROW;
-    b = *reinterpret_cast<const float2*>(st + RG::B + 8 * lane);
-    d = *reinterpret_cast<const float2*>(st + RG::D + 8 * lane);
+  auto read_b = [&](int i) -> Quad {  // terrain of load step i
+    return load_quad(lane16 + RG::B + ((unsigned)i % RG::PB) * kSweepRow);
   };
-  auto read_flux = [&](int slot) -> Flux2 {
-    const unsigned char* st = ring + slot * RG::ROW;
+  auto d_row = [&](int i) {  // depth of load step i
+    return lane16 + RG::D + ((unsigned)i % kSweepDRows) * kSweepRow;
+  };
+  auto read_flux = [&]() -> Flux4 {
+    const unsigned char* st = ring + RG::F;
+    float4 c[4];
     if constexpr (F16) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(st + RG::F + 16 * lane);
-      const float2 a0 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.x)), finv2);
-      const float2 a1 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.y)), finv2);
-      const float2 b0 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.z)), finv2);
-      const float2 b1 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.w)), finv2);
-      return Flux2{make_float2(a0.x, b0.x), make_float2(a0.y, b0.y), make_float2(a1.x, b1.x),
-                   make_float2(a1.y, b1.y)};
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(st + 16 * chunk(2 * lane + k));
+        const float2 a0 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.x)), finv2);
+        const float2 a1 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.y)), finv2);
+        const float2 b0 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.z)), finv2);
+        const float2 b1 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.w)), finv2);
+        c[2 * k] = make_float4(a0.x, a0.y, a1.x, a1.y);
+        c[2 * k + 1] = make_float4(b0.x, b0.y, b1.x, b1.y);
+      }
     } else {
-      const float4 c0 = *reinterpret_cast<const float4*>(st + RG::F + 16 * lane);
-      const float4 c1 = *reinterpret_cast<const float4*>(st + RG::F + 512 + 16 * lane);
-      return Flux2{make_float2(c0.x, c1.x), make_float2(c0.y, c1.y), make_float2(c0.z, c1.z),
-                   make_float2(c0.w, c1.w)};
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        c[k] = *reinterpret_cast<const float4*>(st + 16 * chunk(4 * lane + k));
     }
+    return Flux4{pk4(c[0].x, c[1].x, c[2].x, c[3].x), pk4(c[0].y, c[1].y, c[2].y, c[3].y),
+                 pk4(c[0].z, c[1].z, c[2].z, c[3].z), pk4(c[0].w, c[1].w, c[2].w, c[3].w)};
   };
-  // The sources of row r on this lane's two cells, in source order (as
-  // add_sources applies them).  A DISK is tested inline: an out-of-line call
-  // per cell and level made the warps under a rain disk several times slower
-  // than the rest, and with one wave of warps the launch waits for them.
-  auto sources2 = [&](float2 dv, int r) -> float2 {
-    if (!mask || !(INTERIOR || (r >= 0 && r < H))) return dv;
+  // The sources of row r on this lane's four cells, in source order (as
+  // add_sources applies them).  A warp under a rain disk is the slowest of a
+  // launch, so a DISK's four cells go side by side without a branch; the
+  // brush, rare, is a rolled loop over the cells in `slot` (a call would take
+  // registers from the whole kernel).
+  auto sources4 = [&](Quad dq, unsigned char* slot, int r) -> Quad {
+    if (!INTERIOR && (r < 0 || r >= H)) return dq;
 #pragma unroll 1
     for (int k = 0; k < a.nsrc; ++k) {
       if (!((mask >> k) & 1u)) continue;
@@ -195,234 +366,314 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
       if (src.kind == TWS_SOURCE_DISK) {
         const long long dy = r - src.icy;
         const long long room = (long long)src.ir * src.ir - dy * dy;  // dx^2 allowed
-        const long long dx0 = gx0 - src.icx, dx1 = gx1 - src.icx;
-        if (in0 && gx0 >= src.bx0 && gx0 <= src.bx1 && dx0 * dx0 <= room)
-          dv.x = add_rain(dv.x, src.rate, gx0, r);
-        if (in1 && gx1 >= src.bx0 && gx1 <= src.bx1 && dx1 * dx1 <= room)
-          dv.y = add_rain(dv.y, src.rate, gx1, r);
+        const uint32_t hy = rain_hash32((uint32_t)r);
+        const pair_t rate2 = pk(src.rate, src.rate);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          // add_rain of two cells: TwoSum's sum and error, then one ulp
+          // toward d + rate with the probability that makes it exact
+          const pair_t d2 = dq.p[i], s2 = add2(d2, rate2), bp = sub2(s2, d2);
+          const float2 e = un(add2(sub2(d2, sub2(s2, bp)), sub2(rate2, bp)));
+          const float2 d = un(d2), sv = un(s2);
+          auto pick = [&](int c, float dc, float sc, float ec) {
+            const long long dx = gx + c - src.icx;
+            const bool inside = (INTERIOR || c < cols) && dx * dx <= room;
+            const uint32_t sb = __float_as_uint(sc);
+            const float next = __uint_as_float(((sc > 0.0f) == (ec > 0.0f)) ? sb + 1u : sb - 1u);
+            const uint32_t h =
+                rain_hash32(__float_as_uint(dc) ^ rain_hash32((uint32_t)(gx + c) ^ hy));
+            const float u = fmul(__uint2float_rn(h >> 8), 0x1p-24f);
+            const float o = fmul(u, fabsf(fsub(next, sc))) < fabsf(ec) ? next : sc;
+            return inside ? o : dc;
+          };
+          const float o0 = pick(2 * i, d.x, sv.x, e.x), o1 = pick(2 * i + 1, d.y, sv.y, e.y);
+          dq.p[i] = pk(o0, o1);
+        }
       } else {
-        if (in0) dv.x = add_sources(dv.x, gx0, r, a, 1u << k);
-        if (in1) dv.y = add_sources(dv.y, gx1, r, a, 1u << k);
+        store_quad(slot, dq);
+        float* const dv = reinterpret_cast<float*>(slot);
+#pragma unroll 1
+        for (int c = 0; c < cols; ++c) dv[c] = add_sources_inline(dv[c], gx + c, r, a, 1u << k);
+        dq = load_quad(slot);
       }
     }
-    return dv;
+    return dq;
   };
 
-  // ---- per-level windows (registers; every index below is a compile-time
-  // constant once the level loops are unrolled)
-  float2 H0[K], H1[K];  // h of rows ys - 1 and ys of level s's outflow row ys
-  float2 D0[K], D1[K];  // d of rows ys - 1 and ys
-  float2 B0[K], B1[K];  // terrain of rows ys - 1 and ys (it travels with the rows)
-  // The new outflows of rows ys - 1 and ys - 2 live in shared memory (two
-  // slots per level, swapped every iteration), which leaves registers for
-  // four CTAs per SM.  A lane reads back only what it wrote.
-  unsigned char* const nring = ring + RG::RING;
-  auto n_slot = [&](int s, int q) { return nring + (s * 2 + q) * RG::NSLOT; };
-  auto store_n = [&](int s, int q, const Flux2& v) {
-    unsigned char* sl = n_slot(s, q);
-    *reinterpret_cast<float4*>(sl + 16 * lane) = make_float4(v.x.x, v.x.y, v.y.x, v.y.y);
-    *reinterpret_cast<float4*>(sl + 512 + 16 * lane) = make_float4(v.z.x, v.z.y, v.w.x, v.w.y);
-  };
-  auto load_n = [&](int s, int q) -> Flux2 {
-    const unsigned char* sl = n_slot(s, q);
-    const float4 p = *reinterpret_cast<const float4*>(sl + 16 * lane);
-    const float4 m = *reinterpret_cast<const float4*>(sl + 512 + 16 * lane);
-    return Flux2{make_float2(p.x, p.y), make_float2(p.z, p.w), make_float2(m.x, m.y),
-                 make_float2(m.z, m.w)};
-  };
-  auto load_n_z = [&](int s, int q) -> float2 {  // the +y pair alone
-    return *reinterpret_cast<const float2*>(n_slot(s, q) + 512 + 16 * lane);
-  };
-  const float2 z2 = make_float2(0.0f, 0.0f);
+  // ---- what level s carries from row to row in registers (every index is a
+  // compile-time constant once the level loops are unrolled).  In iteration t
+  // its outflow row is ys = first_row + t - 2s - 1, its depth row ys - 1.
+  // Depths and the outflows of all levels but the last wait in shared memory
+  // (a lane reads back only what it wrote).
+  Quad Qm[K];           // ka * (h(ys - 1) - h(ys)): the +y slope term of row ys - 1,
+                        // and minus the -y slope term of row ys
+  Quad InX[K], Out[K];  // row ys - 1: inflow from the x neighbours, outflow sum
+  // the last level: h of row ys; row ys - 1's x flow, +y and -y outflows, and
+  // row ys - 2's +y outflow
+  const Quad zero{{0, 0}};
+  Quad h_c = zero, vx_m = zero, z_m = zero, w_m = zero, z_mm = zero;
 #pragma unroll
-  for (int s = 0; s < K; ++s) {
-    H0[s] = H1[s] = D0[s] = D1[s] = B0[s] = B1[s] = z2;
-    for (int q = 0; q < 2; ++q) store_n(s, q, zero_flux());
-  }
-  int q_prev = 1, q_prev2 = 0;  // slots of rows ys - 1 and ys - 2
+  for (int s = 0; s < K; ++s) Qm[s] = InX[s] = Out[s] = zero;
 
-  // the ring: rows 0 .. P - 2 in flight before the loop
-#pragma unroll
-  for (int i = 0; i < P - 1; ++i) {
-    if (i < rows) issue_row(first_row + i, i);
-    copy_commit();
-  }
-  Flux2 fin_prev = zero_flux();  // flux of the previously loaded row
+  // Iterations, 4K more than the rows this warp has claimed so far: R of them
+  // at first, and kSweepClaim more with every claim on the unit's range.
+  int rows = R + 2 * HALO;
+  bool more = word != nullptr;
+  unsigned long long claim = 0;
 
-  // FP16 storage: two rows per loop trip (the windows shift by register
-  // renaming; 16384^2 264 -> 272 Gcell-steps/s); FP32 gains nothing from it
-#pragma unroll(F16 ? 2 : 1)
-  for (int t = 0; t < rows; ++t) {
+  issue_row(0);
+  copy_commit();
+
+  auto row = [&](const int t) {
     const int r = first_row + t;
-    const int slot = t % P;
-    // refill the slot of row r - 1 (read in full in the previous iteration)
-    // with row r + P - 1, then wait for row r
-    if (t + P - 1 < rows) issue_row(first_row + t + P - 1, (t + P - 1) % P);
+    // load step t has landed, for every lane
+    copy_wait<0>();
+    __syncwarp();
+    const Flux4 f_row = read_flux();  // flux of row r - 1: level 0's outflow row
+    Flux4 f_in = f_row;
+    Quad d_in = load_quad(d_row(t));
+    __syncwarp();  // the flux row has been read: the next one may take its place
+    if (t + 1 < rows) issue_row(t + 1);
     copy_commit();
-    copy_wait<P - 1>();
-    float2 bl, dl;
-    read_bd(slot, bl, dl);
-    const Flux2 fl = read_flux(slot);
     // level 0's input row: the first step's sources, then h = d + b
-    float2 d_in = sources2(dl, r);
-    float2 h_in = fadd2(d_in, bl);
-    float2 b_in = bl;
-    Flux2 f_in = fin_prev;  // flux of row r - 1: level 0's outflow row
-    fin_prev = fl;
+    if (mask) {
+      d_in = sources4(d_in, d_row(t), r);
+      store_quad(d_row(t), d_in);
+    }
+    Quad h_in = add4(d_in, read_b(t));
+    const int q = t & 1;
 
 #pragma unroll
     for (int s = 0; s < K; ++s) {
       const int ys = r - 2 * s - 1;  // this level's outflow row
-      const bool ys_in = INTERIOR || (ys >= 0 && ys < H);
-      // this level's outflow rows ys - 1 and ys - 2 from shared memory, read
-      // ahead of the arithmetic that hides their latency (row ys - 2's slot
-      // is rewritten only after this read, by the same lane)
-      const Flux2 own = load_n(s, q_prev);
-      Flux2 handoff;  // new outflow of row ys - 2: level s + 1's input
-      float2 Y0;
-      if (s + 1 < K) {
-        handoff = load_n(s, q_prev2);
-        Y0 = handoff.z;
-      } else {
-        Y0 = load_n_z(s, q_prev2);
+      // the y slope term of the row pair (ys, ys + 1)
+      unsigned char* const ds = lane16 + RG::DS + ((s - 1) * 2 + q) * kSweepRow;
+      unsigned char* const ds1 = lane16 + RG::DS + ((s - 1) * 2 + (q ^ 1)) * kSweepRow;
+      const Quad dc = load_quad(s == 0 ? d_row(t - 1) : ds1);
+      const Quad dm = load_quad(s == 0 ? d_row(t - 2) : ds);
+      if (s > 0) {
+        if (mask) d_in = sources4(d_in, ds, ys + 1);
+        store_quad(ds, d_in);
+        h_in = add4(d_in, read_b(t - 2 * s));
       }
-      // the parts of the depth update that do not need this row's outflow
-      // (flowApply.comp:32-39): the x inflows and the outflow sum of row
-      // ys - 1, ahead of the outflow's divergent scaling branch
-      const float2 X1 = make_float2(own.y.y, __shfl_down_sync(0xffffffffu, own.y.x, 1));
-      const float2 X0 = make_float2(__shfl_up_sync(0xffffffffu, own.x.y, 1), own.x.x);
-      const float2 in_x = fadd2(X1, X0);
-      const float2 out = fadd2(fadd2(fadd2(own.x, own.y), own.z), own.w);
+      const Quad hc = s + 1 < K ? add4(dc, read_b(t - 2 * s - 1)) : h_c;
+      if (s + 1 == K) h_c = h_in;
+      const Quad qm = Qm[s], qp = prod4(sub4(hc, h_in), ka2, nz2);
+      Qm[s] = qp;
+      // Rows above the band's first needed outflow row of this level (its
+      // windows are filling): nothing below this level is needed either.
+      if (t < 4 * s + 2) break;
+      unsigned char* const slot = lane16 + RG::N + (s * 2 + q) * RG::NSLOT;
 
-      // -- outflow of row ys, flowUpdate.comp:34-62
-      const float2 hm = H0[s], hc = H1[s], hp = h_in;
-      const float2 h_right = make_float2(hc.y, __shfl_down_sync(0xffffffffu, hc.x, 1));
-      const float2 h_left = make_float2(__shfl_up_sync(0xffffffffu, hc.y, 1), hc.x);
-      Flux2 nf;
-      {
-        const float2 e_px = fsub2(hc, h_right), e_mx = fsub2(hc, h_left);
-        const float2 e_py = fsub2(hc, hp), e_my = fsub2(hc, hm);
-        nf.x = max0x2(sum_products(fmul2(f_in.x, kf2), fmul2(e_px, ka2)));
-        nf.y = max0x2(sum_products(fmul2(f_in.y, kf2), fmul2(e_mx, ka2)));
-        nf.z = max0x2(sum_products(fmul2(f_in.z, kf2), fmul2(e_py, ka2)));
-        nf.w = max0x2(sum_products(fmul2(f_in.w, kf2), fmul2(e_my, ka2)));
-      }
+      // -- outflow of row ys, flowUpdate.comp:34-62.  Neighbouring cells share
+      // the slope term of their common edge up to its sign (a - b and b - a
+      // round alike, and so do the products).
+      const float4 h4 = un4(hc);
+      const float hr = __shfl_down_sync(0xffffffffu, h4.x, 1);
+      const Quad qx = prod4(
+          pk4(fsub(h4.x, h4.y), fsub(h4.y, h4.z), fsub(h4.z, h4.w), fsub(h4.w, hr)), ka2, nz2);
+      const float4 q4 = un4(qx);
+      const float ql = __shfl_up_sync(0xffffffffu, q4.w, 1);
+      Flux4 nf;
+      nf.x = max0q(add4(prod4(f_in.x, kf2, nz2), qx));
+      const float4 fy = un4(prod4(f_in.y, kf2, nz2));
+      nf.y = pk4(max0_fast(fsub(fy.x, ql)), max0_fast(fsub(fy.y, q4.x)),
+                 max0_fast(fsub(fy.z, q4.y)), max0_fast(fsub(fy.w, q4.z)));
+      nf.z = max0q(add4(prod4(f_in.z, kf2, nz2), qp));
+      nf.w = max0q(sub4(prod4(f_in.w, kf2, nz2), qm));
       if constexpr (!INTERIOR) {
-        if (closed) {  // no outflow across a closed wall
-          if (gx0 + 1 >= W) nf.x.x = 0.0f;
-          if (gx1 + 1 >= W) nf.x.y = 0.0f;
-          if (gx0 == 0) nf.y.x = 0.0f;
-          if (gx1 == 0) nf.y.y = 0.0f;
-          if (ys + 1 >= H) nf.z = z2;
-          if (ys == 0) nf.w = z2;
-        }
+        // Only what cells on the grid read of cells off it has to be zero:
+        // the +x outflow of column -1, the -x outflow of column W, the +y
+        // outflow of row -1 and the -y outflow of row H.  A closed wall has
+        // no outflow across it either.
+        if (ys < 0 || ys >= H) nf.z = nf.w = zero;
+        if (closed && ys == H - 1) nf.z = zero;
+        if (closed && ys == 0) nf.w = zero;
+        const int wx = closed ? W - 1 : W;  // +x outflow is zero from here on
+        const float4 ox = un4(nf.x), oy = un4(nf.y);
+        nf.x = pk4(gx >= wx ? 0.0f : ox.x, gx + 1 >= wx ? 0.0f : ox.y,
+                   gx + 2 >= wx ? 0.0f : ox.z, gx + 3 >= wx || gx < 0 ? 0.0f : ox.w);
+        nf.y = pk4(gx >= W || (closed && gx == 0) ? 0.0f : oy.x, gx + 1 >= W ? 0.0f : oy.y,
+                   gx + 2 >= W ? 0.0f : oy.z, gx + 3 >= W ? 0.0f : oy.w);
       }
+      Quad out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
       {
-        const float2 dc = D1[s];
-        const float2 total = fmul2(fadd2(fadd2(fadd2(nf.x, nf.y), nf.z), nf.w), cc2);
-        if (total.x > dc.x) {
-          const float sc = scale_factor(dc.x, total.x);
-          nf.x.x = fmul(nf.x.x, sc);
-          nf.y.x = fmul(nf.y.x, sc);
-          nf.z.x = fmul(nf.z.x, sc);
-          nf.w.x = fmul(nf.w.x, sc);
+        const Quad tq = prod4(out, cc2, nz2);
+        const float4 t4 = un4(tq), d4 = un4(dc);
+        const float t[4] = {t4.x, t4.y, t4.z, t4.w}, d[4] = {d4.x, d4.y, d4.z, d4.w};
+        // The factors: d / total where total > d, else 1, which leaves a cell's
+        // bits.  d / total of a dry cell (d = +-0) is d itself.
+        float f[4];
+        bool div[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const bool over = t[c] > d[c];
+          f[c] = over ? d[c] : 1.0f;
+          div[c] = over & (d[c] != 0.0f);
         }
-        if (total.y > dc.y) {
-          const float sc = scale_factor(dc.y, total.y);
-          nf.x.y = fmul(nf.x.y, sc);
-          nf.y.y = fmul(nf.y.y, sc);
-          nf.z.y = fmul(nf.z.y, sc);
-          nf.w.y = fmul(nf.w.y, sc);
+        if ((div[0] | div[1] | div[2] | div[3])) {
+          bool far = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3])) > kDivMaxT;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) far |= div[c] & (d[c] < kDivMinD);
+          if (!far) {
+            const Quad nt = prod4(out, ncc2, nz2);
+            const float2 lo = un(div2(dc.p[0], tq.p[0], nt.p[0]));
+            const float2 hi = un(div2(dc.p[1], tq.p[1], nt.p[1]));
+            f[0] = div[0] ? lo.x : f[0];
+            f[1] = div[1] ? lo.y : f[1];
+            f[2] = div[2] ? hi.x : f[2];
+            f[3] = div[3] ? hi.y : f[3];
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (div[c]) f[c] = fdiv(d[c], t[c]);
+          }
         }
+        const Quad sc = pk4(f[0], f[1], f[2], f[3]);
+        nf.x = prod4(nf.x, sc, nz2);
+        nf.y = prod4(nf.y, sc, nz2);
+        nf.z = prod4(nf.z, sc, nz2);
+        nf.w = prod4(nf.w, sc, nz2);
+        if constexpr (!F16) out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
       }
       if constexpr (F16) {
-        nf.x = quantize_f16x2(nf.x, fscale2, finv2);
-        nf.y = quantize_f16x2(nf.y, fscale2, finv2);
-        nf.z = quantize_f16x2(nf.z, fscale2, finv2);
-        nf.w = quantize_f16x2(nf.w, fscale2, finv2);
+        auto quant = [&](Quad& v) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float2 o = quantize_f16x2(un(v.p[i]), fscale2, finv2);
+            v.p[i] = pk(o.x, o.y);
+          }
+        };
+        quant(nf.x);
+        quant(nf.y);
+        quant(nf.z);
+        quant(nf.w);
       }
-      if constexpr (!INTERIOR) {  // cells off the grid keep zero outflow
-        if (!ys_in) nf = zero_flux();
-        if (!in0) nf.x.x = nf.y.x = nf.z.x = nf.w.x = 0.0f;
-        if (!in1) nf.x.y = nf.y.y = nf.z.y = nf.w.y = 0.0f;
-      }
+      if constexpr (F16) out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
 
-      store_n(s, q_prev2, nf);  // row ys takes the slot of ys - 2, read above
-
-      // -- depth and flow map of row ys - 1, flowApply.comp:32-52
-      const int yd = ys - 1;
-      const float2 Y1 = nf.w;
-      const float2 in = fadd2(fadd2(in_x, Y1), Y0);
-      const float2 dn = max0x2(sum_products(D0[s], fmul2(fsub2(in, out), cc2)));
-      const float2 b_d = B0[s];  // terrain of the depth row
-      // shift the windows
-      H0[s] = hc;
-      H1[s] = hp;
-      D0[s] = D1[s];
-      D1[s] = d_in;
-      B0[s] = B1[s];
-      B1[s] = b_in;
+      // the outflows of row ys - 2 are level s + 1's input; row ys takes
+      // their slot
+      Quad Y0 = z_mm;
       if (s + 1 < K) {
-        // level s + 1's input row yd: next step's sources, h = d + b
-        const bool yd_in = INTERIOR || (yd >= 0 && yd < H);
-        float2 dnext = dn;
+        f_in.x = load_quad(slot);
+        f_in.y = load_quad(slot + kSweepRow);
+        f_in.z = load_quad(slot + 2 * kSweepRow);
+        f_in.w = load_quad(slot + 3 * kSweepRow);
+        Y0 = f_in.z;
+        store_quad(slot, nf.x);
+        store_quad(slot + kSweepRow, nf.y);
+        store_quad(slot + 2 * kSweepRow, nf.z);
+        store_quad(slot + 3 * kSweepRow, nf.w);
+      }
+
+      // -- depth of row ys - 1, flowApply.comp:32-41
+      const Quad in = add4(add4(InX[s], nf.w), Y0);
+      const Quad dn = max0q(add4(dm, prod4(sub4(in, Out[s]), cc2, nz2)));
+      // this row's x inflow and outflow sum, for the depth of row ys
+      const float4 nx = un4(nf.x), ny = un4(nf.y);
+      const float X1r = __shfl_down_sync(0xffffffffu, ny.x, 1);
+      const float X0l = __shfl_up_sync(0xffffffffu, nx.w, 1);
+      InX[s] = pk4(fadd(ny.y, X0l), fadd(ny.z, nx.x), fadd(ny.w, nx.y), fadd(X1r, nx.z));
+      Out[s] = out;
+
+      const int yd = ys - 1;
+      if (s + 1 < K) {
+        // level s + 1's input row yd; cells off the grid stay empty
+        d_in = dn;
         if constexpr (!INTERIOR) {
-          if (!yd_in) dnext = z2;
-          if (!in0) dnext.x = 0.0f;
-          if (!in1) dnext.y = 0.0f;
+          const int n = yd >= 0 && yd < H ? cols : 0;
+          const float4 o = un4(dn);
+          d_in =
+              pk4(n > 0 ? o.x : 0.0f, n > 1 ? o.y : 0.0f, n > 2 ? o.z : 0.0f, n > 3 ? o.w : 0.0f);
         }
-        dnext = sources2(dnext, yd);
-        d_in = dnext;
-        h_in = fadd2(dnext, b_d);
-        b_in = b_d;
-        f_in = handoff;
-      } else if (yd >= y0 && yd < y0 + R && out_lane && (INTERIOR || yd < H)) {
-        // the last level: depth, flux and flow map of row yd go out
-        const size_t g = (size_t)yd * pitch + (size_t)gx0;
-        const float2 vx = fsub2(fsub2(X1, own.x), fsub2(X0, own.y));
-        const float2 vy = fsub2(fsub2(Y1, own.z), fsub2(Y0, own.w));
-        if (INTERIOR || in1) {
-          *reinterpret_cast<float2*>(d_out + g) = dn;
-          *reinterpret_cast<float4*>(v_out + g) = make_float4(vx.x, vy.x, vx.y, vy.y);
+      } else {
+        // the last level: the flux of row ys, the depth and the flow map
+        // (flowApply.comp:45-46) of row yd go out
+        const float4 nz = un4(nf.z), nw = un4(nf.w);
+        if (t >= 4 * K - 1 && t < rows - 1 && out_lane && (INTERIOR || ys < H)) {
+          const size_t g = (size_t)ys * pitch + (size_t)gx;
+          const float4 c[4] = {make_float4(nx.x, ny.x, nz.x, nw.x),
+                               make_float4(nx.y, ny.y, nz.y, nw.y),
+                               make_float4(nx.z, ny.z, nz.z, nw.z),
+                               make_float4(nx.w, ny.w, nz.w, nw.w)};
           if constexpr (F16) {
-            const __half2 p0 = __float22half2_rn(fmul2(make_float2(own.x.x, own.y.x), fscale2));
-            const __half2 q0 = __float22half2_rn(fmul2(make_float2(own.z.x, own.w.x), fscale2));
-            const __half2 p1 = __float22half2_rn(fmul2(make_float2(own.x.y, own.y.y), fscale2));
-            const __half2 q1 = __float22half2_rn(fmul2(make_float2(own.z.y, own.w.y), fscale2));
-            uint4 packed;
-            packed.x = *reinterpret_cast<const uint32_t*>(&p0);
-            packed.y = *reinterpret_cast<const uint32_t*>(&q0);
-            packed.z = *reinterpret_cast<const uint32_t*>(&p1);
-            packed.w = *reinterpret_cast<const uint32_t*>(&q1);
-            *reinterpret_cast<uint4*>(reinterpret_cast<uint2*>(f_out) + g) = packed;
+            uint2 h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const __half2 l = __float22half2_rn(fmul2(make_float2(c[k].x, c[k].y), fscale2));
+              const __half2 u = __float22half2_rn(fmul2(make_float2(c[k].z, c[k].w), fscale2));
+              h[k].x = *reinterpret_cast<const uint32_t*>(&l);
+              h[k].y = *reinterpret_cast<const uint32_t*>(&u);
+            }
+            uint2* fo = reinterpret_cast<uint2*>(f_out) + g;
+            if (INTERIOR || cols == 4) {
+              store32(fo, __uint_as_float(h[0].x), __uint_as_float(h[0].y),
+                      __uint_as_float(h[1].x), __uint_as_float(h[1].y), __uint_as_float(h[2].x),
+                      __uint_as_float(h[2].y), __uint_as_float(h[3].x), __uint_as_float(h[3].y));
+            } else {  // the grid's last columns
+#pragma unroll
+              for (int k = 0; k < 3; ++k)
+                if (k < cols) fo[k] = h[k];
+            }
           } else {
             float4* fo = reinterpret_cast<float4*>(f_out) + g;
-            fo[0] = make_float4(own.x.x, own.y.x, own.z.x, own.w.x);
-            fo[1] = make_float4(own.x.y, own.y.y, own.z.y, own.w.y);
-          }
-        } else if (in0) {  // the grid's last column (odd width)
-          d_out[g] = dn.x;
-          v_out[g] = make_float2(vx.x, vy.x);
-          if constexpr (F16) {
-            const __half2 p0 = __float22half2_rn(fmul2(make_float2(own.x.x, own.y.x), fscale2));
-            const __half2 q0 = __float22half2_rn(fmul2(make_float2(own.z.x, own.w.x), fscale2));
-            uint2 packed;
-            packed.x = *reinterpret_cast<const uint32_t*>(&p0);
-            packed.y = *reinterpret_cast<const uint32_t*>(&q0);
-            reinterpret_cast<uint2*>(f_out)[g] = packed;
-          } else {
-            reinterpret_cast<float4*>(f_out)[g] =
-                make_float4(own.x.x, own.y.x, own.z.x, own.w.x);
+            if (INTERIOR || cols == 4) {
+              store32(fo, c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w);
+              store32(fo + 2, c[2].x, c[2].y, c[2].z, c[2].w, c[3].x, c[3].y, c[3].z, c[3].w);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 3; ++k)
+                if (k < cols) fo[k] = c[k];
+            }
           }
         }
+        if (t >= 4 * K && out_lane && (INTERIOR || yd < H)) {
+          const size_t g = (size_t)yd * pitch + (size_t)gx;
+          const float4 vx = un4(vx_m), vy = un4(sub4(sub4(nf.w, z_m), sub4(Y0, w_m)));
+          const float4 d4 = un4(dn);
+          if (INTERIOR || cols == 4) {
+            *reinterpret_cast<float4*>(d_out + g) = d4;
+            store32(v_out + g, vx.x, vy.x, vx.y, vy.y, vx.z, vy.z, vx.w, vy.w);
+          } else {
+            const float dk[3] = {d4.x, d4.y, d4.z};
+            const float2 vk[3] = {make_float2(vx.x, vy.x), make_float2(vx.y, vy.y),
+                                  make_float2(vx.z, vy.z)};
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              if (k < cols) {
+                d_out[g + k] = dk[k];
+                v_out[g + k] = vk[k];
+              }
+          }
+        }
+        vx_m = pk4(fsub(fsub(ny.y, nx.x), fsub(X0l, ny.x)),
+                   fsub(fsub(ny.z, nx.y), fsub(nx.x, ny.y)),
+                   fsub(fsub(ny.w, nx.z), fsub(nx.y, ny.z)),
+                   fsub(fsub(X1r, nx.w), fsub(nx.z, ny.w)));
+        z_mm = z_m;
+        z_m = nf.z;
+        w_m = nf.w;
       }
     }
-    // the row of this iteration becomes ys - 1, its predecessor ys - 2
-    const int q_row = q_prev2;
-    q_prev2 = q_prev;
-    q_prev = q_row;
+  };
+  auto extend = [&](const int t) {
+    if (!more) return;
+    if (t == rows - kSweepClaim) {  // asked for ahead of its use
+      if (lane == 0) claim = atomicAdd(word, (unsigned long long)kSweepClaim);
+    } else if (t == rows - 2) {
+      const unsigned long long w = __shfl_sync(0xffffffffu, claim, 0);
+      const int left = range_end(w) - range_cur(w);
+      rows += max(0, min(kSweepClaim, left));
+      more = left > kSweepClaim;
+    }
+  };
+#pragma unroll 1
+  for (int t = 0; t < rows; ++t) {
+    row(t);
+    extend(t);
   }
   copy_wait<0>();
+  __syncwarp();  // every lane has read its last rows: the next unit may refill them
 }
 
 // Queue position i -> (strip, band): the units on the grid's border first
@@ -471,13 +722,13 @@ __device__ __forceinline__ void sweep_band(const SweepBands& sb, int H, int i, i
 
 // Persistent warps (one wave): each takes units (strip, band) from the grid's
 // queue until none is left, so warps that drew cheap units take more of them.
-template <int K, bool F16, int P, bool TAIL>
-__global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 4 : 2))
+template <int K, bool F16>
+__global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
     sweep_kernel(const float* __restrict__ b, const float* __restrict__ d,
                  const void* __restrict__ f, const __grid_constant__ StepArgs a,
                  const SweepBands sb) {
-  using RG = SweepRing<K, F16, P>;
-  constexpr int VALID = kSweepCols - 4 * K;
+  using RG = SweepRing<K, F16>;
+  constexpr int VALID = kSweepCols - 2 * kSweepHaloX(K);
   extern __shared__ __align__(128) unsigned char sweep_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strips = (a.W + VALID - 1) / VALID;
@@ -489,37 +740,82 @@ __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 4 : 2))
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   unsigned char* ring = sweep_smem + warp * RG::WARP;
+  const int warps = gridDim.x * kSweepWarps, me = blockIdx.x * kSweepWarps + warp;
+  unsigned long long* const word = a.ranges + me;
+  uint32_t seed = (uint32_t)me;
+  bool queued = true;
   for (;;) {
-    int u = 0;
-    if (lane == 0) u = atomicAdd(&a.queue[0], 1);
-    u = __shfl_sync(0xffffffffu, u, 0);
-    if (u >= total) break;  // the whole warp
-    int si, bi;
-    sweep_unit_coords(u, strips, bands, si, bi);
-    const int xs = si * VALID - 2 * K;
-    int y0, R;
-    if constexpr (TAIL) {
-      sweep_band(sb, a.H, bi, y0, R);
-    } else {  // uniform bands: the height stays a kernel parameter
-      y0 = bi * sb.tall;
-      R = sb.tall;
+    int si = 0, y0 = 0, y1 = 0;
+    if (queued) {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(&a.queue[0], 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+      queued = u < total;
+      if (queued) {
+        int bi, R;
+        sweep_unit_coords(u, strips, bands, si, bi);
+        sweep_band(sb, a.H, bi, y0, R);
+        y1 = y0 + R;
+      }
     }
+    if (!queued) {
+      // the queue is empty: the largest of 64 other warps' ranges, its back half
+      bool got = false;
+      for (int attempt = 0; attempt < kSweepStealTries && !got; ++attempt) {
+        seed = seed * 1664525u + 1013904223u;  // (Numerical Recipes' generator)
+        const unsigned v = (unsigned)(((unsigned long long)seed * (unsigned)warps) >> 32);
+        unsigned long long w = 0;
+        unsigned best = 0;
+        unsigned victim = 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          unsigned j = v + lane + 32 * i;
+          while (j >= (unsigned)warps) j -= (unsigned)warps;
+          const unsigned long long x = *(volatile unsigned long long*)(a.ranges + j);
+          const unsigned left = (unsigned)max(0, range_end(x) - range_cur(x));
+          if (left > best) best = left, w = x, victim = j;
+        }
+        const unsigned top = __reduce_max_sync(0xffffffffu, best << 5 | (unsigned)lane);
+        if ((int)(top >> 5) < kSweepMinSteal) continue;
+        const int from = (int)(top & 31u);
+        int mid = 0;
+        if (lane == from) {
+          const int cur = range_cur(w), end = range_end(w);
+          mid = cur + (end - cur + 1) / 2;
+          if (atomicCAS(a.ranges + victim, w, range_pack(range_strip(w), cur, mid)) != w) mid = 0;
+        }
+        mid = __shfl_sync(0xffffffffu, mid, from);
+        if (mid == 0) continue;
+        w = __shfl_sync(0xffffffffu, w, from);
+        si = range_strip(w);
+        y0 = mid;
+        y1 = range_end(w);
+        got = true;
+      }
+      if (!got) break;  // the whole warp
+    }
+    // the first rows are this warp's at once, the others can be taken over
+    const int R = min(y1 - y0, kSweepClaim);
+    const bool share = y1 - y0 > R;
+    if (share && lane == 0) atomicExch(word, range_pack(si, y0 + R, y1));
+    const int xs = si * VALID - kSweepHaloX(K);
     uint32_t mask = 0;
 #pragma unroll
     for (int k = 0; k < TWS_MAX_SOURCES; ++k) {
       if (k < a.nsrc) {
         const DevSource& s = a.src[k];
-        if (s.bx1 >= xs && s.bx0 < xs + kSweepCols && s.by1 >= y0 - 2 * K &&
-            s.by0 < y0 + R + 2 * K)
+        if (s.bx1 >= xs && s.bx0 < xs + kSweepCols && s.by1 >= y0 - 2 * K && s.by0 < y1 + 2 * K)
           mask |= 1u << k;
       }
     }
     const bool interior =
-        xs >= 0 && xs + kSweepCols <= a.W && y0 - 2 * K >= 0 && y0 + R + 2 * K <= a.H;
+        xs >= 0 && xs + kSweepCols <= a.W && y0 - 2 * K >= 0 && y1 + 2 * K <= a.H;
     if (interior)
-      sweep_unit<K, F16, true, P>(a, b, d, f, a.d_out, a.f_out, a.v_out, ring, xs, y0, R, mask);
+      sweep_unit<K, F16, true>(a, b, d, f, a.d_out, a.f_out, a.v_out, ring, xs, y0, R, mask,
+                               share ? word : nullptr);
     else
-      sweep_unit<K, F16, false, P>(a, b, d, f, a.d_out, a.f_out, a.v_out, ring, xs, y0, R, mask);
+      sweep_unit<K, F16, false>(a, b, d, f, a.d_out, a.f_out, a.v_out, ring, xs, y0, R, mask,
+                                share ? word : nullptr);
   }
   // The last warp to finish resets the queue for the next launch: every other
   // warp has made its final claim by then, and the next launch reads the
@@ -534,36 +830,29 @@ __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 4 : 2))
   }
 }
 
-template <int K, int P>
-const void* sweep_fn(int flux_storage, bool tail) {
-  if (flux_storage == TWS_FLUX_F16)
-    return tail ? reinterpret_cast<const void*>(&sweep_kernel<K, true, P, true>)
-                : reinterpret_cast<const void*>(&sweep_kernel<K, true, P, false>);
-  return tail ? reinterpret_cast<const void*>(&sweep_kernel<K, false, P, true>)
-              : reinterpret_cast<const void*>(&sweep_kernel<K, false, P, false>);
+template <int K>
+const void* sweep_fn(int flux_storage) {
+  return flux_storage == TWS_FLUX_F16 ? reinterpret_cast<const void*>(&sweep_kernel<K, true>)
+                                      : reinterpret_cast<const void*>(&sweep_kernel<K, false>);
 }
 
 }  // namespace
 
-int sweep_valid_columns(int k) { return kSweepCols - 4 * k; }
-
-size_t sweep_smem_bytes(int k, int flux_storage, int ring) {
-  return (size_t)kSweepWarps * sweep_warp_bytes(k, flux_storage == TWS_FLUX_F16, ring);
+size_t sweep_smem_bytes(int k, int flux_storage) {
+  return (size_t)kSweepWarps * sweep_warp_bytes(k, flux_storage == TWS_FLUX_F16);
 }
 
-cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int ring, int flux_storage,
-                              const float* b, const float* d, const void* f, const StepArgs& a,
-                              cudaStream_t s) {
+cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, const float* b,
+                              const float* d, const void* f, const StepArgs& a, cudaStream_t s) {
   const void* fn = nullptr;
-  if (ring != 4) return cudaErrorInvalidValue;
   switch (k) {
-    case 2: fn = sweep_fn<2, 4>(flux_storage, tail_rows > 0); break;
-    case 3: fn = sweep_fn<3, 4>(flux_storage, tail_rows > 0); break;
-    case 4: fn = sweep_fn<4, 4>(flux_storage, tail_rows > 0); break;
+    case 2: fn = sweep_fn<2>(flux_storage); break;
+    case 3: fn = sweep_fn<3>(flux_storage); break;
+    case 4: fn = sweep_fn<4>(flux_storage); break;
     default: return cudaErrorInvalidValue;
   }
-  if (rows < 1 || tail_rows < 0 || !a.queue) return cudaErrorInvalidValue;
-  const size_t smem = sweep_smem_bytes(k, flux_storage, ring);
+  if (rows < 1 || tail_rows < 0 || !a.queue || !a.ranges) return cudaErrorInvalidValue;
+  const size_t smem = sweep_smem_bytes(k, flux_storage);
   // one wave of persistent CTAs (occupancy of this instantiation, queried once)
   static std::mutex mu;
   static std::map<const void*, int> resident;
@@ -587,25 +876,30 @@ cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int ring, int flux
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
     sms = 1;
-  const int valid = kSweepCols - 4 * k;
+  const int valid = kSweepCols - 2 * kSweepHaloX(k);
   const long long strips = (a.W + valid - 1) / valid;
-  // Band partition: with a tail, about one short unit per resident warp ends
-  // the queue (at most half of the rows).
+  // Band partition: uniform bands are made taller as long as every resident
+  // warp has one; with a tail, about one short unit per resident warp ends the
+  // queue (at most half of the rows).
+  const long long ctas = std::min<long long>((long long)per_sm * sms, kSweepMaxWarps / kSweepWarps);
+  const long long warps = ctas * kSweepWarps;
   SweepBands sb{};
   sb.tall = rows;
-  sb.tail = tail_rows > 0 ? tail_rows : rows;
   long long tail_bands = 0;
   if (tail_rows > 0) {
-    const long long warps = (long long)per_sm * sms * kSweepWarps;
     tail_bands = std::min<long long>((warps + strips - 1) / strips, a.H / (2LL * tail_rows));
+  } else if (strips <= warps) {
+    const long long per_strip = warps / strips;
+    sb.tall = (int)std::max<long long>(rows, (a.H + per_strip - 1) / per_strip);
   }
+  sb.tail = tail_rows > 0 ? tail_rows : sb.tall;
   sb.tall_end = a.H - (int)(tail_bands * sb.tail);
-  sb.tall_count = (sb.tall_end + rows - 1) / rows;
+  sb.tall_count = (sb.tall_end + sb.tall - 1) / sb.tall;
   sb.count = sb.tall_count + (int)tail_bands;
   const long long units = strips * sb.count;
   if (units > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const long long blocks =
-      std::min<long long>((units + kSweepWarps - 1) / kSweepWarps, (long long)per_sm * sms);
+  // four warps per unit where there are few units: the others take over rows
+  const long long blocks = std::min(units, ctas);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
