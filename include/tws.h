@@ -233,6 +233,9 @@ TWS_API int tws_set_wait_limit(tws_grid* grid, long long sm_cycles);
  * Where the grid fits the resident kernel (below), that is timed too; if it
  * is fastest, it runs every later tws_step call of at least 16 steps on
  * grids of this shape, and the fastest tiled variant the shorter calls.
+ * Where the mesh kernel (see tws_step) fits and beats them all, no variant is
+ * pinned: it goes on running the calls long enough for it, and the chosen
+ * variant the shorter ones.
  * Synchronous.  `chosen` (may be NULL) receives the variant index, or
  * TWS_VARIANT_RESIDENT if the resident kernel was fastest.  No counterpart
  * in the reference. */
@@ -260,7 +263,17 @@ TWS_API int tws_set_resident(tws_grid* grid, int ctas);
 /* Advance `nsteps` steps: per step, sources, then the outflow update with
  * non-negativity scaling (flowUpdate.comp:12-63), then the depth update and
  * flow vector (flowApply.comp:13-53), fused.  Replaces the dispatch loop of
- * Terrain::PerformSimulationStep (Terrain.cpp:253-265).  Asynchronous. */
+ * Terrain::PerformSimulationStep (Terrain.cpp:253-265).  Asynchronous.
+ *
+ * With nothing pinned (no variant, no steps-per-launch setting, no resident
+ * kernel), calls of at least 4 steps (8 from about half a million cells on)
+ * on grids of up to about 1.1 million cells with at most two brush sources run as one launch of the mesh kernel: the state stays on chip, spread
+ * over all SMs, whose tiles exchange their borders every few steps.  Mesh
+ * launches of one device run one after another, whatever their streams, and
+ * share one workspace of up to some tens of MB, which goes with the last grid
+ * that could use it.  Its waits for neighbouring tiles are bounded by tws_set_wait_limit too, and a
+ * call being captured into a CUDA graph uses the variants.  Results do not
+ * depend on the choice. */
 TWS_API int tws_step(tws_grid* grid, int nsteps);
 
 /* Total water volume sum(d) * cell_area, accumulated in FP64 on the device

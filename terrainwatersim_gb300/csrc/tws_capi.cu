@@ -48,6 +48,10 @@ struct tws_grid {
   int steps_per_launch = 0;  // 0: library's choice
   int variant = -1;          // pinned kernel variant, -1: automatic
   int resident = 0;          // > 0: the resident kernel runs the steps, on this many CTAs
+  int mesh_brushes = -1;     // brush sources that `mesh` was worked out for (-1: not yet)
+  bool mesh_fits = false;
+  MeshShape mesh{};          // how the mesh kernel takes this grid
+  bool mesh_user = false;    // this grid holds the device's mesh workspace
   int auto_ctas = -1;        // the resident kernel's automatic cluster for this grid (-1: not asked yet)
   std::vector<VariantMaps> maps;
   tws_source src[TWS_MAX_SOURCES];
@@ -140,7 +144,7 @@ float pick_flux_scale(float d_max, float c) {
 }
 
 // The error word, the sweep kernel's queue (at byte 16) and its ranges (at 64).
-constexpr size_t kSweepScratch = 64 + sizeof(unsigned long long) * kSweepMaxWarps;
+constexpr size_t kScratchBytes = 64 + sizeof(unsigned long long) * kSweepMaxWarps;
 
 VariantMaps* maps_for(tws_grid* g, int variant, std::string* why) {
   if ((int)g->maps.size() < step_variant_count()) g->maps.resize(step_variant_count());
@@ -164,10 +168,11 @@ struct TunedKey {
     return w != o.w ? w < o.w : (h != o.h ? h < o.h : fs < o.fs);
   }
 };
-// The fastest tiled variant, and whether the resident kernel beat it.
+// The fastest variant, and whether the resident or the mesh kernel beat it.
 struct Tuned {
   int variant = -1;
   bool resident = false;
+  bool mesh = false;
 };
 std::mutex g_tuned_mu;
 std::map<TunedKey, Tuned> g_tuned;
@@ -221,6 +226,117 @@ int resident_ctas(tws_grid* g, int nsteps) {
   return g->auto_ctas;
 }
 
+// Calls shorter than this stay with the step kernels: a mesh launch loads and
+// stores the whole state and sets up its exchange.  Microseconds per call with the
+// mesh kernel and with two-step tiles, a rain disk: 64^2, 8 steps 14.8 and 37.7
+// (about 10 and 19.5 at 4); 512^2, 8 steps 27.3 and 44.2 (17.5 and 22.7 at 4);
+// 1021 x 763, 8 steps 50.4 and 56.4 (about equal at 4).
+int mesh_min_steps(const MeshShape& s) { return s.ry <= 4 ? 4 : 8; }
+
+// How the mesh kernel runs a call of `nsteps` steps, or null if it does not: it
+// runs the calls of at least mesh_min_steps steps on grids that fit it, unless
+// a variant, a steps-per-launch setting or the resident kernel is chosen or
+// the autotuner found another kernel faster for this grid shape.
+const MeshShape* mesh_for(tws_grid* g, int nsteps) {
+  if (!g->mesh_user || nsteps < 4 || g->resident > 0 || g->variant >= 0 || g->steps_per_launch != 0)
+    return nullptr;
+  int brushes = 0;
+  for (int i = 0; i < g->nsrc; ++i) brushes += g->src[i].kind != TWS_SOURCE_DISK;
+  if (g->mesh_brushes != brushes) {
+    g->mesh_fits = mesh_shape(g->W, g->H, brushes, &g->mesh);
+    g->mesh_brushes = brushes;
+  }
+  if (!g->mesh_fits || nsteps < mesh_min_steps(g->mesh)) return nullptr;
+  const Tuned t = tuned_lookup(g);
+  if (t.variant >= 0 && !t.mesh) return nullptr;
+  return &g->mesh;
+}
+
+// The mesh kernel's inboxes, one set per device, held by the grids that the kernel
+// fits: made with the first, grown for one that needs more, freed with the last.
+// Mesh launches of one device run one after another, whatever their streams (each
+// waits for the previous one's event): they share the inboxes, and their CTAs
+// wait for one another, so two of them must not hold half of the SMs each.
+struct MeshSpace {
+  std::mutex mu;
+  int users = 0;
+  char* inbox = nullptr;
+  size_t bytes = 0;
+  unsigned epoch = 0;         // number of the last exchange
+  cudaEvent_t done = nullptr;  // the last launch, or the inboxes' clearing
+};
+
+MeshSpace* mesh_space(int device) {
+  static MeshSpace spaces[64];
+  return device >= 0 && device < 64 ? &spaces[device] : nullptr;
+}
+
+// Takes (or grows) the inboxes for a grid, in its stream's order.
+cudaError_t mesh_hold(int device, size_t bytes, cudaStream_t s) {
+  MeshSpace* m = mesh_space(device);
+  if (!m) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lk(m->mu);
+  cudaError_t e = cudaSuccess;
+  if (!m->done) e = cudaEventCreateWithFlags(&m->done, cudaEventDisableTiming);
+  if (e == cudaSuccess && bytes > m->bytes) {
+    char* p = nullptr;
+    cudaMemPool_t pool = library_pool(device);
+    e = pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), bytes, pool, s)
+             : cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, s);
+    if (e == cudaSuccess && m->inbox) {
+      e = cudaStreamWaitEvent(s, m->done, 0);
+      if (e == cudaSuccess) e = cudaFreeAsync(m->inbox, s);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(m->done, s);
+    if (e != cudaSuccess) {
+      if (p) cudaFreeAsync(p, s);
+      return e;
+    }
+    m->inbox = p;
+    m->bytes = bytes;
+    m->epoch = 0;
+  }
+  if (e == cudaSuccess) ++m->users;
+  return e;
+}
+
+void mesh_release(int device, cudaStream_t s) {
+  MeshSpace* m = mesh_space(device);
+  if (!m) return;
+  std::lock_guard<std::mutex> lk(m->mu);
+  if (--m->users > 0) return;
+  if (m->inbox && cudaStreamWaitEvent(s, m->done, 0) == cudaSuccess) cudaFreeAsync(m->inbox, s);
+  m->inbox = nullptr;
+  m->bytes = 0;
+  if (m->done) cudaEventDestroy(m->done);
+  m->done = nullptr;
+}
+
+// One launch of `n` steps in the device's mesh order.
+cudaError_t launch_in_mesh_order(tws_grid* g, const MeshShape& shape, const StepArgs& a, int n) {
+  MeshSpace* m = mesh_space(g->device);
+  if (!m) return cudaErrorInvalidDevice;
+  float* d[2] = {g->d[g->cur], g->d[g->cur ^ 1]};
+  void* f[2] = {g->f[g->cur], g->f[g->cur ^ 1]};
+  const unsigned x = (unsigned)mesh_exchanges(shape, n);
+  std::lock_guard<std::mutex> lk(m->mu);
+  cudaError_t e = cudaStreamWaitEvent(g->stream, m->done, 0);
+  if (e == cudaSuccess && (mesh_inbox_bytes(shape) > m->bytes || !m->inbox))
+    e = cudaErrorInvalidValue;
+  if (e == cudaSuccess && m->epoch > 0xffffffffu - x) {  // the numbers start again
+    e = cudaMemsetAsync(m->inbox, 0, m->bytes, g->stream);
+    m->epoch = 0;
+  }
+  if (e == cudaSuccess)
+    e = launch_mesh(shape, g->flux_storage, g->b, d, f, a, n, m->inbox, m->epoch, g->stream);
+  if (e == cudaSuccess) {
+    m->epoch += x;
+    e = cudaEventRecord(m->done, g->stream);
+  }
+  return e;
+}
+
 StepArgs make_step_args(const tws_grid* g) {
   StepArgs a{};
   a.W = g->W;
@@ -246,6 +362,26 @@ StepArgs make_step_args(const tws_grid* g) {
 
 int enqueue_steps(tws_grid* g, int nsteps) {
   StepArgs a = make_step_args(g);
+  const MeshShape* mesh = mesh_for(g, nsteps);
+  if (mesh) {
+    // (the launches' order is kept by an event, which a capture cannot hold)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      mesh = nullptr;
+    }
+  }
+  if (mesh) {
+    for (int left = nsteps; left > 0;) {
+      const int n = std::min(left, kResidentMaxSteps);
+      const cudaError_t e = launch_in_mesh_order(g, *mesh, a, n);
+      if (e != cudaSuccess) return cuda_fail(g, e, "mesh kernel launch");
+      g->cur ^= 1;
+      left -= n;
+    }
+    return TWS_OK;
+  }
   if (const int ctas = resident_ctas(g, nsteps)) {
     for (int left = nsteps; left > 0;) {
       const int n = std::min(left, kResidentMaxSteps);
@@ -397,7 +533,7 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   const size_t ob = take(n * 4), od0 = take(n * 4), od1 = take(n * 4), of0 = take(n * fb),
                of1 = take(n * fb), ov = take(n * 8),
                op = take(sizeof(double) * volume_partials_needed()), oo = take(sizeof(double)),
-               oe = take(kSweepScratch), ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
+               oe = take(kScratchBytes), ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
   cudaMemPool_t pool = library_pool(g->device);
   if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&g->slab), off, pool, g->stream) !=
                    cudaSuccess) {
@@ -424,7 +560,21 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   cudaMemsetAsync(g->f[0], 0, n * fb, g->stream);
   cudaMemsetAsync(g->f[1], 0, n * fb, g->stream);
   cudaMemsetAsync(g->v, 0, n * 8, g->stream);
-  cudaMemsetAsync(g->err, 0, kSweepScratch, g->stream);  // error word, sweep queue and ranges
+  cudaMemsetAsync(g->err, 0, kScratchBytes, g->stream);
+  // the mesh kernel's workspace, where it fits this grid (whatever its sources)
+  size_t inbox = 0;
+  for (int brushes = 0; brushes <= TWS_MAX_SOURCES; ++brushes) {
+    MeshShape shape;
+    if (mesh_shape(width, height, brushes, &shape))
+      inbox = std::max(inbox, mesh_inbox_bytes(shape));
+  }
+  if (inbox > 0) {
+    if (mesh_hold(g->device, inbox, g->stream) != cudaSuccess) {
+      cudaGetLastError();  // the step kernels run without it
+    } else {
+      g->mesh_user = true;
+    }
+  }
   if (cudaStreamSynchronize(g->stream) != cudaSuccess) return bail(TWS_ERR_CUDA);
   *out = g;
   return TWS_OK;
@@ -443,6 +593,7 @@ TWS_API int tws_destroy(tws_grid* g) {
     if (ev) cudaEventDestroy(ev);
   if (g->io_up) cudaStreamDestroy(g->io_up);
   if (g->io_down) cudaStreamDestroy(g->io_down);
+  if (g->mesh_user) mesh_release(g->device, g->stream);
   if (g->slab) cudaFreeAsync(g->slab, g->stream);
   if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
   delete g;
@@ -694,7 +845,7 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
     }
   }
   // the resident kernel, where the grid fits it
-  bool resident_best = false;
+  bool resident_best = false, mesh_best = false;
   int res_ctas = 0;
   if (rc == TWS_OK &&
       resident_supported(g->W, g->H, g->flux_storage, 0, &res_ctas) == cudaSuccess) {
@@ -711,8 +862,32 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
       rbest = std::min(rbest, ms);
     }
     resident_best = rc == TWS_OK && rbest < best_ms;
+    if (resident_best) best_ms = rbest;
     g->resident = 0;
   }
+  // and the mesh kernel
+  {
+    std::lock_guard<std::mutex> lk(g_tuned_mu);
+    g_tuned.erase(TunedKey{g->W, g->H, g->flux_storage});
+  }
+  const int saved_spl = g->steps_per_launch;
+  g->variant = -1;
+  g->steps_per_launch = 0;
+  if (rc == TWS_OK && mesh_for(g, steps)) {
+    float mbest = 1e30f;
+    for (int rep = 0; rep < 2 && rc == TWS_OK; ++rep) {
+      restore();
+      cudaEventRecord(e0, g->stream);
+      rc = enqueue_steps(g, steps);
+      cudaEventRecord(e1, g->stream);
+      if (cudaEventSynchronize(e1) != cudaSuccess) rc = TWS_ERR_CUDA;
+      float ms = 0.0f;
+      cudaEventElapsedTime(&ms, e0, e1);
+      mbest = std::min(mbest, ms);
+    }
+    mesh_best = rc == TWS_OK && mbest < best_ms;
+  }
+  g->steps_per_launch = saved_spl;
   cudaGetLastError();  // a grid that does not fit leaves the query's error behind
   restore();
   cudaFreeAsync(saved, g->stream);
@@ -724,14 +899,14 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
     g->resident = saved_resident;
     return rc;
   }
-  // a resident choice is not pinned: it runs the long calls, the fastest
-  // tiled variant the short ones
-  g->variant = resident_best ? -1 : best;
+  // with a resident or mesh kernel ahead nothing is pinned: it runs the long
+  // calls, the fastest variant the short ones
+  g->variant = resident_best || mesh_best ? -1 : best;
   g->resident = 0;
   const int choice = resident_best ? TWS_VARIANT_RESIDENT : best;
   {
     std::lock_guard<std::mutex> lk(g_tuned_mu);
-    g_tuned[TunedKey{g->W, g->H, g->flux_storage}] = Tuned{best, resident_best};
+    g_tuned[TunedKey{g->W, g->H, g->flux_storage}] = Tuned{best, resident_best, mesh_best};
   }
   if (chosen) *chosen = choice;
   return TWS_OK;

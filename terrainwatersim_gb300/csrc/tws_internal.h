@@ -152,6 +152,29 @@ cudaError_t resident_supported(int W, int H, int flux_storage, int ctas, int* ch
 cudaError_t launch_resident(int flux_storage, int ctas, const float* b, const float* d,
                             const void* f, const StepArgs& a, int nsteps, cudaStream_t s);
 
+// tws_mesh.cu: grids of up to about a million cells with their state on chip
+// across all SMs, all steps of a call in one cooperative launch.
+struct MeshShape {
+  int ry;                // rows per warp
+  int every;             // steps between exchanges
+  int hx, hy;            // halo of a CTA's box
+  int tiles_x, tiles_y;  // CTAs
+  int brushes;           // brush sources (a plane of shared memory each)
+};
+constexpr int kMeshMaxCtas = 256;
+// Whether a W x H grid with that many brush sources fits, and how.
+bool mesh_shape(int W, int H, int brushes, MeshShape* out);
+// Exchanges of a launch.
+int mesh_exchanges(const MeshShape& s, int nsteps);
+// Bytes of the CTAs' inboxes: zeroed once, then every exchange of every launch that
+// uses them has a number of its own (never 0).
+size_t mesh_inbox_bytes(const MeshShape& s);
+// d[0], f[0]: the state; d[1], f[1]: where the result goes.  `epoch`: the number of
+// the last exchange before.
+cudaError_t launch_mesh(const MeshShape& s, int flux_storage, const float* b, float* const d[2],
+                        void* const f[2], const StepArgs& a, int nsteps, void* inbox,
+                        unsigned epoch, cudaStream_t st);
+
 // tws_aux.cu
 cudaError_t launch_apply_source(float* d, int W, int H, int pitch, const DevSource& s,
                                 cudaStream_t st);

@@ -58,6 +58,7 @@
 
 #include "tws_device.cuh"
 #include "tws_internal.h"
+#include "tws_pair.cuh"
 
 namespace tws {
 namespace {
@@ -88,116 +89,6 @@ template <int N>
 __device__ __forceinline__ void copy_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-// A lane's two cells as one packed f32x2 operand, kept in a 64-bit register (its
-// low half is the lane's first column): values that stay packed from one row to
-// the next then cost no moves to line their halves up.
-typedef unsigned long long pair_t;
-__device__ __forceinline__ pair_t pk(float x, float y) {
-  pair_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float2 un(pair_t p) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
-  return r;
-}
-__device__ __forceinline__ pair_t add2(pair_t a, pair_t b) {
-  pair_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ pair_t sub2(pair_t a, pair_t b) {
-  pair_t r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-// a * b rounded, with -0 added: the product's own bits (x + -0 = x for every x,
-// -0 included), as a fused multiply-add that no later sum can be contracted
-// with.  `nz` must reach the kernel as data (StepArgs::neg_zero).
-__device__ __forceinline__ pair_t prod2(pair_t a, pair_t b, pair_t nz) {
-  pair_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
-  return r;
-}
-__device__ __forceinline__ pair_t max0p(pair_t v) {
-  const float2 f = un(v);
-  return pk(max0_fast(f.x), max0_fast(f.y));
-}
-
-// d / t per half, rounded to nearest, for t up to kDivMaxT and d in
-// [kDivMinD, t): nothing on the way then overflows or leaves the normal range.
-// Markstein's division (IBM J. Res. Dev. 34, 1990): a reciprocal refined to
-// its correct rounding with one Newton step in fused arithmetic, a quotient
-// within an ulp, and the exact remainder's correction.  Against the
-// correctly rounded quotient: no difference in 1e11 random and structured
-// pairs of that range, nor in the pairs closest to a rounding boundary.
-// `nt` is -t.
-constexpr float kDivMinD = 0x1p-100f, kDivMaxT = 0x1p20f;
-__device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
-  pair_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ pair_t div2(pair_t d, pair_t t, pair_t nt) {
-  const float2 tv = un(t);
-  float y0, y1;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(tv.x));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(tv.y));
-  pair_t y = pk(y0, y1);
-  y = fma2(fma2(nt, y, pk(1.0f, 1.0f)), y, y);
-  pair_t q;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(d), "l"(y));
-  return fma2(fma2(nt, q, d), y, q);
-}
-
-// A lane's four cells: columns 0, 1 and 2, 3.
-struct Quad {
-  pair_t p[2];
-};
-#define TWS_QUAD_OP(name, op)                                     \
-  __device__ __forceinline__ Quad name(const Quad& a, const Quad& b) { \
-    return Quad{{op(a.p[0], b.p[0]), op(a.p[1], b.p[1])}};          \
-  }
-TWS_QUAD_OP(add4, add2)
-TWS_QUAD_OP(sub4, sub2)
-#undef TWS_QUAD_OP
-__device__ __forceinline__ Quad prod4(const Quad& a, pair_t b, pair_t nz) {
-  return Quad{{prod2(a.p[0], b, nz), prod2(a.p[1], b, nz)}};
-}
-__device__ __forceinline__ Quad prod4(const Quad& a, const Quad& b, pair_t nz) {
-  return Quad{{prod2(a.p[0], b.p[0], nz), prod2(a.p[1], b.p[1], nz)}};
-}
-__device__ __forceinline__ Quad max0q(const Quad& v) {
-  return Quad{{max0p(v.p[0]), max0p(v.p[1])}};
-}
-__device__ __forceinline__ float4 un4(const Quad& v) {
-  const float2 l = un(v.p[0]), h = un(v.p[1]);
-  return make_float4(l.x, l.y, h.x, h.y);
-}
-__device__ __forceinline__ Quad pk4(float x, float y, float z, float w) {
-  return Quad{{pk(x, y), pk(z, w)}};
-}
-__device__ __forceinline__ Quad load_quad(const unsigned char* p) {
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-  return Quad{{v.x, v.y}};
-}
-__device__ __forceinline__ void store_quad(unsigned char* p, const Quad& v) {
-  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.p[0], v.p[1]);
-}
-// One 32-byte store (whole sectors; the address is a multiple of 32).
-__device__ __forceinline__ void store32(void* p, float a, float b, float c, float d, float e,
-                                        float f, float g, float h) {
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b),
-               "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h)
-               : "memory");
-}
-
-// The four outflow channels (+x, -x, +y, -y) of a lane's four cells.
-struct Flux4 {
-  Quad x, y, z, w;
-};
 
 // Shared memory of one warp, in bytes.
 constexpr int kSweepRow = kSweepCols * 4;  // one float per column
@@ -367,28 +258,15 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
         const long long dy = r - src.icy;
         const long long room = (long long)src.ir * src.ir - dy * dy;  // dx^2 allowed
         const uint32_t hy = rain_hash32((uint32_t)r);
-        const pair_t rate2 = pk(src.rate, src.rate);
+        bool in[4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          // add_rain of two cells: TwoSum's sum and error, then one ulp
-          // toward d + rate with the probability that makes it exact
-          const pair_t d2 = dq.p[i], s2 = add2(d2, rate2), bp = sub2(s2, d2);
-          const float2 e = un(add2(sub2(d2, sub2(s2, bp)), sub2(rate2, bp)));
-          const float2 d = un(d2), sv = un(s2);
-          auto pick = [&](int c, float dc, float sc, float ec) {
-            const long long dx = gx + c - src.icx;
-            const bool inside = (INTERIOR || c < cols) && dx * dx <= room;
-            const uint32_t sb = __float_as_uint(sc);
-            const float next = __uint_as_float(((sc > 0.0f) == (ec > 0.0f)) ? sb + 1u : sb - 1u);
-            const uint32_t h =
-                rain_hash32(__float_as_uint(dc) ^ rain_hash32((uint32_t)(gx + c) ^ hy));
-            const float u = fmul(__uint2float_rn(h >> 8), 0x1p-24f);
-            const float o = fmul(u, fabsf(fsub(next, sc))) < fabsf(ec) ? next : sc;
-            return inside ? o : dc;
-          };
-          const float o0 = pick(2 * i, d.x, sv.x, e.x), o1 = pick(2 * i + 1, d.y, sv.y, e.y);
-          dq.p[i] = pk(o0, o1);
+        for (int c = 0; c < 4; ++c) {
+          const long long dx = gx + c - src.icx;
+          in[c] = (INTERIOR || c < cols) && dx * dx <= room;
         }
+        auto cell = [&](int c) { return rain_hash32((uint32_t)(gx + c) ^ hy); };
+        dq.p[0] = rain2(dq.p[0], src.rate, cell(0), cell(1), in[0], in[1]);
+        dq.p[1] = rain2(dq.p[1], src.rate, cell(2), cell(3), in[2], in[3]);
       } else {
         store_quad(slot, dq);
         float* const dv = reinterpret_cast<float*>(slot);
@@ -498,38 +376,7 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
       }
       Quad out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
       {
-        const Quad tq = prod4(out, cc2, nz2);
-        const float4 t4 = un4(tq), d4 = un4(dc);
-        const float t[4] = {t4.x, t4.y, t4.z, t4.w}, d[4] = {d4.x, d4.y, d4.z, d4.w};
-        // The factors: d / total where total > d, else 1, which leaves a cell's
-        // bits.  d / total of a dry cell (d = +-0) is d itself.
-        float f[4];
-        bool div[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const bool over = t[c] > d[c];
-          f[c] = over ? d[c] : 1.0f;
-          div[c] = over & (d[c] != 0.0f);
-        }
-        if ((div[0] | div[1] | div[2] | div[3])) {
-          bool far = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3])) > kDivMaxT;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) far |= div[c] & (d[c] < kDivMinD);
-          if (!far) {
-            const Quad nt = prod4(out, ncc2, nz2);
-            const float2 lo = un(div2(dc.p[0], tq.p[0], nt.p[0]));
-            const float2 hi = un(div2(dc.p[1], tq.p[1], nt.p[1]));
-            f[0] = div[0] ? lo.x : f[0];
-            f[1] = div[1] ? lo.y : f[1];
-            f[2] = div[2] ? hi.x : f[2];
-            f[3] = div[3] ? hi.y : f[3];
-          } else {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (div[c]) f[c] = fdiv(d[c], t[c]);
-          }
-        }
-        const Quad sc = pk4(f[0], f[1], f[2], f[3]);
+        const Quad sc = outflow_factors(out, dc, cc2, ncc2, nz2);
         nf.x = prod4(nf.x, sc, nz2);
         nf.y = prod4(nf.y, sc, nz2);
         nf.z = prod4(nf.z, sc, nz2);
