@@ -12,6 +12,8 @@ namespace {
 
 // ---- one-shot source (the reference's brush dispatch, Terrain.cpp:150-168) --
 __global__ void apply_source_kernel(float* d, int W, int H, int pitch, StepArgs a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int gx = a.src[0].bx0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int gy = a.src[0].by0 + blockIdx.y * blockDim.y + threadIdx.y;
   if (gx > a.src[0].bx1 || gy > a.src[0].by1 || gx >= W || gy >= H) return;
@@ -388,9 +390,9 @@ cudaError_t launch_apply_source(float* d, int W, int H, int pitch, const DevSour
   if (a.src[0].bx0 > a.src[0].bx1 || a.src[0].by0 > a.src[0].by1) return cudaSuccess;
   const int w = a.src[0].bx1 - a.src[0].bx0 + 1, h = a.src[0].by1 - a.src[0].by0 + 1;
   dim3 blk(32, 8), grd((w + 31) / 32, (h + 7) / 8);
-  apply_source_kernel<<<grd, blk, 0, st>>>(d, W, H, pitch, a);
+  const cudaError_t e = launch_after_previous(apply_source_kernel, grd, blk, st, d, W, H, pitch, a);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 int volume_partials_needed() { return kVolMaxBlocks; }

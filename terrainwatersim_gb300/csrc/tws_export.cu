@@ -24,6 +24,22 @@
 namespace tws {
 namespace {
 
+// Programmatic dependent launch, as for the step kernels: a launch may be scheduled
+// while the one before it on the stream finishes, and waits here until that one
+// has completed and its writes are visible; it lets the next one in turn.  A
+// frame (brush, step, export, mips) saves most of the gaps between its launches.
+__device__ __forceinline__ void previous_launch_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Two RGBA32F texels in one 32-byte store (p on a 32-byte boundary).
+__device__ __forceinline__ void store_texels(float4* p, const float4& a, const float4& b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x),
+               "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+
 __device__ __forceinline__ float surf(const float* b, const float* d, size_t i) {
   return fadd(d[i], b[i]);
 }
@@ -45,6 +61,7 @@ __device__ __forceinline__ void heightmap_cross(float A, float B, float& nx, flo
 __global__ void surface_kernel(const float* __restrict__ b, const float* __restrict__ d,
                                const float2* __restrict__ v, int W, int H, int pitch,
                                tws_surface_out o) {
+  previous_launch_done();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= W || y >= H) return;
@@ -89,6 +106,7 @@ __global__ void surface_kernel(const float* __restrict__ b, const float* __restr
 __global__ void surface_kernel4(const float* __restrict__ b, const float* __restrict__ d,
                                 const float2* __restrict__ v, int W, int H, int pitch,
                                 tws_surface_out o) {
+  previous_launch_done();
   const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= W || y >= H) return;
@@ -162,6 +180,7 @@ __global__ void surface_kernel4(const float* __restrict__ b, const float* __rest
 __global__ void export_kernel4(const float* __restrict__ b, const float* __restrict__ d,
                                const float2* __restrict__ v, int W, int H, int pitch,
                                float4* __restrict__ rgba, __half2* __restrict__ flowmap) {
+  previous_launch_done();
   const int x = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= W || y >= H) return;
@@ -191,6 +210,7 @@ __global__ void export_kernel4(const float* __restrict__ b, const float* __restr
 
 __global__ void terrain_rgba_kernel(const float* __restrict__ b, const float* __restrict__ d,
                                     int W, int H, int pitch, float4* __restrict__ out) {
+  previous_launch_done();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= W || y >= H) return;
@@ -200,6 +220,7 @@ __global__ void terrain_rgba_kernel(const float* __restrict__ b, const float* __
 
 __global__ void flowmap_kernel(const float2* __restrict__ v, int W, int H, int pitch,
                                __half2* __restrict__ out) {
+  previous_launch_done();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= W || y >= H) return;
@@ -230,6 +251,7 @@ struct MipChain {
 
 __global__ void __launch_bounds__(256)
     mip_chain_kernel(const float4* __restrict__ src, int sw, int sh, MipChain c) {
+  previous_launch_done();
   constexpr int Q = kMipBlock / 2;  // the first level's texels per block side
   __shared__ float4 buf[2][Q * Q];
   const int bx = blockIdx.x * kMipBlock, by = blockIdx.y * kMipBlock;
@@ -282,30 +304,39 @@ __global__ void __launch_bounds__(256)
 // level, with the filter of mip_chain_kernel.  Texels past a level's edge are
 // computed from zero fill and not written; level-1 texels inside the level
 // use only cells on the grid.
-constexpr int kMipFused = 6;  // 64 -> 32 -> 16 -> 8 -> 4 -> 2 -> 1
+constexpr int kMipFused = 6;  // a block of 64 cells: 32 -> 16 -> 8 -> 4 -> 2 -> 1
 struct MipLevels {
   float4* dst[kMipFused];
   int w[kMipFused], h[kMipFused];  // sizes of the levels written
   int n;                           // levels written, 1 .. kMipFused
 };
 
-__global__ void __launch_bounds__(256)
+// Q: level-1 texels per block side, 32 or 16 (blocks of 64 or 32 cells).  WHOLE: the
+// width is a multiple of 4, terrain_rgba lies on a 32-byte and the flow map on a
+// 16-byte boundary: a thread's four texels go out in whole sectors.  Else any
+// width and alignment, texel by texel.
+template <int Q, bool WHOLE>
+__global__ void __launch_bounds__(8 * Q)
     export_mips_kernel4(const float* __restrict__ b, const float* __restrict__ d,
                         const float2* __restrict__ v, int W, int H, int pitch,
                         float4* __restrict__ rgba, __half2* __restrict__ flowmap, MipLevels m) {
-  constexpr int Q = 32;  // level-1 texels per block side
+  constexpr int HALVES = Q / 16;  // pairs of cell rows per thread: 16 rows of threads
+  constexpr int LEVELS = Q == 32 ? kMipFused : kMipFused - 1;
   __shared__ float4 buf[2][Q * Q];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads
-  const int bx = blockIdx.x * 64, by = blockIdx.y * 64;
+  previous_launch_done();
+  const int tx = threadIdx.x % (Q / 2), ty = threadIdx.x / (Q / 2);
+  const int bx = blockIdx.x * 2 * Q, by = blockIdx.y * 2 * Q;
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
+  for (int half = 0; half < HALVES; ++half) {
     // cells (x .. x + 3, y .. y + 1); level-1 texels (x/2, x/2 + 1) of row y/2
-    const int x = bx + 4 * tx, y = by + 4 * ty + 2 * half;
+    const int x = bx + 4 * tx, y = by + 2 * HALVES * ty + 2 * half;
     float4 t[2][4];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       if (x < W && y + r < H) {
+        // (a pitched row has room for the quad; its cells past the width are not
+        // written, and no texel inside a level uses them)
         const size_t i = (size_t)(y + r) * pitch + x;
         const size_t out = (size_t)(y + r) * W + x;
         const float4 b4 = *reinterpret_cast<const float4*>(b + i);
@@ -314,28 +345,38 @@ __global__ void __launch_bounds__(256)
         t[r][1] = make_float4(b4.y, 0.3f, 0.3f, d4.y);
         t[r][2] = make_float4(b4.z, 0.3f, 0.3f, d4.z);
         t[r][3] = make_float4(b4.w, 0.3f, 0.3f, d4.w);
+        if constexpr (WHOLE) {
+          store_texels(rgba + out, t[r][0], t[r][1]);
+          store_texels(rgba + out + 2, t[r][2], t[r][3]);
+        } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) rgba[out + k] = t[r][k];
+          for (int k = 0; k < 4; ++k)
+            if (x + k < W) rgba[out + k] = t[r][k];
+        }
         if (flowmap) {
           const float4 v01 = *reinterpret_cast<const float4*>(v + i);
           const float4 v23 = *reinterpret_cast<const float4*>(v + i + 2);
-          const __half2 h0 = __floats2half2_rn(v01.x, v01.y);
-          const __half2 h1 = __floats2half2_rn(v01.z, v01.w);
-          const __half2 h2 = __floats2half2_rn(v23.x, v23.y);
-          const __half2 h3 = __floats2half2_rn(v23.z, v23.w);
-          uint4 packed;
-          packed.x = *reinterpret_cast<const uint32_t*>(&h0);
-          packed.y = *reinterpret_cast<const uint32_t*>(&h1);
-          packed.z = *reinterpret_cast<const uint32_t*>(&h2);
-          packed.w = *reinterpret_cast<const uint32_t*>(&h3);
-          *reinterpret_cast<uint4*>(flowmap + out) = packed;
+          const __half2 h[4] = {__floats2half2_rn(v01.x, v01.y), __floats2half2_rn(v01.z, v01.w),
+                                __floats2half2_rn(v23.x, v23.y), __floats2half2_rn(v23.z, v23.w)};
+          if constexpr (WHOLE) {
+            uint4 packed;
+            packed.x = *reinterpret_cast<const uint32_t*>(&h[0]);
+            packed.y = *reinterpret_cast<const uint32_t*>(&h[1]);
+            packed.z = *reinterpret_cast<const uint32_t*>(&h[2]);
+            packed.w = *reinterpret_cast<const uint32_t*>(&h[3]);
+            *reinterpret_cast<uint4*>(flowmap + out) = packed;
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (x + k < W) flowmap[out + k] = h[k];
+          }
         }
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) t[r][k] = z;
       }
     }
-    const int qy = 2 * ty + half, gy = (by >> 1) + qy;
+    const int qy = HALVES * ty + half, gy = (by >> 1) + qy;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const float4 a = t[0][2 * j], c0 = t[0][2 * j + 1], c = t[1][2 * j], e = t[1][2 * j + 1];
@@ -350,7 +391,7 @@ __global__ void __launch_bounds__(256)
   // levels 2 .. m.n, unrolled so that every level index is a constant (an
   // indexed kernel parameter would be copied to local memory)
 #pragma unroll
-  for (int l = 1; l < kMipFused; ++l) {
+  for (int l = 1; l < LEVELS; ++l) {
     if (l >= m.n) break;  // the same for every thread
     const int side = Q >> (l - 1), half = side / 2;
     const float4* in = buf[(l - 1) & 1];
@@ -372,6 +413,22 @@ __global__ void __launch_bounds__(256)
 
 dim3 grid2d(int w, int h) { return dim3((w + 31) / 32, (h + 7) / 8); }
 
+template <class... P, class... A>
+cudaError_t launch(void (*fn)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+  const cudaError_t e = launch_after_previous(fn, grid, block, s, args...);
+  count_launch();
+  return e;
+}
+
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    return cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? v : 1;
+  }();
+  return n;
+}
+
 }  // namespace
 
 // The four-cell kernels need W % 4 == 0 and every caller-owned output on a
@@ -387,25 +444,29 @@ cudaError_t launch_surface(const float* b, const float* d, const float2* v, int 
                     aligned(o.normal, 16) && aligned(o.flow_speed, 16) && aligned(o.foam, 16) &&
                     aligned(o.dry, 4);
   if (wide)
-    surface_kernel4<<<grid2d(W / 4, H), dim3(32, 8), 0, s>>>(b, d, v, W, H, pitch, o);
-  else
-    surface_kernel<<<grid2d(W, H), dim3(32, 8), 0, s>>>(b, d, v, W, H, pitch, o);
-  count_launch();
-  return cudaGetLastError();
+    return launch(surface_kernel4, grid2d(W / 4, H), dim3(32, 8), s, b, d, v, W, H, pitch, o);
+  return launch(surface_kernel, grid2d(W, H), dim3(32, 8), s, b, d, v, W, H, pitch, o);
 }
 
 cudaError_t launch_export(const float* b, const float* d, const float2* v, int W, int H,
                           int pitch, float* terrain_rgba, uint16_t* flowmap, int mip_levels,
                           float* mips, cudaStream_t s) {
   const bool wide = W % 4 == 0 && aligned(terrain_rgba, 16) && aligned(flowmap, 16);
-  // with mips, the first level comes out of the same pass (even heights)
-  const bool fuse_mip1 = wide && terrain_rgba && mips && mip_levels >= 1 && H % 2 == 0;
+  // with mips, the first levels come out of the same pass
+  const bool fuse_mip1 = terrain_rgba && mips && mip_levels >= 1;
   MipLevels fused{};
   if (fuse_mip1) {
     // the export and up to six mip levels in one pass
     float4* p = reinterpret_cast<float4*>(mips);
     int w = W, h = H;
-    while (fused.n < kMipFused && fused.n < mip_levels && w >= 2 && h >= 2) {
+    // Blocks of 32 cells where those of 64 are less than four per SM (a wave of them
+    // leaves SMs idle).  Export with all levels, us, before (64-cell blocks for even
+    // heights and widths of whole quads, 16-byte stores, no early launches) and
+    // now: 1024^2 16.5, 8.0; 1021 x 763 19.9, 9.9; 2048^2 40.6, 34.1; 4096^2
+    // 124.6, 109.7 (0.93 of the copy rate).
+    const bool small = (long long)((W + 63) / 64) * ((H + 63) / 64) < 4LL * sm_count();
+    const int most = small ? kMipFused - 1 : kMipFused;
+    while (fused.n < most && fused.n < mip_levels && w >= 2 && h >= 2) {
       w /= 2;
       h /= 2;
       fused.dst[fused.n] = p;
@@ -414,25 +475,24 @@ cudaError_t launch_export(const float* b, const float* d, const float2* v, int W
       p += (size_t)w * h;
       ++fused.n;
     }
-    export_mips_kernel4<<<dim3((W + 63) / 64, (H + 63) / 64), 256, 0, s>>>(
-        b, d, v, W, H, pitch, reinterpret_cast<float4*>(terrain_rgba),
-        reinterpret_cast<__half2*>(flowmap), fused);
-    count_launch();
+    const bool whole = wide && aligned(terrain_rgba, 32);
+    auto fn = small ? (whole ? export_mips_kernel4<16, true> : export_mips_kernel4<16, false>)
+                    : (whole ? export_mips_kernel4<32, true> : export_mips_kernel4<32, false>);
+    const int side = small ? 32 : 64;
+    launch(fn, dim3((W + side - 1) / side, (H + side - 1) / side), dim3(small ? 128 : 256), s, b, d,
+           v, W, H, pitch, reinterpret_cast<float4*>(terrain_rgba),
+           reinterpret_cast<__half2*>(flowmap), fused);
   } else if (wide && (flowmap || terrain_rgba)) {
-    export_kernel4<<<grid2d(W / 4, H), dim3(32, 8), 0, s>>>(
-        b, d, v, W, H, pitch, reinterpret_cast<float4*>(terrain_rgba),
-        reinterpret_cast<__half2*>(flowmap));
-    count_launch();
+    launch(export_kernel4, grid2d(W / 4, H), dim3(32, 8), s, b, d, v, W, H, pitch,
+           reinterpret_cast<float4*>(terrain_rgba), reinterpret_cast<__half2*>(flowmap));
   } else {
     if (flowmap) {
-      flowmap_kernel<<<grid2d(W, H), dim3(32, 8), 0, s>>>(v, W, H, pitch,
-                                                           reinterpret_cast<__half2*>(flowmap));
-      count_launch();
+      launch(flowmap_kernel, grid2d(W, H), dim3(32, 8), s, v, W, H, pitch,
+             reinterpret_cast<__half2*>(flowmap));
     }
     if (terrain_rgba) {
-      terrain_rgba_kernel<<<grid2d(W, H), dim3(32, 8), 0, s>>>(
-          b, d, W, H, pitch, reinterpret_cast<float4*>(terrain_rgba));
-      count_launch();
+      launch(terrain_rgba_kernel, grid2d(W, H), dim3(32, 8), s, b, d, W, H, pitch,
+             reinterpret_cast<float4*>(terrain_rgba));
     }
   }
   if (terrain_rgba && mips) {
@@ -462,8 +522,7 @@ cudaError_t launch_export(const float* b, const float* d, const float2* v, int W
         ++c.n;
       }
       const dim3 grid((sw + kMipBlock - 1) / kMipBlock, (sh + kMipBlock - 1) / kMipBlock);
-      mip_chain_kernel<<<grid, 256, 0, s>>>(src, sw, sh, c);
-      count_launch();
+      launch(mip_chain_kernel, grid, dim3(256), s, src, sw, sh, c);
       src = c.dst[c.n - 1];
       sw = c.w[c.n - 1];
       sh = c.h[c.n - 1];

@@ -113,7 +113,8 @@ constexpr long long kDefaultWaitCycles = 4000000000LL;
 // Host helpers implemented in tws_step.cu.
 int step_variant_count();
 const StepVariant& step_variant(int i);
-int step_variant_for(int k, int flux_storage);
+constexpr long long kSmallStepCells = 4LL << 20;
+int step_variant_for(int k, int flux_storage, long long cells);
 // The automatic choice for grids of at least kLargeGridCells cells (FP16
 // flux: kLargeF16Cells), or -1.
 constexpr long long kLargeGridCells = 12LL << 20;
@@ -218,6 +219,23 @@ cudaError_t launch_export(const float* b, const float* d, const float2* v, int W
                           float* mips, cudaStream_t s);
 
 DevSource make_dev_source(const tws_source& s);
+// A launch that may be scheduled while the one before it on the stream finishes:
+// the kernel waits for that one itself (griddepcontrol.wait) before it touches
+// memory.
+template <class... P, class... A>
+cudaError_t launch_after_previous(void (*fn)(P...), dim3 grid, dim3 block, cudaStream_t s,
+                                  A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
 void count_launch(uint64_t n = 1);
 
 }  // namespace tws

@@ -1007,11 +1007,14 @@ int step_variant_large_grid(int flux_storage, int W, int H) {
   return pick;
 }
 
-int step_variant_for(int k, int /*flux_storage*/) {
+int step_variant_for(int k, int /*flux_storage*/, long long cells) {
   // Default variant per temporal depth (fastest per depth on 4096^2): the
   // plain 32x32 kernel for K = 1, the unified-layout 32x32 tiles for K > 1.
+  // One step on a smaller grid takes 32x16 tiles, twice as many CTAs (us per
+  // launch, FP32, against 32x32): 256^2 4.1 (5.8), 512^2 5.1 (6.4), 1024^2 10.6
+  // (11.1), 2048^2 39.5 (39.9).
   switch (k) {
-    case 1: return 0;
+    case 1: return cells < kSmallStepCells ? 5 : 0;
     case 2: return 16;
     case 3: return 18;
     case 4: return 20;
