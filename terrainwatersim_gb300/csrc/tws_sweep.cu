@@ -336,8 +336,10 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
       }
       const Quad hc = s + 1 < K ? add4(dc, read_b(t - 2 * s - 1)) : h_c;
       if (s + 1 == K) h_c = h_in;
-      const Quad qm = Qm[s], qp = prod4(sub4(hc, h_in), ka2, nz2);
-      Qm[s] = qp;
+      // (the old value of what a level carries is used up before the new one is
+      // formed, here and below, which saves moves)
+      const Quad w_in = sub4(prod4(f_in.w, kf2, nz2), Qm[s]);
+      Qm[s] = prod4(sub4(hc, h_in), ka2, nz2);
       // Rows above the band's first needed outflow row of this level (its
       // windows are filling): nothing below this level is needed either.
       if (t < 4 * s + 2) break;
@@ -357,8 +359,8 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
       const float4 fy = un4(prod4(f_in.y, kf2, nz2));
       nf.y = pk4(max0_fast(fsub(fy.x, ql)), max0_fast(fsub(fy.y, q4.x)),
                  max0_fast(fsub(fy.z, q4.y)), max0_fast(fsub(fy.w, q4.z)));
-      nf.z = max0q(add4(prod4(f_in.z, kf2, nz2), qp));
-      nf.w = max0q(sub4(prod4(f_in.w, kf2, nz2), qm));
+      nf.z = max0q(add4(prod4(f_in.z, kf2, nz2), Qm[s]));
+      nf.w = max0q(w_in);
       if constexpr (!INTERIOR) {
         // Only what cells on the grid read of cells off it has to be zero:
         // the +x outflow of column -1, the -x outflow of column W, the +y
@@ -374,14 +376,13 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
         nf.y = pk4(gx >= W || (closed && gx == 0) ? 0.0f : oy.x, gx + 1 >= W ? 0.0f : oy.y,
                    gx + 2 >= W ? 0.0f : oy.z, gx + 3 >= W ? 0.0f : oy.w);
       }
-      Quad out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
       {
-        const Quad sc = outflow_factors(out, dc, cc2, ncc2, nz2);
+        const Quad sum = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
+        const Quad sc = outflow_factors(sum, dc, cc2, ncc2, nz2);
         nf.x = prod4(nf.x, sc, nz2);
         nf.y = prod4(nf.y, sc, nz2);
         nf.z = prod4(nf.z, sc, nz2);
         nf.w = prod4(nf.w, sc, nz2);
-        if constexpr (!F16) out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
       }
       if constexpr (F16) {
         auto quant = [&](Quad& v) {
@@ -396,7 +397,6 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
         quant(nf.z);
         quant(nf.w);
       }
-      if constexpr (F16) out = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
 
       // the outflows of row ys - 2 are level s + 1's input; row ys takes
       // their slot
@@ -421,7 +421,7 @@ __device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __res
       const float X1r = __shfl_down_sync(0xffffffffu, ny.x, 1);
       const float X0l = __shfl_up_sync(0xffffffffu, nx.w, 1);
       InX[s] = pk4(fadd(ny.y, X0l), fadd(ny.z, nx.x), fadd(ny.w, nx.y), fadd(X1r, nx.z));
-      Out[s] = out;
+      Out[s] = add4(add4(add4(nf.x, nf.y), nf.z), nf.w);
 
       const int yd = ys - 1;
       if (s + 1 < K) {
