@@ -61,7 +61,7 @@ struct tws_grid {
   double* vol_out = nullptr;
   double vol_host[1] = {0.0};
   int* err = nullptr;     // device error word
-  int* queue = nullptr;   // the sweep kernel's work queue (two ints, zero between launches)
+  int* queue = nullptr;   // the sweep kernel's work queues (three ints, zero between launches)
   unsigned long long* ranges = nullptr;  // and its warps' unclaimed rows (empty between launches)
   int err_host[1] = {0};
   CUtensorMap* desc = nullptr;  // device copies of the maps, 5 per variant (batched kernel)
@@ -143,7 +143,7 @@ float pick_flux_scale(float d_max, float c) {
   return std::ldexp(1.0f, std::max(-24, std::min(24, e)));
 }
 
-// The error word, the sweep kernel's queue (at byte 16) and its ranges (at 64).
+// The error word, the sweep kernel's queues (at byte 16) and its ranges (at 64).
 constexpr size_t kScratchBytes = 64 + sizeof(unsigned long long) * kSweepMaxWarps;
 
 VariantMaps* maps_for(tws_grid* g, int variant, std::string* why) {

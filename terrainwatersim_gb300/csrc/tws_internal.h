@@ -39,8 +39,9 @@ struct StepArgs {
   int* err;              // device error word (bounded-wait time-outs)
   long long wait_cycles; // bounded waits give up after this many SM clocks
   int drop_loads;        // test hook: tile loads arm their barrier but issue no copy
-  int* queue;            // the sweep kernel's work queue: next unit, warps done (zero
-                         // between launches; the last warp of a launch resets it)
+  int* queue;            // the sweep kernel's work queues: next border unit, warps done,
+                         // next inner unit (zero between launches; the last warp of a
+                         // launch resets them)
   unsigned long long* ranges;  // the sweep kernel's unclaimed rows, one word per resident
                          // warp (empty between launches)
 };
@@ -117,8 +118,8 @@ constexpr long long kSmallStepCells = 4LL << 20;
 int step_variant_for(int k, int flux_storage, long long cells);
 // The automatic choice for grids of at least kLargeGridCells cells (FP16
 // flux: kLargeF16Cells), or -1.
-constexpr long long kLargeGridCells = 12LL << 20;
-constexpr long long kLargeF16Cells = 32LL << 20;
+constexpr long long kLargeGridCells = 5LL << 20;
+constexpr long long kLargeF16Cells = 17LL << 20;
 int step_variant_large_grid(int flux_storage, int W, int H);
 // Tile variants read through the tensor maps, stream variants through the
 // raw pointers (b, d, f of the current state).

@@ -974,16 +974,18 @@ int step_variant_count() { return table().n; }
 const StepVariant& step_variant(int i) { return table().e[i].v; }
 
 int step_variant_large_grid(int flux_storage, int W, int H) {
-  // The three-step row sweep: FP32 flux from kLargeGridCells on (4096^2: 256
-  // Gcell-steps/s against 192 for the two-step tiles), FP16 flux from
-  // kLargeF16Cells on.  The band height is the tallest rung of a ladder that
-  // leaves at least 2.5 column-unit bands per resident warp of a 16-warp SM
-  // (8192^2: 310 with 192/48 rows, 305 with uniform bands of 64 to 192;
-  // 16384^2: 337 with 256/64, 320 uniform).
+  // The three-step row sweep: FP32 flux from kLargeGridCells on (Gcell-steps/s
+  // with a rain disk, against the two-step tiles: 2048^2 167 (168), 2300^2 189
+  // (174), 2896^2 223 (183), 4096^2 268 (192)), FP16 flux from kLargeF16Cells
+  // on (4608^2 249 (202), 5120^2 259 (204); 4096^2, 238 (200), keeps the two-step
+  // tiles that callers of that size have as their default).  The band height is the tallest rung of a ladder that leaves at least
+  // 2.5 column-unit bands per resident warp of a 16-warp SM (8192^2: 315 with
+  // 192/48 rows, 305 with uniform bands of 64 to 192; 16384^2: 339 with 256/64,
+  // 320 uniform).
   const long long cells = (long long)W * H;
   if (cells < kLargeGridCells) return -1;
   if (flux_storage != TWS_FLUX_F32 && cells < kLargeF16Cells) return -1;
-  static const int kLadder[][2] = {{40, 0}, {80, 32}, {128, 48}, {192, 48}, {256, 64}};
+  static const int kLadder[][2] = {{32, 0}, {40, 0}, {80, 32}, {128, 48}, {192, 48}, {256, 64}};
   static const int sms = [] {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);

@@ -37,20 +37,22 @@
 //   (12 warps of 3 KB in flight cover the latency).  Cells off the grid are
 //   zero-filled by the copy itself (the shaders' out-of-range image loads
 //   read zero).  cp.async.wait_group and a warp barrier hand a row over.
-// * The warps are persistent and take (strip, band) units from a per-grid
-//   queue, border units first.  A warp that finds the queue empty takes over
-//   half of the rows that another has not begun (range_pack below), so units
-//   under rain, at the border or on shores, which take longer, do not hold
-//   the launch up.
+// * The warps are persistent and take (strip, band) units from two per-grid
+//   queues, border units and inner ones (sweep_next below).  A warp that finds
+//   them empty takes over half of the rows that another has not begun
+//   (range_pack below), so units under rain, at the border or on shores, which
+//   take longer, do not hold the launch up.
 //
 // HBM traffic per launch: the state once in, once out (52 B per cell for FP32
 // flux, 36 B for FP16), plus what L2 does not catch of the overlaps.
 //
 // Measured (CUDA events, Gcell-steps/s on moving water with a rain disk, K = 3;
 // in brackets the two-columns-a-lane kernel with static bands that this
-// replaced): 4096^2 256 (209), 8192^2 311 (250), 16384^2 337 (260), FP16 flux
-// 312 (253).  16384^2 at 337 moves 5.8 TB/s of compulsory bytes, 0.86 of the
-// copy rate.
+// replaced): 4096^2 268 (209), 8192^2 315 (250), 16384^2 339 (260), FP16 flux
+// 320 (253).  16384^2 at 339 moves 5.9 TB/s of compulsory bytes, 0.86 of the
+// copy rate; on smaller grids the halo rows of the bands (4096^2: 84 rows and
+// 12) and the launch's end weigh more, and the scheduler issues in 57% of the
+// cycles (three warps each: fixed-latency waits, shared memory, fetch).
 
 #include <algorithm>
 #include <map>
@@ -74,11 +76,6 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 // cp.async of `bytes` (<= size) from src; the rest of the `size` bytes is zero.
-__device__ __forceinline__ void copy8(void* dst, const void* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(dst)), "l"(src),
-               "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void copy16(void* dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
                "r"(bytes)
@@ -558,6 +555,7 @@ __device__ __forceinline__ void sweep_unit_coords(int i, int S, int B, int& s, i
 // units; tall bands recompute fewer halo rows per output row.
 struct SweepBands {
   int tall, tall_end, tall_count, tail, count;
+  int border_sms;  // SMs whose warps start on the units at the grid's border
 };
 
 // Band i of a partition with a tail: its first row and its height.
@@ -567,8 +565,52 @@ __device__ __forceinline__ void sweep_band(const SweepBands& sb, int H, int i, i
   R = min(tall ? sb.tall : sb.tail, (tall ? sb.tall_end : H) - y0);
 }
 
+// The units at the grid's border come first in the order of sweep_unit_coords.
+__host__ __device__ constexpr int sweep_border_units(int S, int B) {
+  return S < 3 || B < 3 ? S * B : 2 * S + 2 * (B - 2);
+}
+
+// Two queues, the units at a grid's border and the inner ones.  The two are
+// separate code, and warps of both on one SM stall each other on instruction
+// fetch (a border unit then takes 1.6 times an inner one's time, against 1.1
+// among its like), so the warps of `border_sms` SMs start on the border's units
+// and all others on the inner ones; a queue that has run empty hands over to
+// the other.  Words of `queue`: the border's next unit, warps done, the inner
+// units' next.  4096^2 262 -> 268, 2896^2 213 -> 223, 2048^2 140 -> 154
+// Gcell-steps/s against one queue, border first.
+__device__ __forceinline__ int sweep_first_queue(int border_sms) {
+  unsigned smid;
+  asm("mov.u32 %0, %%smid;" : "=r"(smid));
+  return (int)smid < border_sms ? 0 : 1;
+}
+__device__ __forceinline__ int sweep_next(int* queue, int border, int total, int& which,
+                                          int& queues, int lane) {
+  while (queues > 0) {
+    int u = 0;
+    if (lane == 0) u = atomicAdd(&queue[2 * which], 1);
+    u = __shfl_sync(0xffffffffu, u, 0) + (which ? border : 0);
+    if (u < (which ? total : border)) return u;
+    which ^= 1;
+    --queues;
+  }
+  return -1;
+}
+
+// The last warp to finish resets the queues for the next launch: every other
+// warp has made its final claim by then, and the next launch reads them only
+// after this grid has completed.
+__device__ __forceinline__ void sweep_done(int* queue, int lane) {
+  if (lane == 0) {
+    __threadfence();
+    if (atomicAdd(&queue[1], 1) == (int)(gridDim.x * kSweepWarps) - 1) {
+      queue[0] = queue[1] = queue[2] = 0;
+      __threadfence();
+    }
+  }
+}
+
 // Persistent warps (one wave): each takes units (strip, band) from the grid's
-// queue until none is left, so warps that drew cheap units take more of them.
+// queues until none is left, so warps that drew cheap units take more of them.
 template <int K, bool F16>
 __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
     sweep_kernel(const float* __restrict__ b, const float* __restrict__ d,
@@ -590,23 +632,20 @@ __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
   const int warps = gridDim.x * kSweepWarps, me = blockIdx.x * kSweepWarps + warp;
   unsigned long long* const word = a.ranges + me;
   uint32_t seed = (uint32_t)me;
-  bool queued = true;
+  const int border = sweep_border_units(strips, bands);
+  int which = sweep_first_queue(sb.border_sms), queues = 2;
   for (;;) {
     int si = 0, y0 = 0, y1 = 0;
+    const int u = sweep_next(a.queue, border, total, which, queues, lane);
+    const bool queued = u >= 0;
     if (queued) {
-      int u = 0;
-      if (lane == 0) u = atomicAdd(&a.queue[0], 1);
-      u = __shfl_sync(0xffffffffu, u, 0);
-      queued = u < total;
-      if (queued) {
-        int bi, R;
-        sweep_unit_coords(u, strips, bands, si, bi);
-        sweep_band(sb, a.H, bi, y0, R);
-        y1 = y0 + R;
-      }
+      int bi, R;
+      sweep_unit_coords(u, strips, bands, si, bi);
+      sweep_band(sb, a.H, bi, y0, R);
+      y1 = y0 + R;
     }
     if (!queued) {
-      // the queue is empty: the largest of 64 other warps' ranges, its back half
+      // the queues are empty: the largest of 64 other warps' ranges, its back half
       bool got = false;
       for (int attempt = 0; attempt < kSweepStealTries && !got; ++attempt) {
         seed = seed * 1664525u + 1013904223u;  // (Numerical Recipes' generator)
@@ -664,17 +703,7 @@ __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
       sweep_unit<K, F16, false>(a, b, d, f, a.d_out, a.f_out, a.v_out, ring, xs, y0, R, mask,
                                 share ? word : nullptr);
   }
-  // The last warp to finish resets the queue for the next launch: every other
-  // warp has made its final claim by then, and the next launch reads the
-  // queue only after this grid has completed.
-  if (lane == 0) {
-    __threadfence();
-    if (atomicAdd(&a.queue[1], 1) == (int)(gridDim.x * kSweepWarps) - 1) {
-      a.queue[0] = 0;
-      a.queue[1] = 0;
-      __threadfence();
-    }
-  }
+  sweep_done(a.queue, lane);
 }
 
 template <int K>
@@ -683,24 +712,16 @@ const void* sweep_fn(int flux_storage) {
                                       : reinterpret_cast<const void*>(&sweep_kernel<K, false>);
 }
 
-}  // namespace
-
-size_t sweep_smem_bytes(int k, int flux_storage) {
-  return (size_t)kSweepWarps * sweep_warp_bytes(k, flux_storage == TWS_FLUX_F16);
+// SMs that start on `border` of `units` units: their share of the work, a border
+// unit counted as kBorderCost inner ones.
+constexpr double kBorderCost = 1.2;
+int sweep_border_sms(long long border, long long units, int sms) {
+  const double w = kBorderCost * (double)border;
+  return units > 0 ? (int)(w / (w + (double)(units - border)) * sms + 0.5) : 0;
 }
 
-cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, const float* b,
-                              const float* d, const void* f, const StepArgs& a, cudaStream_t s) {
-  const void* fn = nullptr;
-  switch (k) {
-    case 2: fn = sweep_fn<2>(flux_storage); break;
-    case 3: fn = sweep_fn<3>(flux_storage); break;
-    case 4: fn = sweep_fn<4>(flux_storage); break;
-    default: return cudaErrorInvalidValue;
-  }
-  if (rows < 1 || tail_rows < 0 || !a.queue || !a.ranges) return cudaErrorInvalidValue;
-  const size_t smem = sweep_smem_bytes(k, flux_storage);
-  // one wave of persistent CTAs (occupancy of this instantiation, queried once)
+// One wave of persistent CTAs of a kernel (its occupancy, queried once).
+cudaError_t sweep_ctas(const void* fn, size_t smem, long long* ctas, int* sm_count) {
   static std::mutex mu;
   static std::map<const void*, int> resident;
   int per_sm = 0, sms = 0;
@@ -723,12 +744,52 @@ cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, 
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
     sms = 1;
+  *sm_count = sms;
+  *ctas = std::min<long long>((long long)per_sm * sms, kSweepMaxWarps / kSweepWarps);
+  return cudaSuccess;
+}
+
+// A launch that may begin while the previous one on the stream ends.
+cudaLaunchConfig_t sweep_config(long long blocks, size_t smem, cudaStream_t s,
+                                cudaLaunchAttribute* attr) {
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(kSweepThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+}  // namespace
+
+size_t sweep_smem_bytes(int k, int flux_storage) {
+  return (size_t)kSweepWarps * sweep_warp_bytes(k, flux_storage == TWS_FLUX_F16);
+}
+
+cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, const float* b,
+                              const float* d, const void* f, const StepArgs& a, cudaStream_t s) {
+  const void* fn = nullptr;
+  switch (k) {
+    case 2: fn = sweep_fn<2>(flux_storage); break;
+    case 3: fn = sweep_fn<3>(flux_storage); break;
+    case 4: fn = sweep_fn<4>(flux_storage); break;
+    default: return cudaErrorInvalidValue;
+  }
+  if (rows < 1 || tail_rows < 0 || !a.queue || !a.ranges) return cudaErrorInvalidValue;
+  const size_t smem = sweep_smem_bytes(k, flux_storage);
+  long long ctas = 0;
+  int sms = 0;
+  const cudaError_t e0 = sweep_ctas(fn, smem, &ctas, &sms);
+  if (e0 != cudaSuccess) return e0;
   const int valid = kSweepCols - 2 * kSweepHaloX(k);
   const long long strips = (a.W + valid - 1) / valid;
   // Band partition: uniform bands are made taller as long as every resident
   // warp has one; with a tail, about one short unit per resident warp ends the
   // queue (at most half of the rows).
-  const long long ctas = std::min<long long>((long long)per_sm * sms, kSweepMaxWarps / kSweepWarps);
   const long long warps = ctas * kSweepWarps;
   SweepBands sb{};
   sb.tall = rows;
@@ -744,19 +805,12 @@ cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, 
   sb.tall_count = (sb.tall_end + sb.tall - 1) / sb.tall;
   sb.count = sb.tall_count + (int)tail_bands;
   const long long units = strips * sb.count;
+  sb.border_sms = sweep_border_sms(sweep_border_units((int)strips, sb.count), units, sms);
   if (units > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   // four warps per unit where there are few units: the others take over rows
   const long long blocks = std::min(units, ctas);
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)blocks);
-  cfg.blockDim = dim3(kSweepThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  const cudaLaunchConfig_t cfg = sweep_config(blocks, smem, s, attr);
   using Fn = void (*)(const float*, const float*, const void*, StepArgs, SweepBands);
   const cudaError_t e =
       cudaLaunchKernelEx(&cfg, reinterpret_cast<Fn>(const_cast<void*>(fn)), b, d, f, a, sb);

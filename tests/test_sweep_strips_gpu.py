@@ -119,3 +119,24 @@ def test_non_finite_cells_as_the_plain_kernel(tws):
             nan = np.isnan(y)
             assert np.array_equal(nan, np.isnan(x)), vi
             assert np.array_equal(x[~nan].view(np.uint32), y[~nan].view(np.uint32)), vi
+
+
+@pytest.mark.parametrize("size,flux", [((2300, 2290), 0), ((4352, 4100), 1)])
+def test_default_from_its_smallest_grids(tws, size, flux):
+    """The smallest grids that take the three-step sweep unasked (5 Mi cells, FP16
+    flux 17 Mi) against the plain one-step kernel, bit for bit."""
+    W, H = size
+    out = []
+    for variant in (-1, 0):
+        with tws.Grid(W, H, tws.params_physical(boundary=tws.BOUNDARY_OPEN), flux) as g:
+            g.generate_scene(9, 40.0, 15.0)
+            g.set_sources(tws.rain_disks(9, W, H, 40, 0.02, 2))
+            if variant >= 0:
+                g.set_variant(variant)
+            n0 = tws.lib().tws_launch_count()
+            g.step(6)
+            g.sync()
+            out.append((tws.lib().tws_launch_count() - n0, *g.download()))
+    assert (out[0][0], out[1][0]) == (2, 6)
+    for name, x, y in zip(("depth", "flux", "velocity"), out[0][1:], out[1][1:]):
+        np.testing.assert_array_equal(x.view(np.uint8), y.view(np.uint8), name)
