@@ -379,9 +379,12 @@ TWS_API int tws_io_wait(tws_grid* grid);
 TWS_API int tws_get_buffers(tws_grid* grid, tws_buffers* out);
 
 /* ---- batches -----------------------------------------------------------
- * Many grids of different sizes advanced together: one persistent launch per
- * step covers the tiles of every member grid, and chains of 16 steps are
- * replayed from CUDA graphs.  Member grids keep their own buffers,
+ * Many grids of different sizes advanced together: each launch covers the
+ * tiles of every member grid, and chains of up to 16 steps (with the row sweep:
+ * 16 launches) are replayed from CUDA graphs.  A batch whose variant has not
+ * been set takes the row sweep, three steps per launch, where its members are
+ * large enough together (FP32 flux: 6 Mi cells, FP16: 24 Mi) and fill their
+ * strips, and the two-step tiles otherwise; the results are the same.  Member grids keep their own buffers,
  * parameters and sources; while in a batch their work is ordered on the
  * batch's stream.  Grids can join and leave between calls (continuous
  * batching); each call advances every member by its own step count.  No
@@ -394,7 +397,8 @@ TWS_API int tws_batch_destroy(tws_batch* batch); /* removes the members first */
 TWS_API int tws_batch_add(tws_batch* batch, tws_grid* grid);
 TWS_API int tws_batch_remove(tws_batch* batch, tws_grid* grid);
 TWS_API int tws_batch_size(tws_batch* batch);
-/* Batched kernel variants: K steps per launch and the tile. */
+/* Batched kernel variants: K steps per launch and the tile (the last one, the
+ * row sweep: a strip's columns by the least rows of a band). */
 TWS_API int tws_batch_variant_count(void);
 TWS_API int tws_batch_variant_info(int variant, int* steps_per_launch, int* tile_x, int* tile_y);
 TWS_API int tws_batch_set_variant(tws_batch* batch, int variant);

@@ -1205,6 +1205,8 @@ TWS_API int tws_sync(tws_grid* g) {
 
 namespace {
 constexpr int kChainSteps = 16;
+constexpr int kBatchOneStepVariant = 0;
+static_assert(kChainSteps <= kBatchSweepMaxLaunches);
 }
 
 struct tws_batch {
@@ -1213,6 +1215,7 @@ struct tws_batch {
   bool own_stream = false;
   std::vector<tws_grid*> grids;
   int variant = batch_variant_default();  // batched kernel variant
+  bool pinned = false;  // set by the caller or the autotuner: no choice by size
   bool use_graphs = true;
   int cap = 0;   // table capacity (grids)
   int ucap = 0;  // unit table capacity
@@ -1232,7 +1235,9 @@ struct tws_batch {
   };
   std::vector<Graph> graphs;
   uint64_t chains = 0, graph_launches = 0;
-  int* d_err = nullptr;  // one device error word for every member while batched
+  // one device error word for every member while batched, the sweep's queue
+  // (at byte 16) and its ranges (at 64), as in a grid's scratch
+  int* d_err = nullptr;
   int uploaded_variant = -1;  // variant whose unit table the device holds
   int h_err = 0;
   std::string last_error;
@@ -1325,8 +1330,14 @@ int ensure_units(tws_batch* b, int n) {
 
 int run_launches(tws_batch* b, int variant, int launches, int blocks) {
   for (int i = 0; i < launches; ++i) {
+    unsigned char* scratch = reinterpret_cast<unsigned char*>(b->d_err);
     cudaError_t e =
-        launch_batch_step(variant, b->flux_storage, b->d_grids, b->d_units, i, blocks, b->stream);
+        variant == batch_variant_sweep()
+            ? launch_batch_sweep(b->flux_storage, b->d_grids, b->d_units, blocks, i,
+                                 reinterpret_cast<int*>(scratch + 16),
+                                 reinterpret_cast<unsigned long long*>(scratch + 64), b->stream)
+            : launch_batch_step(variant, b->flux_storage, b->d_grids, b->d_units, i, blocks,
+                                b->stream);
     if (e != cudaSuccess) return bfail(b, TWS_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
   }
   return TWS_OK;
@@ -1374,14 +1385,42 @@ cudaGraphExec_t graph_for(tws_batch* b, int variant, int launches, int blocks) {
   return exec;
 }
 
+// Rows per band of a sweep over the members with launches in this chain: the
+// fewest that give every resident warp at most one unit, so that a launch is one
+// wave (a band recomputes about 4K rows of halo; the rows that a slow unit has
+// not begun are taken over).  Members too large for that: bands of 128 rows
+// (halo 9%), several to a warp.
+int sweep_band_rows(const tws_batch* b, const std::vector<int>& launches, int warps) {
+  const int cols = batch_sweep_columns();
+  constexpr int kTall = 128;
+  for (int rows = kBatchSweepMinRows; rows < kTall; rows += std::max(1, rows / 16)) {
+    long long units = 0;
+    for (size_t i = 0; i < launches.size(); ++i)
+      if (launches[i] > 0) {
+        const tws_grid* g = b->grids[i];
+        units += (long long)((g->W + cols - 1) / cols) * ((g->H + rows - 1) / rows);
+      }
+    if (units <= warps) return rows;
+  }
+  return kTall;
+}
+
 // One chain: grid i takes launches[i] launches of `variant` (K steps each).
 int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
   int k, tx, ty, sv;
   batch_variant_info(variant, &k, &tx, &ty, &sv);
+  const bool sweep = sv < 0;
   const int n = (int)b->grids.size();
   int rc = ensure_capacity(b, n);
   if (rc != TWS_OK) return rc;
-  int units = 0, m = 0, max_l = 0;
+  int sms = 0;
+  if (sweep) {
+    int warps = 0;
+    if (batch_sweep_warps(b->flux_storage, &warps, &sms) != cudaSuccess)
+      return bfail(b, TWS_ERR_CUDA, "batched sweep occupancy");
+    ty = sweep_band_rows(b, launches, warps);
+  }
+  int units = sweep ? 1 : 0, m = 0, max_l = 0;  // (a sweep's table begins with its counts)
   for (int i = 0; i < n; ++i) {
     if (launches[i] <= 0) continue;
     const tws_grid* g = b->grids[i];
@@ -1391,6 +1430,8 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
   }
   if (m == 0) return TWS_OK;
   const int blocks = launch_blocks(units);  // a power of two, so graphs stay reusable
+  if (sweep && blocks > kSweepMaxUnits)
+    return bfail(b, TWS_ERR_UNSUPPORTED, "too many units for the batched row sweep");
   rc = ensure_units(b, blocks);
   if (rc != TWS_OK) return rc;
   // wait until the copy that last read this staging slot has completed
@@ -1401,15 +1442,15 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
   BatchUnit* hu = b->h_units[s];
   std::string why;
   m = 0;
-  int u = 0;
+  int u = sweep ? 1 : 0, border = 0;
   for (int i = 0; i < n; ++i) {
     if (launches[i] <= 0) continue;
     tws_grid* g = b->grids[i];
     BatchGrid& e = hg[m];
     std::memset(&e, 0, sizeof(e));  // padding too, so equal tables compare equal
-    VariantMaps* maps = maps_for(g, sv, &why);
-    if (!maps) return bfail(b, TWS_ERR_CUDA, why);
-    if (!maps->on_device) {
+    VariantMaps* maps = sweep ? nullptr : maps_for(g, sv, &why);
+    if (!sweep && !maps) return bfail(b, TWS_ERR_CUDA, why);
+    if (maps && !maps->on_device) {
       // written once per (grid, variant); the first chain's CTAs fence them
       CUtensorMap five[5] = {maps->b, maps->d[0], maps->d[1], maps->f[0], maps->f[1]};
       if (cudaMemcpyAsync(g->desc + 5 * sv, five, sizeof(five), cudaMemcpyHostToDevice,
@@ -1418,11 +1459,14 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
       maps->on_device = true;
       maps->fresh = true;
     }
-    e.tm = g->desc + 5 * sv;
-    e.fence = maps->fresh ? 1 : 0;
-    maps->fresh = false;
+    if (maps) {
+      e.tm = g->desc + 5 * sv;
+      e.fence = maps->fresh ? 1 : 0;
+      maps->fresh = false;
+    }
     e.a = make_step_args(g);
     e.a.err = b->d_err;
+    e.b = g->b;
     e.d[0] = g->d[0];
     e.d[1] = g->d[1];
     e.f[0] = g->f[0];
@@ -1437,23 +1481,29 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
   // one of the two code paths (the edge path is separate code, and mixing
   // the two stalled the schedulers on instruction fetch).  Interior is the
   // kernel's test: the tile's b/d box (halo 2K rounded up to 4 in x, 2K in y)
-  // lies inside the grid.
+  // lies inside the grid.  A sweep takes the edge units, the slower ones, first;
+  // its bands are a member's rows in equal parts.
   const int hx = (2 * k + 3) / 4 * 4, hy = 2 * k;
   for (int pass = 0; pass < 2; ++pass) {
     m = 0;
     for (int i = 0; i < n; ++i) {
       if (launches[i] <= 0) continue;
       const tws_grid* g = b->grids[i];
-      const int meta = launches[i] | (g->cur << 30);
-      for (int y0 = 0; y0 < g->H; y0 += ty)
+      const int bands = (g->H + ty - 1) / ty;
+      const int rows = sweep ? (g->H + bands - 1) / bands : ty;
+      const int meta = sweep ? batch_sweep_meta(launches[i], rows, g->cur)
+                             : launches[i] | (g->cur << 30);
+      for (int y0 = 0; y0 < g->H; y0 += rows)
         for (int x0 = 0; x0 < g->W; x0 += tx) {
           const bool interior = x0 - hx >= 0 && y0 - hy >= 0 && x0 + tx + hx <= g->W &&
-                                y0 + ty + hy <= g->H;
-          if (interior == (pass == 0)) hu[u++] = BatchUnit{m, x0, y0, meta};
+                                y0 + rows + hy <= g->H;
+          if (interior == (pass == (sweep ? 1 : 0))) hu[u++] = BatchUnit{m, x0, y0, meta};
         }
       ++m;
     }
+    if (pass == 0) border = u - 1;
   }
+  if (sweep) hu[0] = BatchUnit{border, u - 1, sweep_border_sms(border, u - 1, sms), 0};
   for (; u < blocks; ++u) hu[u] = BatchUnit{0, 0, 0, 0};  // CTAs past the units return
   // Upload the table unless it equals the one the device already holds (the
   // same members, launch counts and parity: consecutive chains of a steady
@@ -1497,41 +1547,68 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
   return TWS_OK;
 }
 
-// Advance member i by steps[i] steps (chains of up to kChainSteps).
-int batch_advance(tws_batch* b, std::vector<int> left) {
+// Whether a batch that was given no variant takes the row sweep: three steps a
+// launch, and no more than 1.15 times the cells of the 32 x 32 tiles once both are
+// rounded up to whole strips and tiles (2000 x 64^2, 1.75 times: 5088 us against
+// 4544; 64 x 450 x 350, 1.16 times: 3405 against 3322; 500 x 130^2, 1.14 times:
+// 4008 against 4408).
+bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  const int cols = batch_sweep_columns();
+  long long cells = 0, strips = 0, tiles = 0, units = 0;
+  for (size_t i = 0; i < steps.size(); ++i) {
+    if (steps[i] < kBatchSweepK) continue;
+    const long long W = b->grids[i]->W, H = b->grids[i]->H, s = (W + cols - 1) / cols;
+    cells += W * H;
+    strips += s * cols * H;
+    tiles += (W + 31) / 32 * 32 * ((H + 31) / 32 * 32);
+    units += s * ((H + kBatchSweepMinRows - 1) / kBatchSweepMinRows);
+  }
+  return units < kSweepMaxUnits / 2 && 20 * strips <= 23 * tiles &&
+         cells >= (b->flux_storage == TWS_FLUX_F16 ? kBatchSweepF16Cells : kBatchSweepCells);
+}
+
+// Advance member i by steps[i] steps, in chains of up to kChainSteps steps (of
+// as many launches, where the sweep runs).
+int batch_advance(tws_batch* b, const std::vector<int>& steps) {
+  const bool sweep = b->pinned ? b->variant == batch_variant_sweep() : sweep_is_faster(b, steps);
+  const int variant = sweep ? batch_variant_sweep() : b->variant;
   int k;
-  batch_variant_info(b->variant, &k, nullptr, nullptr, nullptr);
+  batch_variant_info(variant, &k, nullptr, nullptr, nullptr);
   const int n = (int)b->grids.size();
-  const int per_chain = std::max(1, kChainSteps / k);  // launches per chain
-  std::vector<int> launches(n);
+  if (n == 0) return TWS_OK;
+  const int per_chain = sweep ? kChainSteps : std::max(1, kChainSteps / k);  // launches per chain
+  // Launches of `variant`, then of the two-step tiles, then of the one-step
+  // kernel.  Where three steps a launch leave one over, the last four go as two
+  // and two.
+  std::vector<int> left(n), two(n, 0), one(n, 0), launches(n);
+  for (int i = 0; i < n; ++i) {
+    left[i] = steps[i] / k;
+    const int rest = steps[i] % k;
+    if (k == 3 && rest == 1 && left[i] > 0) {
+      --left[i];
+      two[i] = 2;
+    } else if (rest == 2) {
+      two[i] = 1;
+    } else {
+      one[i] = rest;
+    }
+  }
   for (;;) {
-    bool work = false;
-    for (int i = 0; i < n; ++i) {
-      launches[i] = std::min(left[i] / k, per_chain);
-      work |= launches[i] > 0;
-    }
-    if (!work) break;
-    const int rc = run_chain(b, b->variant, launches);
+    for (int i = 0; i < n; ++i) launches[i] = std::min(left[i], per_chain);
+    if (*std::max_element(launches.begin(), launches.end()) <= 0) break;
+    const int rc = run_chain(b, variant, launches);
     if (rc != TWS_OK) return rc;
-    for (int i = 0; i < n; ++i) left[i] -= launches[i] * k;
+    for (int i = 0; i < n; ++i) left[i] -= launches[i];
   }
-  // steps left over when K does not divide a grid's count: one-step launches
-  bool any = false;
-  for (int i = 0; i < n; ++i) any |= left[i] > 0;
-  if (any) {
-    int k1 = -1;
-    for (int v = 0; v < batch_variant_count(); ++v) {
-      int kv;
-      batch_variant_info(v, &kv, nullptr, nullptr, nullptr);
-      if (kv == 1) {
-        k1 = v;
-        break;
-      }
-    }
-    if (k1 < 0) return bfail(b, TWS_ERR_UNSUPPORTED, "no one-step batched variant");
-    return run_chain(b, k1, left);
-  }
-  return TWS_OK;
+  int rc = run_chain(b, batch_variant_default(), two);
+  if (rc == TWS_OK) rc = run_chain(b, kBatchOneStepVariant, one);
+  return rc;
 }
 
 }  // namespace
@@ -1553,8 +1630,8 @@ TWS_API int tws_batch_create(int flux_storage, void* stream, tws_batch** out) {
     }
     b->own_stream = true;
   }
-  if (cudaMalloc(&b->d_err, sizeof(int)) != cudaSuccess ||
-      cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream) != cudaSuccess) {
+  if (cudaMalloc(&b->d_err, kScratchBytes) != cudaSuccess ||
+      cudaMemsetAsync(b->d_err, 0, kScratchBytes, b->stream) != cudaSuccess) {
     cudaGetLastError();
     if (b->own_stream) cudaStreamDestroy(b->stream);
     cudaFree(b->d_err);
@@ -1617,6 +1694,7 @@ TWS_API int tws_batch_set_variant(tws_batch* b, int variant) {
   if (!b || variant < 0 || variant >= batch_variant_count())
     return bfail(b, TWS_ERR_INVALID, "no such batched variant");
   b->variant = variant;
+  b->pinned = true;
   return TWS_OK;
 }
 
@@ -1678,6 +1756,8 @@ TWS_API int tws_batch_autotune(tws_batch* b, int trial_steps, int* chosen) {
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   const int saved_variant = b->variant;
+  const bool saved_pinned = b->pinned;
+  b->pinned = true;
   float best_ms = 1e30f;
   int best = saved_variant, rc = TWS_OK;
   for (int v = 0; v < batch_variant_count() && rc == TWS_OK; ++v) {
@@ -1708,6 +1788,7 @@ TWS_API int tws_batch_autotune(tws_batch* b, int trial_steps, int* chosen) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   b->variant = rc == TWS_OK ? best : saved_variant;
+  b->pinned = rc == TWS_OK || saved_pinned;
   if (chosen) *chosen = b->variant;
   return rc;
 }

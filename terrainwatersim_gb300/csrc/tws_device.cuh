@@ -134,7 +134,9 @@ static __device__ __noinline__ float add_sources(float d, int gx, int gy, const 
 // kernels, where one call per cell sat on a launch's critical path (the warps
 // under a rain disk were the slowest of a launch) and the saved registers
 // around a call would cost the unrolled code around it.
-__device__ __forceinline__ float add_sources_inline(float d, int gx, int gy, const StepArgs& a,
+// A: StepArgs, or what else has nsrc and src.
+template <class A>
+__device__ __forceinline__ float add_sources_inline(float d, int gx, int gy, const A& a,
                                                     uint32_t mask) {
 #pragma unroll 1
   for (int k = 0; k < a.nsrc; ++k) {

@@ -77,6 +77,7 @@ struct alignas(16) BatchGrid {
   int fence;
   int pad0_;
   StepArgs a;     // W, H, pitch, constants, sources, flux scale, error word
+  const float* b;
   float* d[2];
   void* f[2];
   float2* v;
@@ -90,19 +91,49 @@ struct alignas(16) BatchGrid {
 // its grid (index into the BatchGrid table), tile origin, and meta =
 // launches this chain gives the grid | (the grid's buffer parity at the chain
 // start) << 30.  Entries past the chain's units have meta = 0.
+// A unit of a batched sweep: x0 is its strip's first output column, and meta
+// holds the unit's rows as well: launches | rows << 8 | parity << 30.  Its table
+// begins with an entry of counts: units at the members' borders (they come
+// first), all units, SMs that start on the border's.
 struct BatchUnit {
   int grid, x0, y0, meta;
 };
+constexpr int kBatchSweepK = 3;  // steps per launch
+constexpr int kBatchSweepMinRows = 16;
+constexpr int kBatchSweepMaxLaunches = 255;
+__host__ __device__ constexpr int batch_sweep_meta(int launches, int rows, int cur) {
+  return launches | rows << 8 | cur << 30;
+}
+__host__ __device__ constexpr int batch_sweep_launches(int meta) { return meta & 0xff; }
+__host__ __device__ constexpr int batch_sweep_rows(int meta) { return meta >> 8 & 0x3fffff; }
 
 // Batched kernel variants (K steps per launch, tile) and their launcher.
 // Launch `launch_idx` of a chain runs CTA u on units[u] (`blocks` CTAs, at
 // least the chain's units) and advances a grid iff launch_idx < its launches.
 int batch_variant_count();
 int batch_variant_default();  // two steps per launch, unified 32x32 tiles
+int batch_variant_sweep();    // the batched row sweep, three steps per launch
+// A batch without a set variant takes the sweep from this many cells on, where its
+// strips waste little more than the tiles (us for 48 steps, sweep against tiles:
+// 4 x 1024^2 1715 (1314), 6 x 1024^2 1749 (1878), 8 x 1024^2 2217 (2495), 64 x
+// 512^2 4426 (4981), 16 x 2048^2 11116 (17635); FP16 16 x 1024^2 4269 (4414), 64 x
+// 512^2 4946 (4765), 128 x 512^2 8782 (9109), 8 x 2048^2 6730 (8430)).
+constexpr long long kBatchSweepCells = 6LL << 20;
+constexpr long long kBatchSweepF16Cells = 24LL << 20;
 void batch_variant_info(int i, int* k, int* tx, int* ty, int* step_variant);
 cudaError_t prepare_batch_variant(int variant, int flux_storage);  // outside any capture
 cudaError_t launch_batch_step(int variant, int flux_storage, const BatchGrid* grids,
                               const BatchUnit* units, int launch_idx, int blocks, cudaStream_t s);
+// tws_sweep.cu: the batched row sweep.  Its units are strips of
+// batch_sweep_columns() columns in bands of rows; `queue` and `ranges` as in
+// StepArgs, the batch's own.
+int batch_sweep_columns();
+cudaError_t batch_sweep_warps(int flux_storage, int* warps, int* sms);  // resident warps
+cudaError_t launch_batch_sweep(int flux_storage, const BatchGrid* grids, const BatchUnit* units,
+                               int entries, int launch_idx, int* queue,
+                               unsigned long long* ranges, cudaStream_t s);
+// SMs whose warps start on the units at the grids' borders
+int sweep_border_sms(long long border, long long units, int sms);
 
 // Device error codes written to StepArgs::err.
 enum : int { kDevErrNone = 0, kDevErrWaitTimeout = 1 };
@@ -133,6 +164,7 @@ cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, 
                               const float* d, const void* f, const StepArgs& a, cudaStream_t s);
 constexpr int kSweepCtaThreads = 128;  // four warps, each its own sweep
 constexpr int kSweepMaxWarps = 4096;   // warps of a sweep launch (words of StepArgs::ranges)
+constexpr int kSweepMaxUnits = 1 << 22;  // units of a batched sweep (a range word's strip field)
 size_t sweep_smem_bytes(int k, int flux_storage);
 // The column unit that the variant table names a sweep by: 64 columns less their
 // halo.  A warp sweeps two such halves side by side (128 columns).

@@ -1149,7 +1149,8 @@ using BatchFn = void (*)(const BatchGrid*, const BatchUnit*, int);
 
 struct BatchEntry {
   int k, tx, ty, uni;
-  int step_variant;  // the single-grid variant with the same boxes (its tensor maps fit)
+  int step_variant;  // the single-grid variant with the same boxes (its tensor maps fit);
+                     // -1: the row sweep, which reads through plain pointers
   const void* fn[2];
   size_t smem[2];
   int ctas_per_sm[2] = {0, 0};
@@ -1186,6 +1187,12 @@ struct BatchTable {
     e[n++] = make_batch_entry<2, 32, 32, true, 5>(16);
     e[n++] = make_batch_entry<2, 64, 16, true, 5>(17);
     e[n++] = make_batch_entry<3, 32, 32, true, 3>(18);
+    BatchEntry sweep{};  // tws_sweep.cu; a tile is a strip's columns by a band's least rows
+    sweep.k = kBatchSweepK;
+    sweep.tx = batch_sweep_columns();
+    sweep.ty = kBatchSweepMinRows;
+    sweep.step_variant = -1;
+    e[n++] = sweep;
   }
 };
 
@@ -1198,6 +1205,7 @@ BatchTable& batch_table() {
 
 int batch_variant_count() { return batch_table().n; }
 int batch_variant_default() { return 4; }
+int batch_variant_sweep() { return 7; }
 
 void batch_variant_info(int i, int* k, int* tx, int* ty, int* step_variant) {
   const BatchEntry& e = batch_table().e[i];
@@ -1212,6 +1220,10 @@ cudaError_t prepare_batch_variant(int variant, int flux_storage) {
   if (variant < 0 || variant >= t.n) return cudaErrorInvalidValue;
   const int fs = flux_storage == TWS_FLUX_F16 ? TWS_FLUX_F16 : TWS_FLUX_F32;
   BatchEntry& e = t.e[variant];
+  if (e.step_variant < 0) {
+    int warps, sms;
+    return batch_sweep_warps(fs, &warps, &sms);
+  }
   const StepVariant& sv = step_variant(e.step_variant);
   if (sv.k != e.k || sv.tx != e.tx || sv.ty != e.ty || sv.uni != e.uni || sv.stages != 1)
     return cudaErrorInvalidValue;  // the tables disagree: the maps would not fit

@@ -135,8 +135,9 @@ __device__ __forceinline__ int range_cur(unsigned long long w) { return (int)(w 
 __device__ __forceinline__ int range_end(unsigned long long w) { return (int)(w >> 21 & 0x1fffff); }
 __device__ __forceinline__ int range_strip(unsigned long long w) { return (int)(w >> 42); }
 
-template <int K, bool F16, bool INTERIOR>
-__device__ __forceinline__ void sweep_unit(const StepArgs& a, const float* __restrict__ gb,
+// A: StepArgs, or SweepArgs where the arguments come from a batch's table.
+template <int K, bool F16, bool INTERIOR, class A>
+__device__ __forceinline__ void sweep_unit(const A& a, const float* __restrict__ gb,
                                            const float* __restrict__ gd,
                                            const void* __restrict__ gf,
                                            float* __restrict__ d_out, void* __restrict__ f_out,
@@ -706,19 +707,136 @@ __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
   sweep_done(a.queue, lane);
 }
 
+// What a sweep reads of its grid's step arguments, for a grid that a warp of a
+// batch's launch drew: the values in registers, the sources in the batch's table.
+struct SweepArgs {
+  int W, H, pitch;
+  float kf, ka, c;
+  int closed, nsrc;
+  float flux_scale, flux_inv_scale, neg_zero;
+  const DevSource* src;
+};
+
+// The sweep over the units of many grids, from the same two queues; a taker of
+// rows reads which grid they belong to from the unit that they were part of.
+// Bound as the single grid's sweep, with more border: 20 FP32 grids of 128 to
+// 2048 a side, 32 steps, 3440 -> 2660 us against the two-step tiles (a third of
+// the units at borders), 16 of 2048^2, 48 steps, 17635 -> 11100.
+template <int K, bool F16>
+__global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
+    batch_sweep_kernel(const BatchGrid* __restrict__ grids, const BatchUnit* __restrict__ units,
+                       int launch_idx, int* queue, unsigned long long* ranges) {
+  using RG = SweepRing<K, F16>;
+  extern __shared__ __align__(128) unsigned char sweep_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // as in sweep_kernel
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  unsigned char* ring = sweep_smem + warp * RG::WARP;
+  const int warps = gridDim.x * kSweepWarps, me = blockIdx.x * kSweepWarps + warp;
+  unsigned long long* const word = ranges + me;
+  uint32_t seed = (uint32_t)me;
+  // the first entry: how many units there are, at the borders and in all
+  const int4 head = __ldg(reinterpret_cast<const int4*>(units));
+  const int4* const table = reinterpret_cast<const int4*>(units) + 1;
+  int which = sweep_first_queue(head.z), queues = 2;
+  for (;;) {
+    int y0 = 0, y1 = 0;
+    int u = sweep_next(queue, head.x, head.y, which, queues, lane);
+    const bool queued = u >= 0;
+    if (!queued) {
+      // the queues are empty: the largest of 64 other warps' ranges, its back half
+      bool got = false;
+      for (int attempt = 0; attempt < kSweepStealTries && !got; ++attempt) {
+        seed = seed * 1664525u + 1013904223u;  // (Numerical Recipes' generator)
+        const unsigned v = (unsigned)(((unsigned long long)seed * (unsigned)warps) >> 32);
+        unsigned long long w = 0;
+        unsigned best = 0;
+        unsigned victim = 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          unsigned j = v + lane + 32 * i;
+          while (j >= (unsigned)warps) j -= (unsigned)warps;
+          const unsigned long long x = *(volatile unsigned long long*)(ranges + j);
+          const unsigned left = (unsigned)max(0, range_end(x) - range_cur(x));
+          if (left > best) best = left, w = x, victim = j;
+        }
+        const unsigned top = __reduce_max_sync(0xffffffffu, best << 5 | (unsigned)lane);
+        if ((int)(top >> 5) < kSweepMinSteal) continue;
+        const int from = (int)(top & 31u);
+        int mid = 0;
+        if (lane == from) {
+          const int cur = range_cur(w), end = range_end(w);
+          mid = cur + (end - cur + 1) / 2;
+          if (atomicCAS(ranges + victim, w, range_pack(range_strip(w), cur, mid)) != w) mid = 0;
+        }
+        mid = __shfl_sync(0xffffffffu, mid, from);
+        if (mid == 0) continue;
+        w = __shfl_sync(0xffffffffu, w, from);
+        u = range_strip(w);
+        y0 = mid;
+        y1 = range_end(w);
+        got = true;
+      }
+      if (!got) break;  // the whole warp
+    }
+    const int4 un = __ldg(table + u);
+    if (launch_idx >= batch_sweep_launches(un.w)) continue;
+    const BatchGrid& G = grids[un.x];
+    const int p = ((un.w >> 30) + launch_idx) & 1;
+    const StepArgs& ga = G.a;
+    const SweepArgs a{ga.W,      ga.H,    ga.pitch,      ga.kf,             ga.ka,       ga.c,
+                      ga.closed, ga.nsrc, ga.flux_scale, ga.flux_inv_scale, ga.neg_zero, ga.src};
+    if (queued) {
+      y0 = un.z;
+      y1 = min(y0 + batch_sweep_rows(un.w), a.H);
+    }
+    // the first rows are this warp's at once, the others can be taken over
+    const int R = min(y1 - y0, kSweepClaim);
+    const bool share = y1 - y0 > R;
+    if (share && lane == 0) atomicExch(word, range_pack(u, y0 + R, y1));
+    const int xs = un.y - kSweepHaloX(K);
+    uint32_t mask = 0;
+#pragma unroll
+    for (int k = 0; k < TWS_MAX_SOURCES; ++k) {
+      if (k < a.nsrc) {
+        const DevSource& s = a.src[k];
+        if (s.bx1 >= xs && s.bx0 < xs + kSweepCols && s.by1 >= y0 - 2 * K && s.by0 < y1 + 2 * K)
+          mask |= 1u << k;
+      }
+    }
+    const bool interior =
+        xs >= 0 && xs + kSweepCols <= a.W && y0 - 2 * K >= 0 && y1 + 2 * K <= a.H;
+    if (interior)
+      sweep_unit<K, F16, true>(a, G.b, G.d[p], G.f[p], G.d[p ^ 1], G.f[p ^ 1], G.v, ring, xs, y0,
+                               R, mask, share ? word : nullptr);
+    else
+      sweep_unit<K, F16, false>(a, G.b, G.d[p], G.f[p], G.d[p ^ 1], G.f[p ^ 1], G.v, ring, xs, y0,
+                                R, mask, share ? word : nullptr);
+  }
+  sweep_done(queue, lane);
+}
+
 template <int K>
 const void* sweep_fn(int flux_storage) {
   return flux_storage == TWS_FLUX_F16 ? reinterpret_cast<const void*>(&sweep_kernel<K, true>)
                                       : reinterpret_cast<const void*>(&sweep_kernel<K, false>);
 }
 
+const void* batch_sweep_fn(int flux_storage) {
+  return flux_storage == TWS_FLUX_F16
+             ? reinterpret_cast<const void*>(&batch_sweep_kernel<kBatchSweepK, true>)
+             : reinterpret_cast<const void*>(&batch_sweep_kernel<kBatchSweepK, false>);
+}
+
 // SMs that start on `border` of `units` units: their share of the work, a border
 // unit counted as kBorderCost inner ones.
 constexpr double kBorderCost = 1.2;
+}  // namespace
 int sweep_border_sms(long long border, long long units, int sms) {
   const double w = kBorderCost * (double)border;
   return units > 0 ? (int)(w / (w + (double)(units - border)) * sms + 0.5) : 0;
 }
+namespace {
 
 // One wave of persistent CTAs of a kernel (its occupancy, queried once).
 cudaError_t sweep_ctas(const void* fn, size_t smem, long long* ctas, int* sm_count) {
@@ -814,6 +932,34 @@ cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, 
   using Fn = void (*)(const float*, const float*, const void*, StepArgs, SweepBands);
   const cudaError_t e =
       cudaLaunchKernelEx(&cfg, reinterpret_cast<Fn>(const_cast<void*>(fn)), b, d, f, a, sb);
+  count_launch();
+  return e;
+}
+
+int batch_sweep_columns() { return kSweepCols - 2 * kSweepHaloX(kBatchSweepK); }
+
+cudaError_t batch_sweep_warps(int flux_storage, int* warps, int* sms) {
+  long long ctas = 0;
+  const cudaError_t e = sweep_ctas(batch_sweep_fn(flux_storage),
+                                   sweep_smem_bytes(kBatchSweepK, flux_storage), &ctas, sms);
+  *warps = (int)ctas * kSweepWarps;
+  return e;
+}
+
+cudaError_t launch_batch_sweep(int flux_storage, const BatchGrid* grids, const BatchUnit* units,
+                               int entries, int launch_idx, int* queue,
+                               unsigned long long* ranges, cudaStream_t s) {
+  const void* fn = batch_sweep_fn(flux_storage);
+  const size_t smem = sweep_smem_bytes(kBatchSweepK, flux_storage);
+  long long ctas = 0;
+  int sms = 0;
+  const cudaError_t e0 = sweep_ctas(fn, smem, &ctas, &sms);
+  if (e0 != cudaSuccess) return e0;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = sweep_config(std::min<long long>(entries, ctas), smem, s, attr);
+  using Fn = void (*)(const BatchGrid*, const BatchUnit*, int, int*, unsigned long long*);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, reinterpret_cast<Fn>(const_cast<void*>(fn)),
+                                           grids, units, launch_idx, queue, ranges);
   count_launch();
   return e;
 }
