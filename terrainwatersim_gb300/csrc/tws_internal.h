@@ -118,7 +118,7 @@ int batch_variant_sweep();    // the batched row sweep, three steps per launch
 // 4 x 1024^2 1715 (1314), 6 x 1024^2 1749 (1878), 8 x 1024^2 2217 (2495), 64 x
 // 512^2 4426 (4981), 16 x 2048^2 11116 (17635); FP16 16 x 1024^2 4269 (4414), 64 x
 // 512^2 4946 (4765), 128 x 512^2 8782 (9109), 8 x 2048^2 6730 (8430)).
-constexpr long long kBatchSweepCells = 6LL << 20;
+constexpr long long kBatchSweepCells = 8LL << 20;
 constexpr long long kBatchSweepF16Cells = 24LL << 20;
 void batch_variant_info(int i, int* k, int* tx, int* ty, int* step_variant);
 cudaError_t prepare_batch_variant(int variant, int flux_storage);  // outside any capture
@@ -149,7 +149,7 @@ constexpr long long kSmallStepCells = 4LL << 20;
 int step_variant_for(int k, int flux_storage, long long cells);
 // The automatic choice for grids of at least kLargeGridCells cells (FP16
 // flux: kLargeF16Cells), or -1.
-constexpr long long kLargeGridCells = 5LL << 20;
+constexpr long long kLargeGridCells = 6LL << 20;
 constexpr long long kLargeF16Cells = 17LL << 20;
 int step_variant_large_grid(int flux_storage, int W, int H);
 // Tile variants read through the tensor maps, stream variants through the

@@ -975,8 +975,9 @@ const StepVariant& step_variant(int i) { return table().e[i].v; }
 
 int step_variant_large_grid(int flux_storage, int W, int H) {
   // The three-step row sweep: FP32 flux from kLargeGridCells on (Gcell-steps/s
-  // with a rain disk, against the two-step tiles: 2048^2 167 (168), 2300^2 189
-  // (174), 2896^2 223 (183), 4096^2 268 (192)), FP16 flux from kLargeF16Cells
+  // with a rain disk, against the two-step tiles: 2048^2 167 (168), 2560^2 204
+  // (178), 2896^2 223 (183), 4096^2 267 (192); with eight disks of radius 64, which
+  // weigh on the sweep's few units, 2300^2 147 (169), 2560^2 180 (173)), FP16 flux from kLargeF16Cells
   // on (4608^2 249 (202), 5120^2 259 (204); 4096^2, 238 (200), keeps the two-step
   // tiles that callers of that size have as their default).  The band height is the tallest rung of a ladder that leaves at least
   // 2.5 column-unit bands per resident warp of a 16-warp SM (8192^2: 315 with
