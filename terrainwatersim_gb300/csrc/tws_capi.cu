@@ -1551,7 +1551,7 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
 // launch, and no more than 1.15 times the cells of the 32 x 32 tiles once both are
 // rounded up to whole strips and tiles (2000 x 64^2, 1.75 times: 5088 us against
 // 4544; 64 x 450 x 350, 1.16 times: 3405 against 3322; 500 x 130^2, 1.14 times:
-// 4008 against 4408).
+// 4008 against 4279).
 bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess ||

@@ -115,9 +115,9 @@ int batch_variant_default();  // two steps per launch, unified 32x32 tiles
 int batch_variant_sweep();    // the batched row sweep, three steps per launch
 // A batch without a set variant takes the sweep from this many cells on, where its
 // strips waste little more than the tiles (us for 48 steps, sweep against tiles:
-// 4 x 1024^2 1715 (1314), 6 x 1024^2 1749 (1878), 8 x 1024^2 2217 (2495), 64 x
-// 512^2 4426 (4981), 16 x 2048^2 11116 (17635); FP16 16 x 1024^2 4269 (4414), 64 x
-// 512^2 4946 (4765), 128 x 512^2 8782 (9109), 8 x 2048^2 6730 (8430)).
+// 6 x 1024^2 1749 (1818), 8 x 1024^2 2208 (2387), 500 x 130^2 4008 (4279), 32
+// steps of 20 grids of 128 to 2048 a side 2830 (3437); FP16 24 x 1024^2 5896
+// (6179), 128 x 512^2 8757 (8752), 8 x 2048^2 6704 (7974)).
 constexpr long long kBatchSweepCells = 8LL << 20;
 constexpr long long kBatchSweepF16Cells = 24LL << 20;
 void batch_variant_info(int i, int* k, int* tx, int* ty, int* step_variant);
@@ -149,7 +149,7 @@ constexpr long long kSmallStepCells = 4LL << 20;
 int step_variant_for(int k, int flux_storage, long long cells);
 // The automatic choice for grids of at least kLargeGridCells cells (FP16
 // flux: kLargeF16Cells), or -1.
-constexpr long long kLargeGridCells = 6LL << 20;
+constexpr long long kLargeGridCells = 7LL << 20;
 constexpr long long kLargeF16Cells = 17LL << 20;
 int step_variant_large_grid(int flux_storage, int W, int H);
 // Tile variants read through the tensor maps, stream variants through the

@@ -153,6 +153,29 @@ __device__ __forceinline__ Quad outflow_factors(const Quad& out, const Quad& dq,
   return pk4(f[0], f[1], f[2], f[3]);
 }
 
+// The same for two cells.
+__device__ __forceinline__ pair_t outflow_factors2(pair_t out, pair_t d2, pair_t cc2, pair_t ncc2,
+                                                   pair_t nz) {
+  const pair_t t2 = prod2(out, cc2, nz);
+  const float2 t = un(t2), d = un(d2);
+  const bool over0 = t.x > d.x, over1 = t.y > d.y;
+  float f0 = over0 ? d.x : 1.0f, f1 = over1 ? d.y : 1.0f;
+  const bool div0 = over0 & (d.x != 0.0f), div1 = over1 & (d.y != 0.0f);
+  if (div0 | div1) {
+    const bool far = (fmaxf(t.x, t.y) > kDivMaxT) | (div0 & (d.x < kDivMinD)) |
+                     (div1 & (d.y < kDivMinD));
+    if (!far) {
+      const float2 q = un(div2(d2, t2, prod2(out, ncc2, nz)));
+      f0 = div0 ? q.x : f0;
+      f1 = div1 ? q.y : f1;
+    } else {
+      if (div0) f0 = fdiv(d.x, t.x);
+      if (div1) f1 = fdiv(d.y, t.y);
+    }
+  }
+  return pk(f0, f1);
+}
+
 // add_rain on two cells side by side, without a branch: TwoSum's sum and error,
 // then one ulp toward d + rate with the probability that makes it exact.  h0 and
 // h1 are the cells' rain_hash32(x ^ rain_hash32(y)); a cell that is not in the

@@ -14,8 +14,9 @@
 // neighbouring CTAs, so there is no inter-CTA dependency inside a launch.
 // Two layouts: the separate one (flux box = the (2K-1)-cell halo, 2-D loops,
 // process_tile) and the unified one (flux box = the b/d box, flat loops over
-// one index, flux in channel planes, packed f32x2 arithmetic:
-// process_tile_flat), which the default variants use.
+// one index, packed f32x2 arithmetic), which the default variants use: with pairs
+// of cells in registers (process_tile_pair) or, on tiles that those do not fit,
+// the flux in channel planes (process_tile_flat).
 //
 // STAGES = 2 makes the CTAs persistent: each walks the tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ... and keeps the TMA load of its next
@@ -38,6 +39,7 @@
 
 #include "tws_device.cuh"
 #include "tws_internal.h"
+#include "tws_pair.cuh"
 
 namespace tws {
 namespace {
@@ -146,7 +148,8 @@ __host__ __device__ constexpr size_t align_up(size_t v, size_t a) { return (v + 
 // h and f share one row stride and one index per cell; interior tiles then
 // walk their rings as flat runs of that index (process_tile_flat).  It loads
 // a few more flux records per tile (served from L2).
-template <int K, int TX, int TY, bool F16, int STAGES, bool UNI = false>
+// PAIR: the unified layout as process_tile_pair uses it (no array for h).
+template <int K, int TX, int TY, bool F16, int STAGES, bool UNI = false, bool PAIR = false>
 struct Tile {
   static constexpr int HX = (2 * K + 3) / 4 * 4;  // x halo of b/d, whole 16-byte units
   static constexpr int HY = 2 * K;                // y halo of b/d
@@ -177,7 +180,7 @@ struct Tile {
   // separate layout) the float4 copy of the flux.  With one step per launch
   // the terrain is not needed once h = d + b is formed, so h overwrites b in
   // place (H_ALIAS) and the tile needs less shared memory (more CTAs per SM).
-  static constexpr bool H_ALIAS = (K == 1);
+  static constexpr bool H_ALIAS = K == 1 || PAIR;
   static constexpr size_t OFF_H = STAGES * ST_BYTES;
   static constexpr size_t OFF_WORK = align_up(OFF_H + (H_ALIAS ? 0 : (size_t)NB * 4), 128);
   static constexpr size_t OFF_BAR =
@@ -379,6 +382,7 @@ __device__ __forceinline__ void ring_for(int tid, F&& body) {
     for (int p = FIRST + tid; p <= LAST; p += kThreads) body(p);
   }
 }
+
 
 // K steps of an interior tile in the unified layout: b, d, h and f share the
 // box index p = r * BW + c (box row r, column c).  The ring of a phase is
@@ -625,12 +629,302 @@ __device__ __forceinline__ void process_tile_flat(const StepArgs& a, float* __re
   static_assert(K <= 4, "steps per launch");
 }
 
+// Where process_tile_pair is the faster one: the pairs of the run fill whole
+// rounds of the CTA, at most four (a pair's state takes 14 registers).
+// Gcell-steps/s on 2048^2, against process_tile_flat: K = 2, 32 x 32 (2.97 rounds)
+// 181 (168), with FP16 flux 192 (175), under two disks of radius 800 111 (98); K =
+// 3, 32 x 32 (3.9) 168 (141); but K = 2, 64 x 16 (3.1) 149 (157), K = 4, 32 x 32
+// (4.3) 132 (140).
+template <int K, int TX, int TY>
+__host__ __device__ constexpr bool pair_tile() {
+  using T = Tile<K, TX, TY, false, 1, true>;
+  constexpr int lo = ((T::HY - T::RF) * T::BW + (T::HX - T::RF)) / 2;
+  constexpr int hi = ((T::HY + TY + T::RF - 1) * T::BW + (T::HX + TX + T::RF - 1)) / 2;
+  constexpr int n = hi - lo + 1, rounds = (n + kThreads - 1) / kThreads;
+  return rounds <= 4 && 8 * n >= 7 * rounds * kThreads;
+}
+
+// K steps of a tile in the unified layout: b, d and f share the box index
+// p = r * BW + c (box row r, column c).  A thread keeps the same pairs of
+// neighbouring cells of a row through all steps: their depth, surface height and
+// flux stay in registers, and shared memory carries only what neighbours read of
+// each other (surface heights, in place of the loaded depths; the outflows across
+// a pair's ends and rows, in place of the loaded flux).  Every phase walks the
+// first step's outflow run, whole pairs of the flat index (box rows are even, so
+// no pair crosses one): the rings of later phases take as many rounds of the CTA,
+// and what the cells outside them compute is read by no cell that counts.  The
+// sums and products are packed f32x2 operations (products formed as in prod2, so
+// nothing is contracted), and a pair's common edge needs one slope; the cell
+// arithmetic is process_tile's, so the results are its bits.
+//
+// INTERIOR: the box lies inside the grid.  Otherwise (a tile at the grid's edge)
+// cells off the grid keep the zero flux, depth and surface that the box loaded
+// with (the shaders' out-of-range reads), and closed walls zero the outflow
+// across the border, as in process_tile.
+//
+// Cell by cell over planes of all four channels (process_tile_flat) a step moves 24
+// words of shared memory per cell, 72% of the wavefronts there are; here it moves
+// 11.  Four CTAs an SM (64 registers a thread; forced to 48 and five CTAs, with
+// spills, 162): what bounds it now is the wait for a tile's loads and between the
+// phases.
+template <int K, int TX, int TY, bool F16, bool INTERIOR>
+__device__ __forceinline__ void process_tile_pair(const StepArgs& a, float* __restrict__ d_out,
+                                                  void* __restrict__ f_out,
+                                                  float2* __restrict__ v_out, int x0, int y0,
+                                                  uint32_t mask, float* sb, float* sd,
+                                                  unsigned char* fbox) {
+  using T = Tile<K, TX, TY, F16, 1, true, true>;
+  constexpr int S = T::BW;
+  static_assert(S % 2 == 0 && TX % 2 == 0 && T::HX % 2 == 0 && T::HX >= 2 * K, "whole pairs");
+  const int tid = threadIdx.x;
+  const int W = a.W, H = a.H;
+  const bool closed = a.closed != 0;
+  const pair_t kf2 = pk(a.kf, a.kf), ka2 = pk(a.ka, a.ka), cc2 = pk(a.c, a.c);
+  const pair_t ncc2 = pk(-a.c, -a.c), nz2 = pk(a.neg_zero, a.neg_zero);
+  const float2 fscale2 = make_float2(a.flux_scale, a.flux_scale);
+  const float2 finv2 = make_float2(a.flux_inv_scale, a.flux_inv_scale);
+  // what neighbours read: +x outflow of the pair's second cell and -x outflow of
+  // its first, one float a pair; +y and -y outflows, one a cell
+  float* const fx = reinterpret_cast<float*>(fbox);
+  float* const fy = fx + T::NB / 2;
+  float* const fz = fx + T::NB;
+  float* const fw = fx + 2 * T::NB;
+  constexpr int LO = ((T::HY - T::RF) * S + (T::HX - T::RF)) / 2 * 2;
+  constexpr int HI = (T::HY + TY + T::RF - 1) * S + (T::HX + TX + T::RF - 1);
+  constexpr int N = (HI - LO) / 2 + 1;  // pairs
+  constexpr int IT = (N + kThreads - 1) / kThreads;
+  static_assert(LO <= 2 * kThreads && T::NB - LO - 2 * N <= 2 * kThreads, "the box's ends");
+  auto ld2 = [](const float* p) { return *reinterpret_cast<const pair_t*>(p); };
+  auto st2 = [](float* p, pair_t v) { *reinterpret_cast<pair_t*>(p) = v; };
+  auto each = [&](auto&& body) {
+#pragma unroll
+    for (int it = 0; it < IT; ++it)
+      if ((it + 1) * kThreads <= N || tid < N - it * kThreads)
+        body(LO + 2 * (it * kThreads + tid), it);
+  };
+  // grid coordinates of box cell p
+  auto coords = [&](int p, int& gx, int& gy) {
+    const int r = p / S;
+    gx = x0 - T::HX + (p - r * S);
+    gy = y0 - T::HY + r;
+  };
+  // The sources of the pair at p, in source order, on its depths in sd.  Both cells
+  // of a DISK go side by side without a branch.
+  auto sources = [&](int p) {
+    int gx, gy;
+    coords(p, gx, gy);
+    const bool row = INTERIOR || (unsigned)gy < (unsigned)H;
+    const bool on0 = row && (INTERIOR || (unsigned)gx < (unsigned)W);
+    const bool on1 = row && (INTERIOR || (unsigned)(gx + 1) < (unsigned)W);
+    pair_t v = ld2(sd + p);
+#pragma unroll 1
+    for (uint32_t left = mask; left; left &= left - 1) {
+      const int k = __ffs((int)left) - 1;
+      const DevSource& src = a.src[k];
+      if (gy < src.by0 || gy > src.by1 || gx + 1 < src.bx0 || gx > src.bx1) continue;
+      if (src.kind == TWS_SOURCE_DISK) {
+        const long long dx = gx - src.icx, dy = gy - src.icy;
+        const long long room = (long long)src.ir * src.ir - dy * dy;  // dx^2 allowed
+        const uint32_t hy = rain_hash32((uint32_t)gy);
+        v = rain2(v, src.rate, rain_hash32((uint32_t)gx ^ hy), rain_hash32((uint32_t)(gx + 1) ^ hy),
+                  on0 && dx * dx <= room, on1 && (dx + 1) * (dx + 1) <= room);
+      } else {
+        float2 c = un(v);
+        if (on0) c.x = add_sources_inline(c.x, gx, gy, a, 1u << k);
+        if (on1) c.y = add_sources_inline(c.y, gx + 1, gy, a, 1u << k);
+        v = pk(c.x, c.y);
+      }
+    }
+    st2(sd + p, v);
+  };
+  auto own_sources = [&]() {
+#pragma unroll 1
+    for (int p = LO + 2 * tid; p < LO + 2 * N; p += 2 * kThreads) sources(p);
+  };
+  struct Flux2 {
+    pair_t x, y, z, w;
+  };
+  Flux2 f[IT];
+  pair_t d[IT], h[IT];
+  float* const sh = sd;  // each thread turns its own depths into heights
+
+  // the box's ends, whose surface the run's first and last rows read
+  for (int end = 0; end < 2; ++end) {
+    const int p = 2 * tid + (end ? LO + 2 * N : 0);
+    if (p < (end ? T::NB : LO)) {
+      if (mask) sources(p);
+      st2(sh + p, add2(ld2(sd + p), ld2(sb + p)));
+    }
+  }
+  auto heights = [&](int p, int it) {
+    d[it] = ld2(sd + p);
+    h[it] = add2(d[it], ld2(sb + p));
+    st2(sh + p, h[it]);
+  };
+  if (mask) own_sources();
+  each(heights);
+
+  // the pair's flux as the TMA box holds it (float4 records, or halves)
+  auto box_flux = [&](int p) -> Flux2 {
+    float4 c0, c1;
+    if constexpr (F16) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(fbox + 8 * p);
+      const float2 l0 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.x)), finv2);
+      const float2 h0 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.y)), finv2);
+      const float2 l1 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.z)), finv2);
+      const float2 h1 = fmul2(__half22float2(*reinterpret_cast<const __half2*>(&raw.w)), finv2);
+      c0 = make_float4(l0.x, l0.y, h0.x, h0.y);
+      c1 = make_float4(l1.x, l1.y, h1.x, h1.y);
+    } else {
+      // every other group of four lanes reads its second record first: the eight
+      // records of a quarter-warp then lie in different banks
+      const int o = (tid >> 2) & 1;
+      const float4* const rec = reinterpret_cast<const float4*>(fbox) + p;
+      const float4 u = rec[o], v = rec[o ^ 1];
+      c0 = o ? v : u;
+      c1 = o ? u : v;
+    }
+    return Flux2{pk(c0.x, c1.x), pk(c0.y, c1.y), pk(c0.z, c1.z), pk(c0.w, c1.w)};
+  };
+  each([&](int p, int it) { f[it] = box_flux(p); });
+  __syncthreads();  // the box has been read, the surface is written
+
+  // outflow flux with non-negativity scaling, flowUpdate.comp:34-62
+  auto outflow = [&](int p, const Flux2& fo, pair_t hc, pair_t dc) -> Flux2 {
+    const float2 hv = un(hc);
+    const float dx = fsub(hv.x, hv.y);
+    const pair_t qx = prod2(pk(dx, fsub(hv.y, sh[p + 2])), ka2, nz2);  // the +x slopes
+    const pair_t qm = prod2(pk(fsub(sh[p - 1], hv.x), dx), ka2, nz2);  // minus the -x slopes
+    const pair_t qz = prod2(sub2(hc, ld2(sh + p + S)), ka2, nz2);
+    const pair_t qw = prod2(sub2(hc, ld2(sh + p - S)), ka2, nz2);
+    Flux2 n;
+    n.x = max0p(add2(prod2(fo.x, kf2, nz2), qx));
+    n.y = max0p(sub2(prod2(fo.y, kf2, nz2), qm));
+    n.z = max0p(add2(prod2(fo.z, kf2, nz2), qz));
+    n.w = max0p(add2(prod2(fo.w, kf2, nz2), qw));
+    if constexpr (!INTERIOR) {
+      int gx, gy;
+      coords(p, gx, gy);
+      const bool row = (unsigned)gy < (unsigned)H;
+      const bool on0 = row && (unsigned)gx < (unsigned)W;
+      const bool on1 = row && (unsigned)(gx + 1) < (unsigned)W;
+      auto keep = [](pair_t v, bool k0, bool k1) {
+        const float2 o = un(v);
+        return pk(k0 ? o.x : 0.0f, k1 ? o.y : 0.0f);
+      };
+      // no outflow of cells off the grid, and none across a closed wall
+      n.x = keep(n.x, on0 && !(closed && gx + 1 >= W), on1 && !(closed && gx + 2 >= W));
+      n.y = keep(n.y, on0 && !(closed && gx == 0), on1);
+      const bool z = !(closed && gy + 1 >= H), w = !(closed && gy == 0);
+      n.z = keep(n.z, on0 && z, on1 && z);
+      n.w = keep(n.w, on0 && w, on1 && w);
+    }
+    const pair_t sc =
+        outflow_factors2(add2(add2(add2(n.x, n.y), n.z), n.w), dc, cc2, ncc2, nz2);
+    n.x = prod2(n.x, sc, nz2);
+    n.y = prod2(n.y, sc, nz2);
+    n.z = prod2(n.z, sc, nz2);
+    n.w = prod2(n.w, sc, nz2);
+    if constexpr (F16) {
+      auto quant = [&](pair_t v) {
+        const float2 o = quantize_f16x2(un(v), fscale2, finv2);
+        return pk(o.x, o.y);
+      };
+      n = Flux2{quant(n.x), quant(n.y), quant(n.z), quant(n.w)};
+    }
+    return n;
+  };
+#pragma unroll
+  for (int s = 0; s < K; ++s) {
+    each([&](int p, int it) {
+      const Flux2 n = f[it] = outflow(p, f[it], h[it], d[it]);
+      fx[p / 2] = un(n.x).y;
+      fy[p / 2] = un(n.y).x;
+      st2(fz + p, n.z);
+      st2(fw + p, n.w);
+    });
+    __syncthreads();
+    // depth update, flowApply.comp:32-41; after the last step depth, flux and
+    // flow map (flowApply.comp:45-52) of the tile go out
+    each([&](int p, int it) {
+      const Flux2 c = f[it];
+      const Flux2 n{pk(un(c.y).y, fy[p / 2 + 1]), pk(fx[p / 2 - 1], un(c.x).x), ld2(fw + p + S),
+                    ld2(fz + p - S)};
+      const pair_t in = add2(add2(add2(n.x, n.y), n.z), n.w);
+      const pair_t out = add2(add2(add2(c.x, c.y), c.z), c.w);
+      d[it] = max0p(add2(d[it], prod2(sub2(in, out), cc2, nz2)));
+      int gx = 0, gy = 0;
+      if constexpr (!INTERIOR) {
+        coords(p, gx, gy);
+        const bool row = (unsigned)gy < (unsigned)H;
+        const float2 o = un(d[it]);
+        d[it] = pk(row && (unsigned)gx < (unsigned)W ? o.x : 0.0f,
+                   row && (unsigned)(gx + 1) < (unsigned)W ? o.y : 0.0f);
+      }
+      if (s + 1 < K) {
+        if (mask) {
+          st2(sd + p, d[it]);  // (no neighbour reads heights in this phase)
+        } else {
+          h[it] = add2(d[it], ld2(sb + p));
+          st2(sh + p, h[it]);
+        }
+      } else {
+        const int r = p / S, i = r - T::HY, j = p - r * S - T::HX;
+        if ((unsigned)i < (unsigned)TY && (unsigned)j < (unsigned)TX &&
+            (INTERIOR || (gx < W && gy < H))) {
+          const size_t g = (size_t)(y0 + i) * (size_t)a.pitch + (size_t)(x0 + j);
+          const bool both = INTERIOR || gx + 1 < W;
+          const float2 dn = un(d[it]);
+          const float2 x = un(c.x), y = un(c.y), z = un(c.z), w = un(c.w);
+          const float2 vx = un(sub2(sub2(n.x, c.x), sub2(n.y, c.y)));
+          const float2 vy = un(sub2(sub2(n.z, c.z), sub2(n.w, c.w)));
+          if (both)
+            *reinterpret_cast<float2*>(d_out + g) = dn;
+          else
+            d_out[g] = dn.x;
+          if constexpr (F16) {
+            auto half2 = [&](float lo, float hi) {
+              const __half2 q = __float22half2_rn(fmul2(make_float2(lo, hi), fscale2));
+              return *reinterpret_cast<const uint32_t*>(&q);
+            };
+            const uint2 o0 = make_uint2(half2(x.x, y.x), half2(z.x, w.x));
+            const uint2 o1 = make_uint2(half2(x.y, y.y), half2(z.y, w.y));
+            uint2* const fo = reinterpret_cast<uint2*>(f_out) + g;
+            if (both)
+              *reinterpret_cast<uint4*>(fo) = make_uint4(o0.x, o0.y, o1.x, o1.y);
+            else
+              *fo = o0;
+          } else {
+            float4* const fo = reinterpret_cast<float4*>(f_out) + g;
+            if (both)
+              store32(fo, x.x, y.x, z.x, w.x, x.y, y.y, z.y, w.y);
+            else
+              *fo = make_float4(x.x, y.x, z.x, w.x);
+          }
+          if (both)
+            *reinterpret_cast<float4*>(v_out + g) = make_float4(vx.x, vy.x, vx.y, vy.y);
+          else
+            v_out[g] = make_float2(vx.x, vy.x);
+        }
+      }
+    });
+    if (s + 1 < K) {
+      if (mask) {
+        own_sources();
+        each(heights);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // ---- the kernel --------------------------------------------------------------
 template <int K, int TX, int TY, bool F16, int STAGES, bool UNI>
 __global__ void __launch_bounds__(kThreads)
     step_kernel(const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_d,
                 const __grid_constant__ CUtensorMap tm_f, const __grid_constant__ StepArgs a) {
-  using T = Tile<K, TX, TY, F16, STAGES, UNI>;
+  constexpr bool PAIR = UNI && pair_tile<K, TX, TY>();
+  using T = Tile<K, TX, TY, F16, STAGES, UNI, PAIR>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = align_smem(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::OFF_BAR);
@@ -712,7 +1006,14 @@ __global__ void __launch_bounds__(kThreads)
 
     const bool interior =
         x0 - T::HX >= 0 && y0 - T::HY >= 0 && x0 + TX + T::HX <= a.W && y0 + TY + T::HY <= a.H;
-    if constexpr (UNI) {
+    if constexpr (PAIR) {
+      if (interior)
+        process_tile_pair<K, TX, TY, F16, true>(a, a.d_out, a.f_out, a.v_out, x0, y0, mask, sb, sd,
+                                                st + T::ST_F);
+      else
+        process_tile_pair<K, TX, TY, F16, false>(a, a.d_out, a.f_out, a.v_out, x0, y0, mask, sb,
+                                                 sd, st + T::ST_F);
+    } else if constexpr (UNI) {
       if (interior)
         process_tile_flat<K, TX, TY, F16, STAGES, true>(a, a.d_out, a.f_out, a.v_out, x0, y0,
                                                         mask, sb, sd, sh, st + T::ST_F);
@@ -759,11 +1060,18 @@ __device__ __forceinline__ void tensormap_acquire(const void* tm) {
 // `launch_idx` of a chain skips grids that have taken all their launches, so
 // grids with different step counts share a chain.  The CTA then runs the
 // same per-tile steps as step_kernel.
+//
+// Four CTAs an SM where the pairs stay in registers, as many as the single-grid
+// kernel holds: us for 48 steps against process_tile_flat at five, one rain disk a
+// grid: 8 FP32 grids of 512^2 762 (816), 64 of 256^2 1560 (1572), 200 of 64^2 536
+// (655); FP16 8 of 512^2 672 (776), 64 of 256^2 1403 (1506).
 template <int K, int TX, int TY, bool F16, bool UNI, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
+__global__ void __launch_bounds__(kThreads,
+                                  UNI && pair_tile<K, TX, TY>() && MINB > 4 ? 4 : MINB)
     batch_kernel(const BatchGrid* __restrict__ grids, const BatchUnit* __restrict__ units,
                  int launch_idx) {
-  using T = Tile<K, TX, TY, F16, 1, UNI>;
+  constexpr bool PAIR = UNI && pair_tile<K, TX, TY>();
+  using T = Tile<K, TX, TY, F16, 1, UNI, PAIR>;
   const int4 un = __ldg(reinterpret_cast<const int4*>(units) + blockIdx.x);
   if (launch_idx >= (un.w & 0x3fffffff)) return;
   const BatchGrid& G = grids[un.x];
@@ -811,7 +1119,14 @@ __global__ void __launch_bounds__(kThreads, MINB)
   const int gw = a.W, gh = a.H;
   const bool interior =
       x0 - T::HX >= 0 && y0 - T::HY >= 0 && x0 + TX + T::HX <= gw && y0 + TY + T::HY <= gh;
-  if constexpr (UNI) {
+  if constexpr (PAIR) {
+    if (interior)
+      process_tile_pair<K, TX, TY, F16, true>(a, G.d[p ^ 1], G.f[p ^ 1], G.v, x0, y0, mask, sb, sd,
+                                              smem + T::ST_F);
+    else
+      process_tile_pair<K, TX, TY, F16, false>(a, G.d[p ^ 1], G.f[p ^ 1], G.v, x0, y0, mask, sb,
+                                               sd, smem + T::ST_F);
+  } else if constexpr (UNI) {
     if (interior)
       process_tile_flat<K, TX, TY, F16, 1, true>(a, G.d[p ^ 1], G.f[p ^ 1], G.v, x0, y0, mask, sb,
                                                  sd, sh, smem + T::ST_F);
@@ -840,8 +1155,9 @@ struct VariantEntry {
 
 template <int K, int TX, int TY, int STAGES, bool UNI>
 VariantEntry make_entry() {
-  using T32 = Tile<K, TX, TY, false, STAGES, UNI>;
-  using T16 = Tile<K, TX, TY, true, STAGES, UNI>;
+  constexpr bool PAIR = UNI && pair_tile<K, TX, TY>();
+  using T32 = Tile<K, TX, TY, false, STAGES, UNI, PAIR>;
+  using T16 = Tile<K, TX, TY, true, STAGES, UNI, PAIR>;
   VariantEntry e;
   e.v.k = K;
   e.v.tx = TX;
@@ -975,10 +1291,11 @@ const StepVariant& step_variant(int i) { return table().e[i].v; }
 
 int step_variant_large_grid(int flux_storage, int W, int H) {
   // The three-step row sweep: FP32 flux from kLargeGridCells on (Gcell-steps/s
-  // with a rain disk, against the two-step tiles: 2048^2 167 (168), 2560^2 204
-  // (178), 2896^2 223 (183), 4096^2 267 (192); with eight disks of radius 64, which
-  // weigh on the sweep's few units, 2300^2 147 (169), 2560^2 180 (173)), FP16 flux from kLargeF16Cells
-  // on (4608^2 249 (202), 5120^2 259 (204); 4096^2, 238 (200), keeps the two-step
+  // with a rain disk, against the two-step tiles: 2048^2 167 (181), 2560^2 210
+  // (190), 2896^2 229 (193), 3400^2 252 (197); with eight disks of a sixteenth of
+  // the side, which weigh on the sweep's few units, 2720^2 171 (176), 2896^2 187
+  // (178), 3400^2 218 (185)), FP16 flux from kLargeF16Cells
+  // on (4608^2 249 (217), with eight disks 229 (209); 4096^2, 238 (216), keeps the two-step
   // tiles that callers of that size have as their default).  The band height is the tallest rung of a ladder that leaves at least
   // 2.5 column-unit bands per resident warp of a 16-warp SM (8192^2: 315 with
   // 192/48 rows, 305 with uniform bands of 64 to 192; 16384^2: 339 with 256/64,
@@ -1171,8 +1488,9 @@ BatchEntry make_batch_entry(int step_variant) {
   e.step_variant = step_variant;
   e.fn[TWS_FLUX_F32] = reinterpret_cast<const void*>(&batch_kernel<K, TX, TY, false, UNI, MINB>);
   e.fn[TWS_FLUX_F16] = reinterpret_cast<const void*>(&batch_kernel<K, TX, TY, true, UNI, MINB>);
-  e.smem[TWS_FLUX_F32] = Tile<K, TX, TY, false, 1, UNI>::SMEM;
-  e.smem[TWS_FLUX_F16] = Tile<K, TX, TY, true, 1, UNI>::SMEM;
+  constexpr bool PAIR = UNI && pair_tile<K, TX, TY>();
+  e.smem[TWS_FLUX_F32] = Tile<K, TX, TY, false, 1, UNI, PAIR>::SMEM;
+  e.smem[TWS_FLUX_F16] = Tile<K, TX, TY, true, 1, UNI, PAIR>::SMEM;
   return e;
 }
 
