@@ -266,14 +266,15 @@ TWS_API int tws_set_resident(tws_grid* grid, int ctas);
  * Terrain::PerformSimulationStep (Terrain.cpp:253-265).  Asynchronous.
  *
  * With nothing pinned (no variant, no steps-per-launch setting, no resident
- * kernel), calls of at least 4 steps (8 from about half a million cells on)
- * on grids of up to about 1.1 million cells with at most two brush sources run as one launch of the mesh kernel: the state stays on chip, spread
- * over all SMs, whose tiles exchange their borders every few steps.  Mesh
- * launches of one device run one after another, whatever their streams, and
+ * kernel), calls of at least 4 steps (8 from about half a million cells on, 12
+ * from about 0.8 million) on grids of up to about 1.1 million cells with at most
+ * two brush sources run as one launch of the mesh kernel: the state stays on
+ * chip, spread over all SMs, whose tiles exchange their borders every few steps.
+ * Mesh launches of one device run one after another, whatever their streams, and
  * share one workspace of up to some tens of MB, which goes with the last grid
- * that could use it.  Its waits for neighbouring tiles are bounded by tws_set_wait_limit too, and a
- * call being captured into a CUDA graph uses the variants.  Results do not
- * depend on the choice. */
+ * that could use it.  Its waits for neighbouring tiles are bounded by
+ * tws_set_wait_limit too, and a call being captured into a CUDA graph uses the
+ * variants.  Results do not depend on the choice. */
 TWS_API int tws_step(tws_grid* grid, int nsteps);
 
 /* Total water volume sum(d) * cell_area, accumulated in FP64 on the device

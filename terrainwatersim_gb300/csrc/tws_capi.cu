@@ -228,10 +228,11 @@ int resident_ctas(tws_grid* g, int nsteps) {
 
 // Calls shorter than this stay with the step kernels: a mesh launch loads and
 // stores the whole state and sets up its exchange.  Microseconds per call with the
-// mesh kernel and with two-step tiles, a rain disk: 64^2, 8 steps 14.8 and 37.7
-// (about 10 and 19.5 at 4); 512^2, 8 steps 27.3 and 44.2 (17.5 and 22.7 at 4);
-// 1021 x 763, 8 steps 50.4 and 56.4 (about equal at 4).
-int mesh_min_steps(const MeshShape& s) { return s.ry <= 4 ? 4 : 8; }
+// mesh kernel and with two-step tiles, a rain disk: 64^2, 4 steps 9.4 and 13.8; 512^2,
+// 4 steps 17.1 and 16.9, 8 steps 27.5 and 33.0; 1021 x 763, 8 steps 50.8 and 51.3, 16
+// steps 91 and 101; 1024^2, 8 steps 63.4 and 58.8, 12 steps 88.1 and 87.9, 16 steps
+// 113 and 116.
+int mesh_min_steps(const MeshShape& s) { return s.ry <= 4 ? 4 : s.ry <= 7 ? 8 : 12; }
 
 // How the mesh kernel runs a call of `nsteps` steps, or null if it does not: it
 // runs the calls of at least mesh_min_steps steps on grids that fit it, unless

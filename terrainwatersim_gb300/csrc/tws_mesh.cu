@@ -31,8 +31,8 @@
 // chosen per grid from a measured cost model (mesh_shape).
 //
 // Measured (us per step of long calls, CUDA events, one rain disk; in brackets the
-// two-step tiles): 64^2 1.2 (4.5), 256^2 1.7 (4.3), 512^2 2.4 (5.0), 1021 x 763
-// 4.9 (6.8), 1024^2 6.2 (8.1).  Four columns per lane (boxes of 128 columns) issue
+// two-step tiles): 64^2 1.3 (3.1), 256^2 1.7 (3.3), 512^2 2.5 (3.9), 1021 x 763
+// 4.9 (6.2), 1024^2 5.9 (7.1).  Four columns per lane (boxes of 128 columns) issue
 // less per cell but leave a quarter of the warps' parallelism: 256^2 2.5 against
 // 1.4 without rain.
 //
