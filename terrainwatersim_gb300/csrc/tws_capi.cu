@@ -532,9 +532,9 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
     return o;
   };
   const size_t ob = take(n * 4), od0 = take(n * 4), od1 = take(n * 4), of0 = take(n * fb),
-               of1 = take(n * fb), ov = take(n * 8),
+               of1 = take(n * fb), ov = take(n * 8), oe = take(kScratchBytes), zeroed = off,
                op = take(sizeof(double) * volume_partials_needed()), oo = take(sizeof(double)),
-               oe = take(kScratchBytes), ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
+               ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
   cudaMemPool_t pool = library_pool(g->device);
   if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&g->slab), off, pool, g->stream) !=
                    cudaSuccess) {
@@ -553,15 +553,10 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   g->queue = reinterpret_cast<int*>(g->slab + oe + 16);
   g->ranges = reinterpret_cast<unsigned long long*>(g->slab + oe + 64);
   g->desc = reinterpret_cast<CUtensorMap*>(g->slab + ot);
-  // Zero everything, padding included (the F16 flux map reads the padding
-  // cell of odd-width rows and relies on it staying zero).
-  cudaMemsetAsync(g->b, 0, n * 4, g->stream);
-  cudaMemsetAsync(g->d[0], 0, n * 4, g->stream);
-  cudaMemsetAsync(g->d[1], 0, n * 4, g->stream);
-  cudaMemsetAsync(g->f[0], 0, n * fb, g->stream);
-  cudaMemsetAsync(g->f[1], 0, n * fb, g->stream);
-  cudaMemsetAsync(g->v, 0, n * 8, g->stream);
-  cudaMemsetAsync(g->err, 0, kScratchBytes, g->stream);
+  // Zero the state and the scratch, padding included (the F16 flux map reads the
+  // padding cell of odd-width rows and relies on it staying zero): the front of
+  // the allocation, in one fill.
+  cudaMemsetAsync(g->slab, 0, zeroed, g->stream);
   // the mesh kernel's workspace, where it fits this grid (whatever its sources)
   size_t inbox = 0;
   for (int brushes = 0; brushes <= TWS_MAX_SOURCES; ++brushes) {
