@@ -1215,7 +1215,7 @@ struct VariantTable {
     add<4, 64, 16, 1, true>();  // 21
     add<3, 64, 32, 1, true>();  // 22
     // row sweeps: 128-column warp strips, K time levels on chip, the rows
-    // of a band.  4096^2 FP32 (Gcell-steps/s): K = 3 256, K = 2 200, K = 4 196.
+    // of a band.  4096^2 FP32 (Gcell-steps/s): K = 3 274, K = 2 223, K = 4 265.
     add_sweep(2, 32);  // 23
     add_sweep(2, 48);  // 24
     add_sweep(3, 32);  // 25
