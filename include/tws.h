@@ -384,8 +384,9 @@ TWS_API int tws_get_buffers(tws_grid* grid, tws_buffers* out);
  * tiles of every member grid, and chains of up to 16 steps (with the row sweep:
  * 16 launches) are replayed from CUDA graphs.  A batch whose variant has not
  * been set takes the row sweep, three steps per launch, where its members are
- * large enough together (FP32 flux: 8 Mi cells, FP16: 24 Mi) and fill their
- * strips, and the two-step tiles otherwise; the results are the same.  Member grids keep their own buffers,
+ * large enough together (FP32 flux: 8 Mi cells, FP16: 24 Mi; more where sources
+ * reach many of the units) and fill their strips, and the two-step tiles
+ * otherwise; the results are the same.  Member grids keep their own buffers,
  * parameters and sources; while in a batch their work is ordered on the
  * batch's stream.  Grids can join and leave between calls (continuous
  * batching); each call advances every member by its own step count.  No

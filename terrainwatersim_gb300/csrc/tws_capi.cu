@@ -1546,8 +1546,13 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
 // Whether a batch that was given no variant takes the row sweep: three steps a
 // launch, and no more than 1.15 times the cells of the 32 x 32 tiles once both are
 // rounded up to whole strips and tiles (2000 x 64^2, 1.75 times: 5088 us against
-// 4544; 64 x 450 x 350, 1.16 times: 3405 against 3322; 500 x 130^2, 1.14 times:
-// 4008 against 4279).
+// 4544; 64 x 450 x 350, 1.16 times: 3405 against 3322).  Units that a source reaches take longer, and there are few
+// units: their share raises the least size by five times itself, and from a
+// quarter of the units on the tiles stay (48 steps, eight disks a grid: 12 x
+// 1024^2, radius 16, 7% of the units 3506 us against 3810; 4 x 2048^2, radius 64, 9%
+// 3857 against 4730; 16 x 1024^2, radius 64, 34% 5393 against 5355; 64 x 512^2,
+// radius 16, 48% 6380 against 5595; two disks of radius 64: 8 x 1024^2, 7% 2701
+// against 2477, 16 x 1024^2, 9% 4352 against 4716).
 bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess ||
@@ -1555,18 +1560,37 @@ bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
     cudaGetLastError();
     return false;
   }
-  const int cols = batch_sweep_columns();
-  long long cells = 0, strips = 0, tiles = 0, units = 0;
-  for (size_t i = 0; i < steps.size(); ++i) {
-    if (steps[i] < kBatchSweepK) continue;
-    const long long W = b->grids[i]->W, H = b->grids[i]->H, s = (W + cols - 1) / cols;
+  std::vector<int> part(steps);
+  for (int& n : part)
+    if (n < kBatchSweepK) n = 0;
+  int warps = 0, sms = 0;
+  if (batch_sweep_warps(b->flux_storage, &warps, &sms) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const long long cols = batch_sweep_columns(), rows = sweep_band_rows(b, part, warps);
+  long long cells = 0, strips = 0, tiles = 0, units = 0, wet = 0;
+  for (size_t i = 0; i < part.size(); ++i) {
+    if (part[i] == 0) continue;
+    const tws_grid* g = b->grids[i];
+    const long long W = g->W, H = g->H, s = (W + cols - 1) / cols, n = s * ((H + rows - 1) / rows);
     cells += W * H;
     strips += s * cols * H;
     tiles += (W + 31) / 32 * 32 * ((H + 31) / 32 * 32);
-    units += s * ((H + kBatchSweepMinRows - 1) / kBatchSweepMinRows);
+    units += n;
+    long long w = 0;
+    for (int k = 0; k < g->nsrc; ++k) {
+      const DevSource d = make_dev_source(g->src[k]);
+      const long long x0 = std::max(d.bx0, 0), x1 = std::min<long long>(d.bx1, W - 1);
+      const long long y0 = std::max(d.by0, 0), y1 = std::min<long long>(d.by1, H - 1);
+      if (x0 <= x1 && y0 <= y1) w += (x1 / cols - x0 / cols + 1) * (y1 / rows - y0 / rows + 1);
+    }
+    wet += std::min(w, n);
   }
-  return units < kSweepMaxUnits / 2 && 20 * strips <= 23 * tiles &&
-         cells >= (b->flux_storage == TWS_FLUX_F16 ? kBatchSweepF16Cells : kBatchSweepCells);
+  const long long least =
+      b->flux_storage == TWS_FLUX_F16 ? kBatchSweepF16Cells : kBatchSweepCells;
+  return units > 0 && units < kSweepMaxUnits / 2 && 20 * strips <= 23 * tiles &&
+         4 * wet <= units && (double)cells >= (double)least * (1.0 + 5.0 * (double)wet / (double)units);
 }
 
 // Advance member i by steps[i] steps, in chains of up to kChainSteps steps (of

@@ -65,11 +65,12 @@ def test_matches_each_grid_alone(tws, flux, steps):
 def test_taken_for_large_batches_only(tws):
     """Three steps a launch from the size on where it is the faster one, unless a
     variant is set."""
-    def launches(W, H, variant=None):
+    def launches(W, H, variant=None, disks=0):
         with tws.Batch() as batch:
             gs = [tws.Grid(W, H, tws.params_physical())
                   for _ in range(2)]
             for g in gs:
+                g.set_sources(tws.rain_disks(3, W, H, 500, 0.01, disks) if disks else [])
                 batch.add(g)
             if variant is not None:
                 batch.set_variant(variant)
@@ -85,4 +86,5 @@ def test_taken_for_large_batches_only(tws):
     assert launches(512, 512) == 6
     assert launches(4096, 2048) == 4
     assert launches(4096, 2048, variant=4) == 6
+    assert launches(4096, 2048, disks=8) == 6  # rain on most units
     assert launches(512, 512, variant=SWEEP) == 4
