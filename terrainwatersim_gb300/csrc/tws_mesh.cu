@@ -130,10 +130,13 @@ __global__ void __launch_bounds__(kMeshThreads, 1)
   const int gy0 = ty * (kMeshWarps * RY - 2 * hy) - hy + row0;
   const int cols = gx < 0 ? 0 : min(2, max(0, W - gx));
   const bool closed = a.closed != 0;
-  // (a CTA whose box lies inside the grid skips the border's rules)
+  // A CTA whose box lies inside the grid skips the border's rules.  A box without
+  // halo rows may end on the grid's first and last row, whose walls it then has; in
+  // x every box has halo columns, and one that ends on a wall's column only has
+  // it among the cells that go stale.
   const int by = gy0 - row0;
-  const bool edge = gx - 2 * lane < 0 || gx - 2 * lane + kMeshCols > W || by < 0 ||
-                    by + kMeshWarps * RY > H;
+  const bool edge = gx - 2 * lane < 0 || gx - 2 * lane + kMeshCols > W || by <= 0 ||
+                    by + kMeshWarps * RY >= H;
   // (the border's rules as bit masks of the lane's two cells: +x outflows, -x
   // outflows and depths that may be nonzero)
   auto cell_mask = [](bool lo, bool hi) {
