@@ -143,6 +143,9 @@ enum : int { kDevErrNone = 0, kDevErrWaitTimeout = 1 };
 constexpr long long kDefaultWaitCycles = 4000000000LL;
 
 // Host helpers implemented in tws_step.cu.
+// Raises the kernel's shared memory limit on the current device to `smem` bytes, and
+// the CTAs of `threads` threads that an SM then holds; both asked once per device.
+cudaError_t kernel_limits(const void* fn, int threads, size_t smem, int* ctas_per_sm);
 int step_variant_count();
 const StepVariant& step_variant(int i);
 constexpr long long kSmallStepCells = 4LL << 20;

@@ -39,8 +39,6 @@
 // The arithmetic is the tiled kernels', operation for operation.
 
 #include <algorithm>
-#include <map>
-#include <mutex>
 
 #include "tws_device.cuh"
 #include "tws_internal.h"
@@ -681,18 +679,10 @@ cudaError_t launch_mesh(const MeshShape& s, int flux_storage, const float* b, fl
   MeshFn fn = mesh_fn(s.ry, flux_storage);
   if (!fn || nsteps < 1 || !inbox) return cudaErrorInvalidValue;
   const int smem = mesh_launch_smem(s);
-  {
-    static std::mutex mu;
-    static std::map<MeshFn, int> set;
-    std::lock_guard<std::mutex> lk(mu);
-    int& have = set[fn];
-    if (smem > have) {
-      const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      have = smem;
-    }
-  }
+  int per_sm = 0;  // (one: the cooperative launch checks it)
+  const cudaError_t limit =
+      kernel_limits(reinterpret_cast<const void*>(fn), kMeshThreads, (size_t)smem, &per_sm);
+  if (limit != cudaSuccess) return limit;
   MeshArgs m{};
   m.b = b;
   for (int i = 0; i < 2; ++i) {

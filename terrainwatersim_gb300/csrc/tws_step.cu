@@ -39,6 +39,7 @@
 
 #include "tws_device.cuh"
 #include "tws_internal.h"
+#include "tws_limits.h"
 #include "tws_pair.cuh"
 
 namespace tws {
@@ -1149,8 +1150,6 @@ struct VariantEntry {
   StepVariant v;
   const void* fn[2];  // [flux storage]
   size_t smem[2];
-  int ctas_per_sm[2] = {0, 0};  // occupancy, filled on first launch
-  bool attr_set[2] = {false, false};
 };
 
 template <int K, int TX, int TY, int STAGES, bool UNI>
@@ -1184,7 +1183,6 @@ struct VariantTable {
   static constexpr int kMax = 48;
   VariantEntry e[kMax + 1];  // one spare slot: an entry past kMax is dropped, not written over n
   int n = 0;
-  std::mutex mu;
   VariantTable() {
     // Entries 0..3 are the first tile choice for K = 1..4 in the separate
     // layout (measured on 4096^2: one CTA per tile with a small shared-memory
@@ -1285,6 +1283,19 @@ EncodeTiledFn encode_fn(std::string* why) {
 }
 
 }  // namespace
+
+cudaError_t kernel_limits(const void* fn, int threads, size_t smem, int* ctas_per_sm) {
+  static KernelLimits limits;
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  return limits.get(dev, fn, smem, ctas_per_sm, [&](int* n) {
+    const cudaError_t set =
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return set != cudaSuccess ? set
+                              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, fn, threads, smem);
+  });
+}
 
 int step_variant_count() { return table().n; }
 const StepVariant& step_variant(int i) { return table().e[i].v; }
@@ -1413,20 +1424,9 @@ cudaError_t launch_step(int variant, int flux_storage, const CUtensorMap* tm_b,
   if (!tm_b || !tm_d || !tm_f) return cudaErrorInvalidValue;
   const void* fn = e.fn[fs];
   const size_t smem = e.smem[fs];
-  int ctas_per_sm;
-  {
-    std::lock_guard<std::mutex> lk(t.mu);
-    if (!e.attr_set[fs]) {
-      cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (err != cudaSuccess) return err;
-      int n = 0;
-      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, smem);
-      if (err != cudaSuccess) return err;
-      e.ctas_per_sm[fs] = n > 0 ? n : 1;
-      e.attr_set[fs] = true;
-    }
-    ctas_per_sm = e.ctas_per_sm[fs];
-  }
+  int ctas_per_sm = 0;
+  const cudaError_t limit = kernel_limits(fn, kThreads, smem, &ctas_per_sm);
+  if (limit != cudaSuccess) return limit;
   const StepVariant& v = e.v;
   const int tiles_x = (a.W + v.tx - 1) / v.tx, tiles_y = (a.H + v.ty - 1) / v.ty;
   dim3 grid(tiles_x, tiles_y);  // one CTA per tile
@@ -1471,8 +1471,6 @@ struct BatchEntry {
                      // -1: the row sweep, which reads through plain pointers
   const void* fn[2];
   size_t smem[2];
-  int ctas_per_sm[2] = {0, 0};
-  bool set[2] = {false, false};
 };
 
 // MINB: CTAs per SM the register allocation must allow (the batched kernel
@@ -1497,7 +1495,6 @@ BatchEntry make_batch_entry(int step_variant) {
 struct BatchTable {
   BatchEntry e[8];
   int n = 0;
-  std::mutex mu;
   BatchTable() {
     e[n++] = make_batch_entry<1, 32, 32, false, 5>(0);
     e[n++] = make_batch_entry<2, 32, 32, false, 5>(10);
@@ -1546,18 +1543,8 @@ cudaError_t prepare_batch_variant(int variant, int flux_storage) {
   const StepVariant& sv = step_variant(e.step_variant);
   if (sv.k != e.k || sv.tx != e.tx || sv.ty != e.ty || sv.uni != e.uni || sv.stages != 1)
     return cudaErrorInvalidValue;  // the tables disagree: the maps would not fit
-  std::lock_guard<std::mutex> lk(t.mu);
-  if (!e.set[fs]) {
-    cudaError_t err =
-        cudaFuncSetAttribute(e.fn[fs], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem[fs]);
-    if (err != cudaSuccess) return err;
-    int n = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, e.fn[fs], kThreads, e.smem[fs]);
-    if (err != cudaSuccess) return err;
-    e.ctas_per_sm[fs] = n > 0 ? n : 1;
-    e.set[fs] = true;
-  }
-  return cudaSuccess;
+  int ctas_per_sm = 0;
+  return kernel_limits(e.fn[fs], kThreads, e.smem[fs], &ctas_per_sm);
 }
 
 cudaError_t launch_batch_step(int variant, int flux_storage, const BatchGrid* grids,

@@ -55,8 +55,6 @@
 // cycles (three warps each: fixed-latency waits, shared memory, fetch).
 
 #include <algorithm>
-#include <map>
-#include <mutex>
 
 #include "tws_device.cuh"
 #include "tws_internal.h"
@@ -840,26 +838,11 @@ int sweep_border_sms(long long border, long long units, int sms) {
 }
 namespace {
 
-// One wave of persistent CTAs of a kernel (its occupancy, queried once).
+// One wave of persistent CTAs of a kernel.
 cudaError_t sweep_ctas(const void* fn, size_t smem, long long* ctas, int* sm_count) {
-  static std::mutex mu;
-  static std::map<const void*, int> resident;
   int per_sm = 0, sms = 0;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = resident.find(fn);
-    if (it == resident.end()) {
-      cudaError_t e = cudaSuccess;
-      if (smem > 48 * 1024)
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      int n = 0;
-      if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kSweepThreads, smem);
-      if (e != cudaSuccess) return e;
-      it = resident.emplace(fn, n > 0 ? n : 1).first;
-    }
-    per_sm = it->second;
-  }
+  const cudaError_t e = kernel_limits(fn, kSweepThreads, smem, &per_sm);
+  if (e != cudaSuccess) return e;
   int dev = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
