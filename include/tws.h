@@ -270,9 +270,11 @@ TWS_API int tws_set_resident(tws_grid* grid, int ctas);
  * from about 0.8 million) on grids of up to about 1.1 million cells with at most
  * two brush sources run as one launch of the mesh kernel: the state stays on
  * chip, spread over all SMs, whose tiles exchange their borders every few steps.
- * Mesh launches of one device run one after another, whatever their streams, and
- * share one workspace of up to some tens of MB, which goes with the last grid
- * that could use it.  Its waits for neighbouring tiles are bounded by
+ * Mesh launches of one device share one workspace of up to some tens of MB, which
+ * goes with the last grid that could use it, and never run side by side: a call
+ * that finds step work of such a grid on another stream under way uses the
+ * variants instead, beside it (grids of one CTA, up to 60 x 144 cells, run as one
+ * launch all the same).  No stream waits for another.  Its waits for neighbouring tiles are bounded by
  * tws_set_wait_limit too, and a call being captured into a CUDA graph uses the
  * variants.  Results do not depend on the choice. */
 TWS_API int tws_step(tws_grid* grid, int nsteps);

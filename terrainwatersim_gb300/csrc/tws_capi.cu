@@ -255,16 +255,25 @@ const MeshShape* mesh_for(tws_grid* g, int nsteps) {
 
 // The mesh kernel's inboxes, one set per device, held by the grids that the kernel
 // fits: made with the first, grown for one that needs more, freed with the last.
-// Mesh launches of one device run one after another, whatever their streams (each
-// waits for the previous one's event): they share the inboxes, and their CTAs
-// wait for one another, so two of them must not hold half of the SMs each.
+//
+// Mesh launches share the inboxes, and their CTAs wait for one another, so two of
+// them must not run side by side (each might hold half of the SMs).  On one stream
+// they do not; across streams a call that finds step work of another stream's mesh
+// grid under way takes the step kernels instead of waiting for it: no stream
+// depends on another, and the GPU is shared (grids stepped on streams of their
+// own fill it better with tiles than in turn, one mesh launch after the other).
+struct MeshStream {
+  unsigned long long id;  // cudaStreamGetId: never given to a second stream
+  cudaEvent_t last;       // after the last call's work (or the inboxes' clearing)
+  bool busy;              // not yet seen complete
+};
 struct MeshSpace {
   std::mutex mu;
   int users = 0;
   char* inbox = nullptr;
   size_t bytes = 0;
-  unsigned epoch = 0;         // number of the last exchange
-  cudaEvent_t done = nullptr;  // the last launch, or the inboxes' clearing
+  unsigned epoch = 0;  // number of the last exchange
+  std::vector<MeshStream> streams;
 };
 
 MeshSpace* mesh_space(int device) {
@@ -272,70 +281,147 @@ MeshSpace* mesh_space(int device) {
   return device >= 0 && device < 64 ? &spaces[device] : nullptr;
 }
 
+// Whether the stream's work is still under way.  (A query is refused, and another
+// thread's capture with it, while one of global mode is being made, unless this
+// thread says that it has no part in it.)
+bool mesh_still_busy(MeshStream& s) {
+  if (!s.busy) return false;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaEventQuery(s.last);
+  if (e != cudaSuccess) cudaGetLastError();
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  s.busy = e != cudaSuccess;
+  return s.busy;
+}
+
+// The entry of a stream; a new one takes the place of one whose work is done.
+MeshStream* mesh_stream(MeshSpace* m, cudaStream_t s) {
+  unsigned long long id = 0;
+  if (cudaStreamGetId(s, &id) != cudaSuccess) return nullptr;
+  for (MeshStream& e : m->streams)
+    if (e.id == id) return &e;
+  for (MeshStream& e : m->streams)
+    if (!mesh_still_busy(e)) {
+      e.id = id;
+      return &e;
+    }
+  MeshStream e{id, nullptr, false};
+  if (cudaEventCreateWithFlags(&e.last, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+  m->streams.push_back(e);
+  return &m->streams.back();
+}
+
+bool mesh_others_busy(MeshSpace* m, const MeshStream* self) {
+  // (the first busy one will do: a query takes half a microsecond)
+  for (MeshStream& e : m->streams)
+    if (&e != self && mesh_still_busy(e)) return true;
+  return false;
+}
+
+cudaError_t mesh_record(MeshStream* self, cudaStream_t s) {
+  const cudaError_t e = cudaEventRecord(self->last, s);
+  self->busy = true;
+  return e;
+}
+
+// Gives the inboxes back once the work that may use them is done, without making a
+// stream of the caller's wait for it.
+void mesh_free_inbox(MeshSpace* m, int device) {
+  if (!m->inbox) return;
+  int current = device;
+  cudaGetDevice(&current);
+  if (current != device) cudaSetDevice(device);
+  cudaStream_t t = nullptr;
+  bool ok = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) == cudaSuccess;
+  for (MeshStream& e : m->streams)
+    if (mesh_still_busy(e)) ok = ok && cudaStreamWaitEvent(t, e.last, 0) == cudaSuccess;
+  if (ok) {
+    cudaFreeAsync(m->inbox, t);
+  } else {
+    cudaGetLastError();
+    cudaFree(m->inbox);  // (waits for the device)
+  }
+  if (t) cudaStreamDestroy(t);
+  if (current != device) cudaSetDevice(current);
+  m->inbox = nullptr;
+  m->bytes = 0;
+}
+
 // Takes (or grows) the inboxes for a grid, in its stream's order.
 cudaError_t mesh_hold(int device, size_t bytes, cudaStream_t s) {
   MeshSpace* m = mesh_space(device);
   if (!m) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lk(m->mu);
-  cudaError_t e = cudaSuccess;
-  if (!m->done) e = cudaEventCreateWithFlags(&m->done, cudaEventDisableTiming);
-  if (e == cudaSuccess && bytes > m->bytes) {
-    char* p = nullptr;
+  if (bytes > m->bytes) {
+    MeshStream* self = mesh_stream(m, s);
     cudaMemPool_t pool = library_pool(device);
-    e = pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), bytes, pool, s)
-             : cudaErrorMemoryAllocation;
-    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, s);
-    if (e == cudaSuccess && m->inbox) {
-      e = cudaStreamWaitEvent(s, m->done, 0);
-      if (e == cudaSuccess) e = cudaFreeAsync(m->inbox, s);
-    }
-    if (e == cudaSuccess) e = cudaEventRecord(m->done, s);
+    if (!self || !pool) return cudaErrorMemoryAllocation;
+    char* p = nullptr;
+    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), bytes, pool, s);
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(p, 0, bytes, s);
+    // (other streams leave the new inboxes alone until they are cleared)
+    if (e == cudaSuccess) e = mesh_record(self, s);
     if (e != cudaSuccess) {
-      if (p) cudaFreeAsync(p, s);
+      cudaFreeAsync(p, s);
       return e;
     }
+    mesh_free_inbox(m, device);
     m->inbox = p;
     m->bytes = bytes;
     m->epoch = 0;
   }
-  if (e == cudaSuccess) ++m->users;
-  return e;
+  ++m->users;
+  return cudaSuccess;
 }
 
-void mesh_release(int device, cudaStream_t s) {
+void mesh_release(int device) {
   MeshSpace* m = mesh_space(device);
   if (!m) return;
   std::lock_guard<std::mutex> lk(m->mu);
   if (--m->users > 0) return;
-  if (m->inbox && cudaStreamWaitEvent(s, m->done, 0) == cudaSuccess) cudaFreeAsync(m->inbox, s);
-  m->inbox = nullptr;
-  m->bytes = 0;
-  if (m->done) cudaEventDestroy(m->done);
-  m->done = nullptr;
+  mesh_free_inbox(m, device);
+  for (MeshStream& e : m->streams) cudaEventDestroy(e.last);
+  m->streams.clear();
 }
 
-// One launch of `n` steps in the device's mesh order.
-cudaError_t launch_in_mesh_order(tws_grid* g, const MeshShape& shape, const StepArgs& a, int n) {
+// One launch of `n` steps, unless another stream's work is in its way (*ran).  A
+// grid of one CTA waits for no other and uses no inbox.
+cudaError_t launch_mesh_steps(tws_grid* g, const MeshShape& shape, const StepArgs& a, int n,
+                              bool* ran) {
+  *ran = false;
   MeshSpace* m = mesh_space(g->device);
   if (!m) return cudaErrorInvalidDevice;
   float* d[2] = {g->d[g->cur], g->d[g->cur ^ 1]};
   void* f[2] = {g->f[g->cur], g->f[g->cur ^ 1]};
   const unsigned x = (unsigned)mesh_exchanges(shape, n);
   std::lock_guard<std::mutex> lk(m->mu);
-  cudaError_t e = cudaStreamWaitEvent(g->stream, m->done, 0);
-  if (e == cudaSuccess && (mesh_inbox_bytes(shape) > m->bytes || !m->inbox))
-    e = cudaErrorInvalidValue;
-  if (e == cudaSuccess && m->epoch > 0xffffffffu - x) {  // the numbers start again
+  MeshStream* self = mesh_stream(m, g->stream);
+  if (!self || mesh_inbox_bytes(shape) > m->bytes || !m->inbox) return cudaErrorInvalidValue;
+  if (shape.tiles_x * shape.tiles_y > 1 && mesh_others_busy(m, self)) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  if (m->epoch > 0xffffffffu - x) {  // the numbers start again
     e = cudaMemsetAsync(m->inbox, 0, m->bytes, g->stream);
     m->epoch = 0;
   }
   if (e == cudaSuccess)
     e = launch_mesh(shape, g->flux_storage, g->b, d, f, a, n, m->inbox, m->epoch, g->stream);
   if (e == cudaSuccess) {
+    *ran = true;
     m->epoch += x;
-    e = cudaEventRecord(m->done, g->stream);
+    e = mesh_record(self, g->stream);
   }
   return e;
+}
+
+// After a call that the mesh kernel could have run.
+void mesh_note_steps(tws_grid* g) {
+  MeshSpace* m = mesh_space(g->device);
+  if (!m) return;
+  std::lock_guard<std::mutex> lk(m->mu);
+  MeshStream* self = mesh_stream(m, g->stream);
+  if (!self || mesh_record(self, g->stream) != cudaSuccess) cudaGetLastError();
 }
 
 StepArgs make_step_args(const tws_grid* g) {
@@ -361,11 +447,13 @@ StepArgs make_step_args(const tws_grid* g) {
   return a;
 }
 
+int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps);
+
 int enqueue_steps(tws_grid* g, int nsteps) {
-  StepArgs a = make_step_args(g);
+  const StepArgs a = make_step_args(g);
   const MeshShape* mesh = mesh_for(g, nsteps);
   if (mesh) {
-    // (the launches' order is kept by an event, which a capture cannot hold)
+    // (other streams' work is told by events, which a capture cannot record)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess ||
         cap != cudaStreamCaptureStatusNone) {
@@ -373,16 +461,24 @@ int enqueue_steps(tws_grid* g, int nsteps) {
       mesh = nullptr;
     }
   }
-  if (mesh) {
-    for (int left = nsteps; left > 0;) {
-      const int n = std::min(left, kResidentMaxSteps);
-      const cudaError_t e = launch_in_mesh_order(g, *mesh, a, n);
-      if (e != cudaSuccess) return cuda_fail(g, e, "mesh kernel launch");
-      g->cur ^= 1;
-      left -= n;
-    }
-    return TWS_OK;
+  int left = nsteps;
+  while (mesh && left > 0) {
+    const int n = std::min(left, kResidentMaxSteps);
+    bool ran = false;
+    const cudaError_t e = launch_mesh_steps(g, *mesh, a, n, &ran);
+    if (e != cudaSuccess) return cuda_fail(g, e, "mesh kernel launch");
+    if (!ran) break;
+    g->cur ^= 1;
+    left -= n;
   }
+  if (left == 0) return TWS_OK;
+  const int rc = enqueue_variant_steps(g, a, left);
+  if (mesh) mesh_note_steps(g);
+  return rc;
+}
+
+// Steps by the resident kernel or the variants.
+int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps) {
   if (const int ctas = resident_ctas(g, nsteps)) {
     for (int left = nsteps; left > 0;) {
       const int n = std::min(left, kResidentMaxSteps);
@@ -589,7 +685,7 @@ TWS_API int tws_destroy(tws_grid* g) {
     if (ev) cudaEventDestroy(ev);
   if (g->io_up) cudaStreamDestroy(g->io_up);
   if (g->io_down) cudaStreamDestroy(g->io_down);
-  if (g->mesh_user) mesh_release(g->device, g->stream);
+  if (g->mesh_user) mesh_release(g->device);
   if (g->slab) cudaFreeAsync(g->slab, g->stream);
   if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
   delete g;

@@ -1287,14 +1287,27 @@ EncodeTiledFn encode_fn(std::string* why) {
 cudaError_t kernel_limits(const void* fn, int threads, size_t smem, int* ctas_per_sm) {
   static KernelLimits limits;
   int dev = 0;
-  const cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  return limits.get(dev, fn, smem, ctas_per_sm, [&](int* n) {
+  // a thread's launches of one kernel follow one another (a call's steps): the
+  // last answer saves the lock and the search, 1-2% of a launch's host time
+  static thread_local struct {
+    const void* fn;
+    size_t smem;
+    int dev, ctas;
+  } last{};
+  if (last.fn == fn && last.dev == dev && last.smem == smem) {
+    *ctas_per_sm = last.ctas;
+    return cudaSuccess;
+  }
+  e = limits.get(dev, fn, smem, ctas_per_sm, [&](int* n) {
     const cudaError_t set =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return set != cudaSuccess ? set
                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, fn, threads, smem);
   });
+  if (e == cudaSuccess) last = {fn, smem, dev, *ctas_per_sm};
+  return e;
 }
 
 int step_variant_count() { return table().n; }
