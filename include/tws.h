@@ -195,8 +195,8 @@ TWS_API int tws_variant_info(int variant, int* steps_per_launch, int* tile_x, in
  * down a band of tile_y rows, the steps' time levels on chip; without a tail
  * the bands are taller where every resident warp still gets one, and idle warps
  * take over rows of others' bands.  tile_x = 64 - 4K names the column unit; a
- * strip is two of them side by side, 128 columns less their common halo).  Only the tile variants wait on barriers that
- * tws_set_wait_limit bounds. */
+ * strip is two of them side by side, 128 columns less their common halo).  Of the
+ * variants only the tiles wait on barriers that tws_set_wait_limit bounds. */
 #define TWS_VARIANT_TILE 0
 #define TWS_VARIANT_STREAM 1
 #define TWS_VARIANT_SWEEP 2
@@ -220,7 +220,10 @@ TWS_API int tws_current_variant(tws_grid* grid, int* variant);
  * no waits that can run out).  A step kernel waits on a barrier for each of
  * its tile loads; the wait gives up after `sm_cycles` SM clocks (0: the
  * default, about two seconds), sets the grid's error word and returns
- * without writing that tile.  The next tws_sync then reports TWS_ERR_TIMEOUT
+ * without writing that tile.  A wait of the mesh kernel (see tws_step) for its
+ * neighbours' borders gives up after `sm_cycles` and 20 million clocks (it
+ * includes the neighbours' steps), counted from when every tile of the launch
+ * has an SM, or after about half a minute if one does not get any.  The next tws_sync then reports TWS_ERR_TIMEOUT
  * once and clears the word; the state is undefined after it and must be
  * uploaded again, and the context stays usable.  (The test hook that makes
  * the waits run out is declared in tws_testing.h, not here.) */

@@ -15,7 +15,8 @@ extern "C" {
 #endif
 
 /* Failure-detection hook.  With drop = 1 every tile load of this grid's step
- * kernels arms its barrier for the tile's bytes but issues no copy, so each
+ * kernels arms its barrier for the tile's bytes but issues no copy, and the
+ * tiles of the mesh kernel send their neighbours nothing, so each
  * bounded wait (tws_set_wait_limit) runs out with nothing in flight: the
  * kernel records the time-out and returns, and the next tws_sync or
  * tws_batch_sync reports TWS_ERR_TIMEOUT once.  drop = 0 turns it off.

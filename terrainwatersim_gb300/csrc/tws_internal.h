@@ -203,14 +203,15 @@ constexpr int kMeshMaxCtas = 256;
 bool mesh_shape(int W, int H, int brushes, MeshShape* out);
 // Exchanges of a launch.
 int mesh_exchanges(const MeshShape& s, int nsteps);
-// Bytes of the CTAs' inboxes: zeroed once, then every exchange of every launch that
-// uses them has a number of its own (never 0).
+// Bytes of the workspace (a count, and the CTAs' inboxes): zeroed once, then every
+// exchange of every launch that uses it has a number of its own (never 0).
 size_t mesh_inbox_bytes(const MeshShape& s);
+inline int mesh_ctas(const MeshShape& s) { return s.tiles_x * s.tiles_y; }
 // d[0], f[0]: the state; d[1], f[1]: where the result goes.  `epoch`: the number of
-// the last exchange before.
+// the last exchange before, `begun`: the CTAs of all launches of several before.
 cudaError_t launch_mesh(const MeshShape& s, int flux_storage, const float* b, float* const d[2],
                         void* const f[2], const StepArgs& a, int nsteps, void* inbox,
-                        unsigned epoch, cudaStream_t st);
+                        unsigned epoch, unsigned begun, cudaStream_t st);
 
 // tws_aux.cu
 cudaError_t launch_apply_source(float* d, int W, int H, int pitch, const DevSource& s,

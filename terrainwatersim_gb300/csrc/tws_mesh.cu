@@ -23,7 +23,9 @@
 // halves used in turn: a word is overwritten two exchanges later, and its
 // reader has then sent the exchange in between.  All CTAs are resident
 // (cooperative launch), the waits are bounded like those of the tile kernels,
-// and a wait that runs out sets the grid's error word.
+// and a wait that runs out sets the grid's error word.  A CTA takes a whole SM and
+// may have to wait for one while another stream's kernels hold it, so the clocks of
+// a wait count from when every CTA has begun.
 //
 // What bounds it: the latency of one step's dependent chain and two barriers on
 // the smallest grids, instruction issue on the largest, and the exchange
@@ -52,6 +54,13 @@ constexpr int kMeshThreads = 32 * kMeshWarps;
 constexpr int kMeshCols = 64;
 constexpr int kMeshRowBytes = kMeshCols * 4;
 constexpr int kMeshBrushes = 2;  // brush sources a launch takes (one shared plane each)
+constexpr size_t kMeshHeadBytes = 256;  // of the workspace: the count of CTAs that have begun
+// An exchange waits for a neighbour's steps since the last one too, not for a load
+// alone, so this much comes on top of the grid's wait limit (about 10 ms; the longest
+// exchange of a sound launch takes microseconds).
+constexpr long long kMeshExchangeCycles = 20000000;
+// How long CTAs wait for others that have no SM yet (about half a minute).
+constexpr long long kMeshBeginCycles = 60000000000;
 
 struct MeshArgs {
   const float* b;
@@ -65,6 +74,10 @@ struct MeshArgs {
   ulonglong2* inbox;  // two halves per CTA, `half` pairs of words each
   int half;
   unsigned epoch;     // number of the last exchange before this launch
+  unsigned* begun;    // CTAs that have begun, of this launch and those before it
+  unsigned all;       // what it says once all of this launch's have
+  // clocks that a wait may take from when all have begun, and longer until then
+  long long limit, begin_limit;
 };
 
 // Two words of an inbox: each a value and, in its high half, the number of the
@@ -112,6 +125,18 @@ struct MeshRoute {
 };
 constexpr int kMeshChannels = 5;  // depth and the four outflows
 
+// After a wait that has run out once: until every CTA of the launch has begun (not
+// inlined, nor a part of the waiting loop: with its state there, the steps' registers
+// were allocated otherwise and 256^2 took 1655 us for 1000 steps, not 1620).  True
+// if some CTA has not.
+__device__ __noinline__ bool mesh_begin_runs_out(const unsigned* begun, unsigned all,
+                                                 long long limit) {
+  const long long t0 = clock64();
+  while ((int)(*(const volatile unsigned*)begun - all) < 0)
+    if (clock64() - t0 > limit) return true;
+  return false;
+}
+
 template <int RY, bool F16>
 __global__ void __launch_bounds__(kMeshThreads, 1)
     mesh_kernel(const __grid_constant__ StepArgs a, const __grid_constant__ MeshArgs m) {
@@ -122,6 +147,7 @@ __global__ void __launch_bounds__(kMeshThreads, 1)
   const int W = a.W, H = a.H;
   const size_t pitch = (size_t)a.pitch;
   const int tx = blockIdx.x % m.tiles_x, ty = blockIdx.x / m.tiles_x;
+  if (threadIdx.x == 0 && gridDim.x > 1) atomicAdd(m.begun, 1u);
   const int hx = m.hx, hy = m.hy;
   const int row0 = warp * RY;                                // box row of this warp's first row
   const int gx = tx * (kMeshCols - 2 * hx) - hx + 2 * lane;  // this lane's first column
@@ -382,7 +408,7 @@ __global__ void __launch_bounds__(kMeshThreads, 1)
     const int dy = r < hy ? -1 : (r >= ROWS - hy ? 1 : 0);
     auto exists = [&](int x, int y) { return x >= 0 && x < m.tiles_x && y >= 0 && y < m.tiles_y; };
     MeshRoute e{-1, 0};
-    if (exists(tx - dx, ty - dy)) {
+    if (exists(tx - dx, ty - dy) && !a.drop_loads) {  // (the test hook sends nothing)
       e.src = mesh_pair(RY, hx, hy, r - dy * (ROWS - 2 * hy), c - dx * (C - hx), 1);
       e.dst = (ty - dy) * m.tiles_x + tx - dx;
     }
@@ -554,19 +580,22 @@ __global__ void __launch_bounds__(kMeshThreads, 1)
     // ---- and the own inbox into shared memory
     bool late = false;
     const ulonglong2* const own_part = part + (size_t)blockIdx.x * 2 * m.half;
-    for (int q = threadIdx.x; q < pairs; q += kMeshThreads) {
+    for (int q = threadIdx.x; q < pairs && !late; q += kMeshThreads) {
       if (route[q].dst < 0) continue;
       ulonglong2 w[kMeshChannels];
-      const long long t0 = clock64();
-      for (;;) {
-        bool all = true;
+      for (int period = 0;; ++period) {  // the second one: from the last CTA's begin
+        bool all = false;
+        const long long t0 = clock64();
+        do {
 #pragma unroll
-        for (int ch = 0; ch < kMeshChannels; ++ch) w[ch] = words_load(own_part + ch * pairs + q);
+          for (int ch = 0; ch < kMeshChannels; ++ch) w[ch] = words_load(own_part + ch * pairs + q);
+          all = true;
 #pragma unroll
-        for (int ch = 0; ch < kMeshChannels; ++ch)
-          all &= (unsigned)(w[ch].x >> 32) == epoch && (unsigned)(w[ch].y >> 32) == epoch;
+          for (int ch = 0; ch < kMeshChannels; ++ch)
+            all &= (unsigned)(w[ch].x >> 32) == epoch && (unsigned)(w[ch].y >> 32) == epoch;
+        } while (!all && clock64() - t0 <= m.limit);
         if (all) break;
-        if (clock64() - t0 > a.wait_cycles) {
+        if (period > 0 || mesh_begin_runs_out(m.begun, m.all, m.begin_limit)) {
           late = true;
           break;
         }
@@ -669,13 +698,13 @@ bool mesh_shape(int W, int H, int brushes, MeshShape* out) {
 }
 
 size_t mesh_inbox_bytes(const MeshShape& s) {
-  return sizeof(ulonglong2) * 2 * kMeshChannels * mesh_pairs(s.ry, s.hx, s.hy) * s.tiles_x *
+  return kMeshHeadBytes + sizeof(ulonglong2) * 2 * kMeshChannels * mesh_pairs(s.ry, s.hx, s.hy) * s.tiles_x *
          s.tiles_y;
 }
 
 cudaError_t launch_mesh(const MeshShape& s, int flux_storage, const float* b, float* const d[2],
                         void* const f[2], const StepArgs& a, int nsteps, void* inbox,
-                        unsigned epoch, cudaStream_t st) {
+                        unsigned epoch, unsigned begun, cudaStream_t st) {
   MeshFn fn = mesh_fn(s.ry, flux_storage);
   if (!fn || nsteps < 1 || !inbox) return cudaErrorInvalidValue;
   const int smem = mesh_launch_smem(s);
@@ -697,7 +726,11 @@ cudaError_t launch_mesh(const MeshShape& s, int flux_storage, const float* b, fl
   m.every = alone ? nsteps : s.every;
   m.nsteps = nsteps;
   m.brushes = s.brushes;
-  m.inbox = static_cast<ulonglong2*>(inbox);
+  m.begun = static_cast<unsigned*>(inbox);
+  m.all = begun + (unsigned)mesh_ctas(s);
+  m.limit = std::min(a.wait_cycles, (long long)1 << 60) + kMeshExchangeCycles;
+  m.begin_limit = kMeshBeginCycles;
+  m.inbox = reinterpret_cast<ulonglong2*>(static_cast<char*>(inbox) + kMeshHeadBytes);
   m.half = kMeshChannels * mesh_pairs(s.ry, s.hx, s.hy);
   m.epoch = epoch;
   cudaLaunchAttribute attr[1];
