@@ -23,6 +23,13 @@ extern "C" {
  * Returns TWS_ERR_INVALID for other values. */
 TWS_API int tws_test_drop_tile_loads(tws_grid* grid, int drop);
 
+/* With refuse = 1 every launch of the mesh kernel (see tws_step) for this grid
+ * fails as one that is too large for its stream's SMs does
+ * (cudaErrorCooperativeLaunchTooLarge), before anything is launched: the calls
+ * run as the kernel variants.  refuse = 0 turns it off; TWS_ERR_INVALID for
+ * other values. */
+TWS_API int tws_test_refuse_mesh(tws_grid* grid, int refuse);
+
 #ifdef __cplusplus
 }
 #endif

@@ -115,6 +115,7 @@ def _declare(L):
         "tws_set_variant": ([vp, i], i),
         "tws_set_wait_limit": ([vp, C.c_longlong], i),
         "tws_test_drop_tile_loads": ([vp, i], i),
+        "tws_test_refuse_mesh": ([vp, i], i),
         "tws_autotune": ([vp, i, vp], i),
         "tws_resident_fits": ([i, i, i], i),
         "tws_set_resident": ([vp, i], i),
@@ -396,6 +397,10 @@ class Grid:
         issues no copy, so its bounded wait runs out with nothing in flight
         (False turns it off)."""
         _check(lib().tws_test_drop_tile_loads(self._h, 1 if drop else 0), self._h)
+
+    def test_refuse_mesh(self, refuse: bool = True):
+        """Test hook (tws_testing.h): launches of the mesh kernel are refused."""
+        _check(lib().tws_test_refuse_mesh(self._h, 1 if refuse else 0), self._h)
 
     def set_resident(self, on: bool = True, ctas: int | None = None):
         """Run the steps with the resident kernel (the whole grid in one

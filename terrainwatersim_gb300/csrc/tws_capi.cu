@@ -67,6 +67,7 @@ struct tws_grid {
   CUtensorMap* desc = nullptr;  // device copies of the maps, 5 per variant (batched kernel)
   long long wait_cycles = kDefaultWaitCycles;  // SM clocks a tile-load wait may take
   int drop_loads = 0;     // test hook: tile loads arm their barrier but issue no copy
+  int refuse_mesh = 0;    // test hook: mesh launches are refused
   tws_batch* batch = nullptr;  // batch this grid belongs to (its stream is the batch's)
   cudaStream_t home_stream = nullptr;
   // Asynchronous host I/O, made on first use: packed staging (upload b, d, f
@@ -389,19 +390,21 @@ void mesh_release(int device) {
   m->streams.clear();
 }
 
-// One launch of `n` steps, unless another stream's work is in its way (*ran).  A
-// grid of one CTA waits for no other and uses no inbox.
+// One launch of `n` steps, unless another stream's work is in its way or it is
+// refused (*ran false: nothing has been launched, the step kernels take over).  A
+// grid of one CTA waits for no other and uses no inbox.  Refused are more CTAs than
+// the stream has SMs for, as on a stream of a partition of the device.
 cudaError_t launch_mesh_steps(tws_grid* g, const MeshShape& shape, const StepArgs& a, int n,
                               bool* ran) {
   *ran = false;
   MeshSpace* m = mesh_space(g->device);
-  if (!m) return cudaErrorInvalidDevice;
+  if (!m) return cudaSuccess;
   float* d[2] = {g->d[g->cur], g->d[g->cur ^ 1]};
   void* f[2] = {g->f[g->cur], g->f[g->cur ^ 1]};
   const unsigned x = (unsigned)mesh_exchanges(shape, n);
   std::lock_guard<std::mutex> lk(m->mu);
   MeshStream* self = mesh_stream(m, g->stream);
-  if (!self || mesh_inbox_bytes(shape) > m->bytes || !m->inbox) return cudaErrorInvalidValue;
+  if (!self || mesh_inbox_bytes(shape) > m->bytes || !m->inbox) return cudaSuccess;
   if (mesh_ctas(shape) > 1 && mesh_others_busy(m, self)) return cudaSuccess;
   cudaError_t e = cudaSuccess;
   if (m->epoch > 0xffffffffu - x) {  // the numbers start again
@@ -409,15 +412,17 @@ cudaError_t launch_mesh_steps(tws_grid* g, const MeshShape& shape, const StepArg
     m->epoch = m->begun = 0;
   }
   if (e == cudaSuccess)
-    e = launch_mesh(shape, g->flux_storage, g->b, d, f, a, n, m->inbox, m->epoch, m->begun,
-                    g->stream);
-  if (e == cudaSuccess) {
-    *ran = true;
-    m->epoch += x;
-    if (mesh_ctas(shape) > 1) m->begun += (unsigned)mesh_ctas(shape);
-    e = mesh_record(self, g->stream);
+    e = g->refuse_mesh ? cudaErrorCooperativeLaunchTooLarge
+                       : launch_mesh(shape, g->flux_storage, g->b, d, f, a, n, m->inbox, m->epoch,
+                                     m->begun, g->stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (a context that is lost says so again)
+    return cudaSuccess;
   }
-  return e;
+  *ran = true;
+  m->epoch += x;
+  if (mesh_ctas(shape) > 1) m->begun += (unsigned)mesh_ctas(shape);
+  return mesh_record(self, g->stream);
 }
 
 // After a call that the mesh kernel could have run.
@@ -891,6 +896,12 @@ TWS_API int tws_set_wait_limit(tws_grid* g, long long sm_cycles) {
 TWS_API int tws_test_drop_tile_loads(tws_grid* g, int drop) {
   if (!g || (drop != 0 && drop != 1)) return fail(g, TWS_ERR_INVALID, "drop must be 0 or 1");
   g->drop_loads = drop;
+  return TWS_OK;
+}
+
+TWS_API int tws_test_refuse_mesh(tws_grid* g, int refuse) {
+  if (!g || (refuse != 0 && refuse != 1)) return fail(g, TWS_ERR_INVALID, "refuse must be 0 or 1");
+  g->refuse_mesh = refuse;
   return TWS_OK;
 }
 

@@ -744,7 +744,7 @@ cudaError_t launch_mesh(const MeshShape& s, int flux_storage, const float* b, fl
   cfg.attrs = attr;
   cfg.numAttrs = alone ? 0 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, a, m);
-  count_launch();
+  if (e == cudaSuccess) count_launch();
   return e;
 }
 
