@@ -278,9 +278,11 @@ TWS_API int tws_set_resident(tws_grid* grid, int ctas);
  * that finds step work of such a grid on another stream under way uses the
  * variants instead, beside it (grids of one CTA, up to 60 x 144 cells, run as one
  * launch all the same), and so does one whose launch is refused, as on a stream
- * with fewer SMs than the launch has tiles.  No stream waits for another.  Its waits for neighbouring tiles are bounded by
- * tws_set_wait_limit too, and a call being captured into a CUDA graph uses the
- * variants.  Results do not depend on the choice. */
+ * with fewer SMs than the launch has tiles.  No stream waits for another.  Its
+ * waits for neighbouring tiles are bounded by tws_set_wait_limit too.  Calls that
+ * are captured into a CUDA graph use the variants, and so do all later ones of
+ * such a grid: a graph finds the state only after as many changes of buffers as
+ * the variants make.  Results do not depend on the choice. */
 TWS_API int tws_step(tws_grid* grid, int nsteps);
 
 /* Total water volume sum(d) * cell_area, accumulated in FP64 on the device

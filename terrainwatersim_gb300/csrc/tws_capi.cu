@@ -52,6 +52,7 @@ struct tws_grid {
   bool mesh_fits = false;
   MeshShape mesh{};          // how the mesh kernel takes this grid
   bool mesh_user = false;    // this grid holds the device's mesh workspace
+  bool captured = false;     // a call has been captured into a CUDA graph
   int auto_ctas = -1;        // the resident kernel's automatic cluster for this grid (-1: not asked yet)
   std::vector<VariantMaps> maps;
   tws_source src[TWS_MAX_SOURCES];
@@ -240,7 +241,7 @@ int mesh_min_steps(const MeshShape& s) { return s.ry <= 4 ? 4 : s.ry <= 7 ? 8 : 
 // a variant, a steps-per-launch setting or the resident kernel is chosen or
 // the autotuner found another kernel faster for this grid shape.
 const MeshShape* mesh_for(tws_grid* g, int nsteps) {
-  if (!g->mesh_user || nsteps < 4 || g->resident > 0 || g->variant >= 0 || g->steps_per_launch != 0)
+  if (!g->mesh_user || g->captured || nsteps < 4 || g->resident > 0 || g->variant >= 0 || g->steps_per_launch != 0)
     return nullptr;
   int brushes = 0;
   for (int i = 0; i < g->nsrc; ++i) brushes += g->src[i].kind != TWS_SOURCE_DISK;
@@ -461,16 +462,18 @@ int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps);
 
 int enqueue_steps(tws_grid* g, int nsteps) {
   const StepArgs a = make_step_args(g);
-  const MeshShape* mesh = mesh_for(g, nsteps);
-  if (mesh) {
-    // (other streams' work is told by events, which a capture cannot record)
+  // A graph's launches read and write the buffers that they were captured with.
+  // The state changes buffers with every launch, once for a mesh call of any
+  // length: from a grid's first captured call on, mesh calls between replays
+  // would leave the state where the graph does not look for it.  (Nor can a capture
+  // record the events that tell of other streams' work.)
+  if (g->mesh_user && !g->captured) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      mesh = nullptr;
-    }
+    g->captured = cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess ||
+                  cap != cudaStreamCaptureStatusNone;
+    if (g->captured) cudaGetLastError();
   }
+  const MeshShape* mesh = mesh_for(g, nsteps);
   int left = nsteps;
   while (mesh && left > 0) {
     const int n = std::min(left, kResidentMaxSteps);
