@@ -170,11 +170,15 @@ struct TunedKey {
     return w != o.w ? w < o.w : (h != o.h ? h < o.h : fs < o.fs);
   }
 };
-// The fastest variant, and whether the resident or the mesh kernel beat it.
+// The fastest variant, whether the resident kernel beat it, and how the mesh kernel
+// did against both.  It is not tried where it could not run when the grid was tuned
+// (too many brush sources, another stream's work): that says nothing about later
+// grids of the shape.
+enum class MeshTrial { kNone, kWon, kLost };
 struct Tuned {
   int variant = -1;
   bool resident = false;
-  bool mesh = false;
+  MeshTrial mesh = MeshTrial::kNone;
 };
 std::mutex g_tuned_mu;
 std::map<TunedKey, Tuned> g_tuned;
@@ -236,13 +240,10 @@ int resident_ctas(tws_grid* g, int nsteps) {
 // 113 and 116.
 int mesh_min_steps(const MeshShape& s) { return s.ry <= 4 ? 4 : s.ry <= 7 ? 8 : 12; }
 
-// How the mesh kernel runs a call of `nsteps` steps, or null if it does not: it
-// runs the calls of at least mesh_min_steps steps on grids that fit it, unless
-// a variant, a steps-per-launch setting or the resident kernel is chosen or
-// the autotuner found another kernel faster for this grid shape.
-const MeshShape* mesh_for(tws_grid* g, int nsteps) {
-  if (!g->mesh_user || g->captured || nsteps < 4 || g->resident > 0 || g->variant >= 0 || g->steps_per_launch != 0)
-    return nullptr;
+// How the mesh kernel can run a call of `nsteps` steps, or null: calls of at least
+// mesh_min_steps steps on grids that fit it.
+const MeshShape* mesh_fit(tws_grid* g, int nsteps) {
+  if (!g->mesh_user || g->captured || nsteps < 4) return nullptr;
   int brushes = 0;
   for (int i = 0; i < g->nsrc; ++i) brushes += g->src[i].kind != TWS_SOURCE_DISK;
   if (g->mesh_brushes != brushes) {
@@ -252,9 +253,16 @@ const MeshShape* mesh_for(tws_grid* g, int nsteps) {
   if (!g->mesh_fits || nsteps < mesh_min_steps(g->mesh)) return nullptr;
   // (the test hook is for waits that run out: a call without an exchange has none)
   if (g->drop_loads && mesh_exchanges(g->mesh, nsteps) == 0) return nullptr;
-  const Tuned t = tuned_lookup(g);
-  if (t.variant >= 0 && !t.mesh) return nullptr;
   return &g->mesh;
+}
+
+// The same where it also is to: unless a variant, a steps-per-launch setting or the
+// resident kernel is chosen, or the autotuner found another kernel faster for this
+// grid shape.
+const MeshShape* mesh_for(tws_grid* g, int nsteps) {
+  if (g->resident > 0 || g->variant >= 0 || g->steps_per_launch != 0) return nullptr;
+  const MeshShape* mesh = mesh_fit(g, nsteps);
+  return mesh && tuned_lookup(g).mesh != MeshTrial::kLost ? mesh : nullptr;
 }
 
 // The mesh kernel's inboxes, one set per device, held by the grids that the kernel
@@ -458,6 +466,21 @@ StepArgs make_step_args(const tws_grid* g) {
   return a;
 }
 
+// As many of the steps as the mesh kernel runs now; *left: the others.
+int enqueue_mesh_steps(tws_grid* g, const MeshShape& shape, const StepArgs& a, int nsteps,
+                       int* left) {
+  for (*left = nsteps; *left > 0;) {
+    const int n = std::min(*left, kResidentMaxSteps);
+    bool ran = false;
+    const cudaError_t e = launch_mesh_steps(g, shape, a, n, &ran);
+    if (e != cudaSuccess) return cuda_fail(g, e, "mesh kernel launch");
+    if (!ran) break;
+    g->cur ^= 1;
+    *left -= n;
+  }
+  return TWS_OK;
+}
+
 int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps);
 
 int enqueue_steps(tws_grid* g, int nsteps) {
@@ -475,17 +498,9 @@ int enqueue_steps(tws_grid* g, int nsteps) {
   }
   const MeshShape* mesh = mesh_for(g, nsteps);
   int left = nsteps;
-  while (mesh && left > 0) {
-    const int n = std::min(left, kResidentMaxSteps);
-    bool ran = false;
-    const cudaError_t e = launch_mesh_steps(g, *mesh, a, n, &ran);
-    if (e != cudaSuccess) return cuda_fail(g, e, "mesh kernel launch");
-    if (!ran) break;
-    g->cur ^= 1;
-    left -= n;
-  }
-  if (left == 0) return TWS_OK;
-  const int rc = enqueue_variant_steps(g, a, left);
+  int rc = mesh ? enqueue_mesh_steps(g, *mesh, a, nsteps, &left) : TWS_OK;
+  if (rc != TWS_OK || left == 0) return rc;
+  rc = enqueue_variant_steps(g, a, left);
   if (mesh) mesh_note_steps(g);
   return rc;
 }
@@ -977,28 +992,25 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
     g->resident = 0;
   }
   // and the mesh kernel
-  {
-    std::lock_guard<std::mutex> lk(g_tuned_mu);
-    g_tuned.erase(TunedKey{g->W, g->H, g->flux_storage});
-  }
-  const int saved_spl = g->steps_per_launch;
-  g->variant = -1;
-  g->steps_per_launch = 0;
-  if (rc == TWS_OK && mesh_for(g, steps)) {
+  const MeshShape* mesh = mesh_fit(g, steps);
+  bool mesh_tried = rc == TWS_OK && mesh;
+  if (mesh_tried) {
+    const StepArgs a = make_step_args(g);
     float mbest = 1e30f;
-    for (int rep = 0; rep < 2 && rc == TWS_OK; ++rep) {
+    for (int rep = 0; rep < 2 && rc == TWS_OK && mesh_tried; ++rep) {
       restore();
+      int left = 0;
       cudaEventRecord(e0, g->stream);
-      rc = enqueue_steps(g, steps);
+      rc = enqueue_mesh_steps(g, *mesh, a, steps, &left);
       cudaEventRecord(e1, g->stream);
+      mesh_tried = left == 0;
       if (cudaEventSynchronize(e1) != cudaSuccess) rc = TWS_ERR_CUDA;
       float ms = 0.0f;
       cudaEventElapsedTime(&ms, e0, e1);
       mbest = std::min(mbest, ms);
     }
-    mesh_best = rc == TWS_OK && mbest < best_ms;
+    mesh_best = rc == TWS_OK && mesh_tried && mbest < best_ms;
   }
-  g->steps_per_launch = saved_spl;
   cudaGetLastError();  // a grid that does not fit leaves the query's error behind
   restore();
   cudaFreeAsync(saved, g->stream);
@@ -1017,7 +1029,10 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
   const int choice = resident_best ? TWS_VARIANT_RESIDENT : best;
   {
     std::lock_guard<std::mutex> lk(g_tuned_mu);
-    g_tuned[TunedKey{g->W, g->H, g->flux_storage}] = Tuned{best, resident_best, mesh_best};
+    Tuned& t = g_tuned[TunedKey{g->W, g->H, g->flux_storage}];
+    t.variant = best;
+    t.resident = resident_best;
+    if (mesh_tried) t.mesh = mesh_best ? MeshTrial::kWon : MeshTrial::kLost;
   }
   if (chosen) *chosen = choice;
   return TWS_OK;
