@@ -239,8 +239,9 @@ TWS_API int tws_set_wait_limit(tws_grid* grid, long long sm_cycles);
  * Where the mesh kernel (see tws_step) fits and beats them all, no variant is
  * pinned: it goes on running the calls long enough for it, and the chosen
  * variant the shorter ones.
- * Synchronous.  `chosen` (may be NULL) receives the variant index, or
- * TWS_VARIANT_RESIDENT if the resident kernel was fastest.  No counterpart
+ * Synchronous.  `chosen` (may be NULL) receives the variant index (with the mesh
+ * kernel ahead: of the calls too short for it), or TWS_VARIANT_RESIDENT if the
+ * resident kernel was fastest of all.  No counterpart
  * in the reference. */
 #define TWS_VARIANT_RESIDENT (-2)
 TWS_API int tws_autotune(tws_grid* grid, int trial_steps, int* chosen);

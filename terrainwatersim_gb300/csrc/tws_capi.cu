@@ -1026,7 +1026,8 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
   // calls, the fastest variant the short ones
   g->variant = resident_best || mesh_best ? -1 : best;
   g->resident = 0;
-  const int choice = resident_best ? TWS_VARIANT_RESIDENT : best;
+  // (the mesh kernel, which is not a variant, goes before both)
+  const int choice = resident_best && !mesh_best ? TWS_VARIANT_RESIDENT : best;
   {
     std::lock_guard<std::mutex> lk(g_tuned_mu);
     Tuned& t = g_tuned[TunedKey{g->W, g->H, g->flux_storage}];

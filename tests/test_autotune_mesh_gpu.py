@@ -36,3 +36,24 @@ def test_tuning_where_the_mesh_kernel_cannot_run_does_not_rule_it_out(tws):
         assert launches(tws, g, 40) > 1
     with scene(tws, W, H) as g:
         assert launches(tws, g, 40) == 1
+
+
+@pytest.mark.parametrize("W,H", [(64, 48), (72, 64)])
+def test_resident_is_reported_where_it_runs(tws, W, H):
+    """Lost borders (the test hook) end a mesh launch; the resident kernel has no
+    such wait."""
+    with scene(tws, W, H) as g:
+        best = g.autotune(240)
+        g.set_wait_limit(2_000_000)
+        g.test_drop_tile_loads(True)
+        n = 0
+        try:
+            n = launches(tws, g, 40)
+            mesh = False
+        except tws.TwsError as e:
+            assert e.code == tws.ERR_TIMEOUT
+            mesh = True
+        if best == tws.VARIANT_RESIDENT:
+            assert not mesh and n == 1
+        else:
+            assert 0 <= best < len(tws.variants())
