@@ -232,7 +232,8 @@ TWS_API int tws_set_wait_limit(tws_grid* grid, long long sm_cycles);
 /* Autotuner: times every variant for `trial_steps` steps on this grid's
  * current state (restored afterwards, so the simulation is unchanged), picks
  * the fastest per cell-step, pins it on this grid and records it for every
- * later grid of the same width, height and flux storage in this process.
+ * later grid of the same width, height and flux storage in this process.  The
+ * choice goes before an earlier tws_set_steps_per_launch.
  * Where the grid fits the resident kernel (below), that is timed too; if it
  * is fastest, it runs every later tws_step call of at least 16 steps on
  * grids of this shape, and the fastest tiled variant the shorter calls.

@@ -1023,8 +1023,10 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
     return rc;
   }
   // with a resident or mesh kernel ahead nothing is pinned: it runs the long
-  // calls, the fastest variant the short ones
+  // calls, the fastest variant the short ones (a steps-per-launch setting, which
+  // bars both, gives way as it does to a pinned variant)
   g->variant = resident_best || mesh_best ? -1 : best;
+  if (g->variant < 0) g->steps_per_launch = 0;
   g->resident = 0;
   // (the mesh kernel, which is not a variant, goes before both)
   const int choice = resident_best && !mesh_best ? TWS_VARIANT_RESIDENT : best;

@@ -57,3 +57,16 @@ def test_resident_is_reported_where_it_runs(tws, W, H):
             assert not mesh and n == 1
         else:
             assert 0 <= best < len(tws.variants())
+
+
+def test_tuning_supersedes_a_steps_per_launch_setting(tws):
+    with scene(tws, 208, 176) as g:
+        g.set_steps_per_launch(1)
+        assert launches(tws, g, 40) == 40
+        best = g.autotune(240)
+        n = launches(tws, g, 40)
+        if best == tws.VARIANT_RESIDENT:
+            assert n == 1
+        else:
+            assert n in (1, 40 // tws.variants()[best][0])
+            assert n < 40
