@@ -489,7 +489,8 @@ TWS_API int tws_server_result(tws_server* server, int index, tws_result* out);
 TWS_API int tws_server_stats(tws_server* server, double* cell_steps, double* seconds,
                              double* peak_bytes, uint64_t* chains);
 
-/* Device bytes a grid of this size holds (tws_create's allocations). */
+/* Device bytes that tws_create allocates for a grid of this size alone (the mesh
+ * kernel's workspace, see tws_step, is one for all grids of a device). */
 TWS_API double tws_grid_bytes(int width, int height, int flux_storage);
 
 /* Block the host until the grid's queued work (asynchronous host copies

@@ -148,6 +148,35 @@ float pick_flux_scale(float d_max, float c) {
 // The error word, the sweep kernel's queues (at byte 16) and its ranges (at 64).
 constexpr size_t kScratchBytes = 64 + sizeof(unsigned long long) * kSweepMaxWarps;
 
+int pitch_of(int width) { return (width + 31) / 32 * 32; }
+
+// Where the parts of a grid's one allocation lie.
+struct GridLayout {
+  size_t b, d[2], f[2], v, scratch;
+  size_t zeroed;  // everything up to here starts as zero
+  size_t partials, volume, maps;
+  size_t bytes = 0;
+  GridLayout(int width, int height, int flux_storage) {
+    const size_t n = (size_t)pitch_of(width) * height, fb = flux_bytes_per_cell(flux_storage);
+    b = take(n * 4);
+    for (size_t& o : d) o = take(n * 4);
+    for (size_t& o : f) o = take(n * fb);
+    v = take(n * 8);
+    scratch = take(kScratchBytes);
+    zeroed = bytes;
+    partials = take(sizeof(double) * volume_partials_needed());
+    volume = take(sizeof(double));
+    maps = take(sizeof(CUtensorMap) * 5 * step_variant_count());
+  }
+
+ private:
+  size_t take(size_t size) {
+    const size_t o = bytes;
+    bytes += (size + 255) / 256 * 256;
+    return o;
+  }
+};
+
 VariantMaps* maps_for(tws_grid* g, int variant, std::string* why) {
   if ((int)g->maps.size() < step_variant_count()) g->maps.resize(step_variant_count());
   VariantMaps& m = g->maps[variant];
@@ -618,7 +647,7 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
   if (!g) return TWS_ERR_OOM;
   g->W = width;
   g->H = height;
-  g->pitch = (width + 31) / 32 * 32;
+  g->pitch = pitch_of(width);
   g->params = *params;
   g->flux_storage = flux_storage;
   g->flux_scale = flux_storage == TWS_FLUX_F16
@@ -644,43 +673,32 @@ TWS_API int tws_create(int width, int height, const tws_sim_params* params, int 
       return bail(TWS_ERR_CUDA);
     g->own_stream = true;
   }
-  const size_t n = (size_t)g->pitch * g->H;
-  const size_t fb = flux_bytes_per_cell(flux_storage);
   // All device state in one stream-ordered allocation from the library's
   // pool: creating and destroying grids (the serving loop does it per
   // request) never synchronises the device.
-  size_t off = 0;
-  auto take = [&](size_t bytes) {
-    const size_t o = off;
-    off += (bytes + 255) / 256 * 256;
-    return o;
-  };
-  const size_t ob = take(n * 4), od0 = take(n * 4), od1 = take(n * 4), of0 = take(n * fb),
-               of1 = take(n * fb), ov = take(n * 8), oe = take(kScratchBytes), zeroed = off,
-               op = take(sizeof(double) * volume_partials_needed()), oo = take(sizeof(double)),
-               ot = take(sizeof(CUtensorMap) * 5 * step_variant_count());
+  const GridLayout at(width, height, flux_storage);
   cudaMemPool_t pool = library_pool(g->device);
-  if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&g->slab), off, pool, g->stream) !=
+  if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&g->slab), at.bytes, pool, g->stream) !=
                    cudaSuccess) {
     cudaGetLastError();
     return bail(TWS_ERR_OOM);
   }
-  g->b = reinterpret_cast<float*>(g->slab + ob);
-  g->d[0] = reinterpret_cast<float*>(g->slab + od0);
-  g->d[1] = reinterpret_cast<float*>(g->slab + od1);
-  g->f[0] = g->slab + of0;
-  g->f[1] = g->slab + of1;
-  g->v = reinterpret_cast<float2*>(g->slab + ov);
-  g->vol_partials = reinterpret_cast<double*>(g->slab + op);
-  g->vol_out = reinterpret_cast<double*>(g->slab + oo);
-  g->err = reinterpret_cast<int*>(g->slab + oe);
-  g->queue = reinterpret_cast<int*>(g->slab + oe + 16);
-  g->ranges = reinterpret_cast<unsigned long long*>(g->slab + oe + 64);
-  g->desc = reinterpret_cast<CUtensorMap*>(g->slab + ot);
+  g->b = reinterpret_cast<float*>(g->slab + at.b);
+  for (int i = 0; i < 2; ++i) {
+    g->d[i] = reinterpret_cast<float*>(g->slab + at.d[i]);
+    g->f[i] = g->slab + at.f[i];
+  }
+  g->v = reinterpret_cast<float2*>(g->slab + at.v);
+  g->err = reinterpret_cast<int*>(g->slab + at.scratch);
+  g->queue = reinterpret_cast<int*>(g->slab + at.scratch + 16);
+  g->ranges = reinterpret_cast<unsigned long long*>(g->slab + at.scratch + 64);
+  g->vol_partials = reinterpret_cast<double*>(g->slab + at.partials);
+  g->vol_out = reinterpret_cast<double*>(g->slab + at.volume);
+  g->desc = reinterpret_cast<CUtensorMap*>(g->slab + at.maps);
   // Zero the state and the scratch, padding included (the F16 flux map reads the
   // padding cell of odd-width rows and relies on it staying zero): the front of
   // the allocation, in one fill.
-  cudaMemsetAsync(g->slab, 0, zeroed, g->stream);
+  cudaMemsetAsync(g->slab, 0, at.zeroed, g->stream);
   // the mesh kernel's workspace, where it fits this grid (whatever its sources)
   size_t inbox = 0;
   for (int brushes = 0; brushes <= TWS_MAX_SOURCES; ++brushes) {
@@ -1969,9 +1987,7 @@ TWS_API const char* tws_batch_last_error(tws_batch* b) {
 
 TWS_API double tws_grid_bytes(int width, int height, int flux_storage) {
   if (width < 1 || height < 1) return 0.0;
-  const double cells = (double)((width + 31) / 32 * 32) * height;
-  return cells * (4.0 + 8.0 + 2.0 * flux_bytes_per_cell(flux_storage) + 8.0) +
-         sizeof(double) * (volume_partials_needed() + 1) + sizeof(int);
+  return (double)GridLayout(width, height, flux_storage).bytes;
 }
 
 TWS_API int tws_batch_stats(tws_batch* b, uint64_t* chains, uint64_t* graph_launches) {
