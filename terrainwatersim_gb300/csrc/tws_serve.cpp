@@ -1,5 +1,6 @@
 // tws_serve.cpp -- the serving loop: continuous batching of simulation
-// requests over one GPU, written against the public C ABI (include/tws.h).
+// requests over one GPU, written against the public C ABI (include/tws.h; its grids
+// are made without the mesh kernel's workspace, tws_grids.h).
 //
 // Batched mode, per iteration:
 //   1. enqueue one chain (up to chain_steps steps) for every resident grid;
@@ -24,6 +25,7 @@
 #include <vector>
 
 #include "../../include/tws.h"
+#include "tws_grids.h"
 
 namespace {
 
@@ -69,7 +71,7 @@ bool valid_request(const tws_request& r) {
 // Create the grid of a request and queue its scene on the grid's stream.
 int make_grid(const tws_server_config& cfg, const tws_request& r, tws_grid** out) {
   tws_grid* g = nullptr;
-  int rc = tws_create(r.width, r.height, &r.params, cfg.flux_storage, nullptr, &g);
+  int rc = tws::create_grid(r.width, r.height, &r.params, cfg.flux_storage, nullptr, &g);
   if (rc != TWS_OK) return rc;
   rc = tws_generate_scene(g, r.seed, r.height_scale, r.fill);
   if (rc == TWS_OK) rc = tws_set_sources(g, r.sources, r.nsources);
@@ -178,6 +180,7 @@ int run_batched(tws_server* s) {
       tws_volume(a.grid, &res.volume);
       if (a.grid && tws_batch_size(batch) > 0) tws_batch_remove(batch, a.grid);
       if (cfg.keep_grids) {
+        tws::take_mesh_workspace(a.grid);  // its new owner may step it by itself
         res.grid = a.grid;
       } else {
         tws_destroy(a.grid);
@@ -305,10 +308,12 @@ int run_serial(tws_server* s) {
     res.status = rc;
     res.done_s = since(t0);
     if (g) {
-      if (cfg.keep_grids && rc == TWS_OK)
+      if (cfg.keep_grids && rc == TWS_OK) {
+        tws::take_mesh_workspace(g);
         res.grid = g;
-      else
+      } else {
         tws_destroy(g);
+      }
     }
     s->results.push_back(res);
   }
