@@ -1726,7 +1726,23 @@ int run_chain(tws_batch* b, int variant, const std::vector<int>& launches) {
 // 3857 against 4730; 16 x 1024^2, radius 64, 34% 5393 against 5355; 64 x 512^2,
 // radius 16, 48% 6380 against 5595; two disks of radius 64: 8 x 1024^2, 7% 2701
 // against 2477, 16 x 1024^2, 9% 4352 against 4716).
+// The sizes alone are looked at first: they rule out the sweep for batches of many
+// small grids, and the search for the bands, dozens of passes over the members, was
+// a fifth of a millisecond of every call with 2000 of them.
 bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
+  const long long cols = batch_sweep_columns();
+  const long long least =
+      b->flux_storage == TWS_FLUX_F16 ? kBatchSweepF16Cells : kBatchSweepCells;
+  long long cells = 0, strips = 0, tiles = 0;
+  for (size_t i = 0; i < steps.size(); ++i) {
+    if (steps[i] < kBatchSweepK) continue;
+    const long long W = b->grids[i]->W, H = b->grids[i]->H;
+    cells += W * H;
+    strips += (W + cols - 1) / cols * cols * H;
+    tiles += (W + 31) / 32 * 32 * ((H + 31) / 32 * 32);
+  }
+  if (cells < least || 20 * strips > 23 * tiles) return false;
+
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess ||
       cap != cudaStreamCaptureStatusNone) {
@@ -1741,15 +1757,12 @@ bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
     cudaGetLastError();
     return false;
   }
-  const long long cols = batch_sweep_columns(), rows = sweep_band_rows(b, part, warps);
-  long long cells = 0, strips = 0, tiles = 0, units = 0, wet = 0;
+  const long long rows = sweep_band_rows(b, part, warps);
+  long long units = 0, wet = 0;
   for (size_t i = 0; i < part.size(); ++i) {
     if (part[i] == 0) continue;
     const tws_grid* g = b->grids[i];
-    const long long W = g->W, H = g->H, s = (W + cols - 1) / cols, n = s * ((H + rows - 1) / rows);
-    cells += W * H;
-    strips += s * cols * H;
-    tiles += (W + 31) / 32 * 32 * ((H + 31) / 32 * 32);
+    const long long W = g->W, H = g->H, n = (W + cols - 1) / cols * ((H + rows - 1) / rows);
     units += n;
     long long w = 0;
     for (int k = 0; k < g->nsrc; ++k) {
@@ -1760,10 +1773,8 @@ bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
     }
     wet += std::min(w, n);
   }
-  const long long least =
-      b->flux_storage == TWS_FLUX_F16 ? kBatchSweepF16Cells : kBatchSweepCells;
-  return units > 0 && units < kSweepMaxUnits / 2 && 20 * strips <= 23 * tiles &&
-         4 * wet <= units && (double)cells >= (double)least * (1.0 + 5.0 * (double)wet / (double)units);
+  return units > 0 && units < kSweepMaxUnits / 2 && 4 * wet <= units &&
+         (double)cells >= (double)least * (1.0 + 5.0 * (double)wet / (double)units);
 }
 
 // Advance member i by steps[i] steps, in chains of up to kChainSteps steps (of
