@@ -271,9 +271,11 @@ TWS_API int tws_set_resident(tws_grid* grid, int ctas);
  * Terrain::PerformSimulationStep (Terrain.cpp:253-265).  Asynchronous.
  *
  * With nothing pinned (no variant, no steps-per-launch setting, no resident
- * kernel), calls of at least 4 steps (8 from about half a million cells on, 12
- * from about 0.8 million) on grids of up to about 1.1 million cells with at most
- * two brush sources run as one launch of the mesh kernel: the state stays on
+ * kernel), calls of at least 4 steps (8 from about 0.35 million cells on, 12 from
+ * 0.8 million; 32 above 1.1 million, and with a brush above 0.9 million) on grids
+ * of up to about 1.2 million cells (with two brush sources 0.95 million, with more
+ * of them none) run as one launch of
+ * the mesh kernel (on long narrow grids the limits are lower): the state stays on
  * chip, spread over all SMs, whose tiles exchange their borders every few steps.
  * Mesh launches of one device share one workspace of up to some tens of MB, which
  * goes with the last grid that could use it, and never run side by side: a call

@@ -267,8 +267,13 @@ int resident_ctas(tws_grid* g, int nsteps) {
 // mesh kernel and with two-step tiles, a rain disk: 64^2, 4 steps 9.4 and 13.8; 512^2,
 // 4 steps 17.1 and 16.9, 8 steps 27.5 and 33.0; 1021 x 763, 8 steps 50.8 and 51.3, 16
 // steps 91 and 101; 1024^2, 8 steps 63.4 and 58.8, 12 steps 88.1 and 87.9, 16 steps
-// 113 and 116.
-int mesh_min_steps(const MeshShape& s) { return s.ry <= 4 ? 4 : s.ry <= 7 ? 8 : 12; }
+// 113 and 116.  The largest grids with a brush exchange after every step, which
+// longer calls have to repay (1024^2, one brush, against the two-step tiles of before
+// the mesh kernel: 12 steps 102 and 96, 40 steps 311 and 317; 1100^2, 40 steps 315, with
+// the present tiles 324).
+int mesh_min_steps(const MeshShape& s) {
+  return s.ry <= 4 ? 4 : s.ry <= 7 ? 8 : s.every > 1 ? 12 : 32;
+}
 
 // How the mesh kernel can run a call of `nsteps` steps, or null: calls of at least
 // mesh_min_steps steps on grids that fit it.
