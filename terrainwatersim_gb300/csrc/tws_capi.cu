@@ -235,7 +235,7 @@ int chosen_variant(const tws_grid* g) {
     if (v >= 0) return v;
   }
   const int k = g->steps_per_launch > 0 ? g->steps_per_launch : default_steps_per_launch(g);
-  return step_variant_for(k, g->flux_storage, (long long)g->W * g->H);
+  return step_variant_for(k, g->flux_storage, g->W, g->H);
 }
 
 // Calls shorter than this keep the tiled kernels when the resident kernel
@@ -563,7 +563,7 @@ int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps) {
   while (left > 0) {
     const int k = std::min(kmax, left);
     // the remainder of a chain that is not a multiple of K runs shallower
-    const int variant = k == kmax ? main_variant : step_variant_for(k, g->flux_storage, (long long)g->W * g->H);
+    const int variant = k == kmax ? main_variant : step_variant_for(k, g->flux_storage, g->W, g->H);
     VariantMaps* m = nullptr;
     if (step_variant(variant).kind == kKindTile) {
       m = maps_for(g, variant, &why);

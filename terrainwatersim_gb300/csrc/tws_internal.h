@@ -148,10 +148,10 @@ constexpr long long kDefaultWaitCycles = 4000000000LL;
 cudaError_t kernel_limits(const void* fn, int threads, size_t smem, int* ctas_per_sm);
 int step_variant_count();
 const StepVariant& step_variant(int i);
-constexpr long long kSmallStepCells = 4LL << 20;
-int step_variant_for(int k, int flux_storage, long long cells);
+constexpr long long kSmallStepTiles = 4096;  // of 32 x 32 cells
+int step_variant_for(int k, int flux_storage, int W, int H);
 // The automatic choice for grids of at least kLargeGridCells cells (FP16
-// flux: kLargeF16Cells), or -1.
+// flux: kLargeF16Cells), or -1 (smaller ones).
 constexpr long long kLargeGridCells = 7LL << 20;
 constexpr long long kLargeF16Cells = 17LL << 20;
 int step_variant_large_grid(int flux_storage, int W, int H);
@@ -172,6 +172,7 @@ size_t sweep_smem_bytes(int k, int flux_storage);
 // The column unit that the variant table names a sweep by: 64 columns less their
 // halo.  A warp sweeps two such halves side by side (128 columns).
 constexpr int sweep_column_unit(int k) { return 64 - 4 * k; }
+constexpr int sweep_strip_columns(int k) { return 128 - 2 * ((2 * k + 3) / 4 * 4); }
 // tws_stream.cu
 cudaError_t launch_stream_step(int ry, int flux_storage, const float* b, const float* d,
                                const void* f, const StepArgs& a, cudaStream_t s);

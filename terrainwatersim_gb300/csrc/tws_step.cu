@@ -1327,6 +1327,15 @@ int step_variant_large_grid(int flux_storage, int W, int H) {
   const long long cells = (long long)W * H;
   if (cells < kLargeGridCells) return -1;
   if (flux_storage != TWS_FLUX_F32 && cells < kLargeF16Cells) return -1;
+  // A narrow grid wastes much of its last strip (112 columns that count): the sweep
+  // holds its own while the strips cover at most 1.4 times the columns of 32-wide
+  // tiles (us per step, sweep and two-step tiles, one disk): 16 x 475000 (3.5 times)
+  // 169 and 78, the plain kernel 96; 56 x 135714 (1.75) 57 and 48, 113 x 67256 57 and 47,
+  // FP16 64 x 284375 124 and 98; 144 x 88888 (1.40) 72.9 and 73.4, 256 x 50000 (1.31)
+  // 61.6 and 64.8, 72 x 105555 (1.17) 47.5 and 54.3.
+  const long long cols = sweep_strip_columns(3);
+  const long long covered = (W + cols - 1) / cols * cols, tiled = (W + 31) / 32 * 32;
+  if (5 * covered > 7 * tiled) return step_variant_for(2, flux_storage, W, H);
   static const int kLadder[][2] = {{32, 0}, {40, 0}, {80, 32}, {128, 48}, {192, 48}, {256, 64}};
   static const int sms = [] {
     int dev = 0, n = 0;
@@ -1351,14 +1360,16 @@ int step_variant_large_grid(int flux_storage, int W, int H) {
   return pick;
 }
 
-int step_variant_for(int k, int /*flux_storage*/, long long cells) {
+int step_variant_for(int k, int /*flux_storage*/, int W, int H) {
   // Default variant per temporal depth (fastest per depth on 4096^2): the
   // plain 32x32 kernel for K = 1, the unified-layout 32x32 tiles for K > 1.
   // One step on a smaller grid takes 32x16 tiles, twice as many CTAs (us per
   // launch, FP32, against 32x32): 256^2 4.1 (5.8), 512^2 5.1 (6.4), 1024^2 10.6
-  // (11.1), 2048^2 39.5 (39.9).
+  // (11.1), 2048^2 39.5 (39.9).  What counts is the number of tiles: 8 x 500000, of
+  // as few cells as 2048^2 but four times the tiles, takes 109 (93).
+  const long long tiles = (long long)((W + 31) / 32) * ((H + 31) / 32);
   switch (k) {
-    case 1: return cells < kSmallStepCells ? 5 : 0;
+    case 1: return tiles < kSmallStepTiles ? 5 : 0;
     case 2: return 16;
     case 3: return 18;
     case 4: return 20;

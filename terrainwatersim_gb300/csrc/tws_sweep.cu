@@ -112,6 +112,7 @@ struct SweepRing {
   static constexpr int N = F + sweep_flux_row_bytes(F16);
   static constexpr int NSLOT = kSweepSlotBytes;
   static constexpr int WARP = sweep_warp_bytes(K, F16);
+  static_assert(sweep_strip_columns(K) == kSweepCols - 2 * kSweepHaloX(K), "columns that count");
   static_assert(WARP == N + (K - 1) * 2 * NSLOT && PB >= 2 * K, "ring sizes");
 };
 
@@ -921,7 +922,7 @@ cudaError_t launch_sweep_step(int k, int rows, int tail_rows, int flux_storage, 
   return e;
 }
 
-int batch_sweep_columns() { return kSweepCols - 2 * kSweepHaloX(kBatchSweepK); }
+int batch_sweep_columns() { return sweep_strip_columns(kBatchSweepK); }
 
 cudaError_t batch_sweep_warps(int flux_storage, int* warps, int* sms) {
   long long ctas = 0;
