@@ -238,6 +238,20 @@ int chosen_variant(const tws_grid* g) {
   return step_variant_for(k, g->flux_storage, g->W, g->H);
 }
 
+// Whether the last four steps of a call that the library gives to the three-step
+// sweep go as two and two in tiles, not as three and one (us for 4 steps with one
+// disk, three and one against two and two: 2720^2 181 and 154, 3500^2 266 and 249,
+// 4096^2 343 and 333, 5000^2 494 and 494, 8192^2 1217 and 1291; FP16 4400^2 388 and
+// 353, 6000^2 669 and 643, 8192^2 1175 and 1176).  Not where the tiles reach far over
+// the grid's border (200000 x 40: 199 and 265).  The launches are two either way.
+bool last_four_as_two_twos(const tws_grid* g) {
+  if (g->variant >= 0 || g->steps_per_launch != 0 || tuned_lookup(g).variant >= 0) return false;
+  const long long W = g->W, H = g->H, cells = W * H;
+  const long long tiled = (W + 31) / 32 * 32 * ((H + 31) / 32 * 32);
+  return 10 * tiled <= 11 * cells &&
+         cells <= (g->flux_storage == TWS_FLUX_F16 ? 48LL << 20 : 16LL << 20);
+}
+
 // Calls shorter than this keep the tiled kernels when the resident kernel
 // was chosen by the autotuner (whose trials are long calls): one resident
 // launch loads and stores the whole state, which a step or two cannot repay.
@@ -558,10 +572,11 @@ int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps) {
   }
   const int main_variant = chosen_variant(g);
   const int kmax = step_variant(main_variant).k;
+  const bool two_and_two = kmax == 3 && last_four_as_two_twos(g);
   int left = nsteps;
   std::string why;
   while (left > 0) {
-    const int k = std::min(kmax, left);
+    const int k = two_and_two && left == 4 ? 2 : std::min(kmax, left);
     // the remainder of a chain that is not a multiple of K runs shallower
     const int variant = k == kmax ? main_variant : step_variant_for(k, g->flux_storage, g->W, g->H);
     VariantMaps* m = nullptr;
