@@ -30,6 +30,10 @@ TWS_API int tws_test_drop_tile_loads(tws_grid* grid, int drop);
  * other values. */
 TWS_API int tws_test_refuse_mesh(tws_grid* grid, int refuse);
 
+/* The packed division of the step kernels, q[i] = d[i] / t[i] for device arrays of
+ * n floats (n even), on `stream` (NULL: the legacy default).  Asynchronous. */
+TWS_API int tws_test_divide(const float* d, const float* t, float* q, long long n, void* stream);
+
 /* Bytes of the mesh kernel's workspace on the current device now (0: no grid
  * holds one). */
 TWS_API size_t tws_test_mesh_workspace(void);

@@ -117,6 +117,7 @@ def _declare(L):
         "tws_test_drop_tile_loads": ([vp, i], i),
         "tws_test_refuse_mesh": ([vp, i], i),
         "tws_test_mesh_workspace": ([], C.c_size_t),
+        "tws_test_divide": ([vp, vp, vp, C.c_longlong, vp], i),
         "tws_autotune": ([vp, i, vp], i),
         "tws_resident_fits": ([i, i, i], i),
         "tws_set_resident": ([vp, i], i),

@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "tws_device.cuh"
+#include "tws_pair.cuh"
 #include "tws_internal.h"
 
 namespace tws {
@@ -670,4 +671,31 @@ extern "C" TWS_API int tws_volume_noalloc(const float* depth, int width, int hei
     if (e == cudaSuccess) tws::count_launch(1);
   }
   return e == cudaSuccess ? TWS_OK : TWS_ERR_CUDA;
+}
+
+namespace tws {
+namespace {
+
+// The packed division alone, for the tests.
+__global__ void divide_kernel(const float2* __restrict__ d, const float2* __restrict__ t,
+                              float2* __restrict__ q, long long pairs) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pairs) return;
+  const float2 dv = d[i], tv = t[i];
+  q[i] = un(div2(pk(dv.x, dv.y), pk(tv.x, tv.y), pk(-tv.x, -tv.y)));
+}
+
+}  // namespace
+}  // namespace tws
+
+extern "C" TWS_API int tws_test_divide(const float* d, const float* t, float* q, long long n,
+                                       void* stream) {
+  if (!d || !t || !q || n < 2 || n % 2 != 0 || n > 1LL << 32) return TWS_ERR_INVALID;
+  for (const void* p : {(const void*)d, (const void*)t, (const void*)q})
+    if (reinterpret_cast<uintptr_t>(p) % 8 != 0) return TWS_ERR_INVALID;
+  const long long pairs = n / 2;
+  tws::divide_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const float2*>(d), reinterpret_cast<const float2*>(t),
+      reinterpret_cast<float2*>(q), pairs);
+  return cudaGetLastError() == cudaSuccess ? TWS_OK : TWS_ERR_CUDA;
 }

@@ -46,9 +46,9 @@ __device__ __forceinline__ pair_t max0p(pair_t v) {
 // [kDivMinD, t): nothing on the way then overflows or leaves the normal range.
 // Markstein's division (IBM J. Res. Dev. 34, 1990): a reciprocal refined to
 // its correct rounding with one Newton step in fused arithmetic, a quotient
-// within an ulp, and the exact remainder's correction.  Against the
-// correctly rounded quotient: no difference in 1e11 random and structured
-// pairs of that range, nor in the pairs closest to a rounding boundary.
+// within an ulp, and the exact remainder's correction.  The tests compare it with
+// the correctly rounded quotient over that range, at its limits and for the
+// quotients closest to a rounding boundary (tests/test_division_gpu.py).
 // `nt` is -t.
 constexpr float kDivMinD = 0x1p-100f, kDivMaxT = 0x1p20f;
 __device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
