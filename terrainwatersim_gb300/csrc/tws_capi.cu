@@ -212,8 +212,10 @@ struct Tuned {
 };
 std::mutex g_tuned_mu;
 std::map<TunedKey, Tuned> g_tuned;
+std::atomic<bool> g_tuned_any{false};  // most processes tune nothing: no lock for them
 
 Tuned tuned_lookup(const tws_grid* g) {
+  if (!g_tuned_any.load(std::memory_order_acquire)) return Tuned{};
   std::lock_guard<std::mutex> lk(g_tuned_mu);
   auto it = g_tuned.find(TunedKey{g->W, g->H, g->flux_storage});
   return it == g_tuned.end() ? Tuned{} : it->second;
@@ -387,25 +389,34 @@ cudaError_t mesh_record(MeshStream* self, cudaStream_t s) {
   return e;
 }
 
-// Gives the inboxes back once the work that may use them is done, without making a
-// stream of the caller's wait for it.
-void mesh_free_inbox(MeshSpace* m, int device) {
+// Gives the inboxes back once the work that may use them is done: in the order of
+// stream `s`, or, where other streams' work is still under way, on a stream that
+// waits for it, so that none of the caller's does.
+void mesh_free_inbox(MeshSpace* m, int device, cudaStream_t s) {
   if (!m->inbox) return;
-  int current = device;
-  cudaGetDevice(&current);
-  if (current != device) cudaSetDevice(device);
-  cudaStream_t t = nullptr;
-  bool ok = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) == cudaSuccess;
-  for (MeshStream& e : m->streams)
-    if (mesh_still_busy(e)) ok = ok && cudaStreamWaitEvent(t, e.last, 0) == cudaSuccess;
-  if (ok) {
-    cudaFreeAsync(m->inbox, t);
+  unsigned long long id = 0;
+  const bool known = cudaStreamGetId(s, &id) == cudaSuccess;
+  bool others = !known;
+  for (MeshStream& e : m->streams) others = others || (e.id != id && mesh_still_busy(e));
+  if (!others) {
+    cudaFreeAsync(m->inbox, s);
   } else {
-    cudaGetLastError();
-    cudaFree(m->inbox);  // (waits for the device)
+    int current = device;
+    cudaGetDevice(&current);
+    if (current != device) cudaSetDevice(device);
+    cudaStream_t t = nullptr;
+    bool ok = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) == cudaSuccess;
+    for (MeshStream& e : m->streams)
+      if (mesh_still_busy(e)) ok = ok && cudaStreamWaitEvent(t, e.last, 0) == cudaSuccess;
+    if (ok) {
+      cudaFreeAsync(m->inbox, t);
+    } else {
+      cudaGetLastError();
+      cudaFree(m->inbox);  // (waits for the device)
+    }
+    if (t) cudaStreamDestroy(t);
+    if (current != device) cudaSetDevice(current);
   }
-  if (t) cudaStreamDestroy(t);
-  if (current != device) cudaSetDevice(current);
   m->inbox = nullptr;
   m->bytes = 0;
 }
@@ -429,7 +440,7 @@ cudaError_t mesh_hold(int device, size_t bytes, cudaStream_t s) {
       cudaFreeAsync(p, s);
       return e;
     }
-    mesh_free_inbox(m, device);
+    mesh_free_inbox(m, device, s);
     m->inbox = p;
     m->bytes = bytes;
     m->epoch = m->begun = 0;
@@ -438,12 +449,12 @@ cudaError_t mesh_hold(int device, size_t bytes, cudaStream_t s) {
   return cudaSuccess;
 }
 
-void mesh_release(int device) {
+void mesh_release(int device, cudaStream_t s) {
   MeshSpace* m = mesh_space(device);
   if (!m) return;
   std::lock_guard<std::mutex> lk(m->mu);
   if (--m->users > 0) return;
-  mesh_free_inbox(m, device);
+  mesh_free_inbox(m, device, s);
   for (MeshStream& e : m->streams) cudaEventDestroy(e.last);
   m->streams.clear();
 }
@@ -530,22 +541,27 @@ int enqueue_mesh_steps(tws_grid* g, const MeshShape& shape, const StepArgs& a, i
   return TWS_OK;
 }
 
-int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps);
+int enqueue_variant_steps(tws_grid* g, StepArgs& a, int nsteps);
 
 int enqueue_steps(tws_grid* g, int nsteps) {
-  const StepArgs a = make_step_args(g);
+  StepArgs a = make_step_args(g);
   // A graph's launches read and write the buffers that they were captured with.
   // The state changes buffers with every launch, once for a mesh call of any
   // length: from a grid's first captured call on, mesh calls between replays
   // would leave the state where the graph does not look for it.  (Nor can a capture
   // record the events that tell of other streams' work.)
-  if (g->mesh_user && !g->captured) {
+  bool mesh_open = g->mesh_user && !g->captured;
+  if (mesh_open) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    g->captured = cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess ||
-                  cap != cudaStreamCaptureStatusNone;
-    if (g->captured) cudaGetLastError();
+    if (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess) {
+      cudaGetLastError();
+      mesh_open = false;
+    } else if (cap != cudaStreamCaptureStatusNone) {
+      g->captured = true;
+      mesh_open = false;
+    }
   }
-  const MeshShape* mesh = mesh_for(g, nsteps);
+  const MeshShape* mesh = mesh_open ? mesh_for(g, nsteps) : nullptr;
   int left = nsteps;
   int rc = mesh ? enqueue_mesh_steps(g, *mesh, a, nsteps, &left) : TWS_OK;
   if (rc != TWS_OK || left == 0) return rc;
@@ -555,7 +571,7 @@ int enqueue_steps(tws_grid* g, int nsteps) {
 }
 
 // Steps by the resident kernel or the variants.
-int enqueue_variant_steps(tws_grid* g, StepArgs a, int nsteps) {
+int enqueue_variant_steps(tws_grid* g, StepArgs& a, int nsteps) {
   if (const int ctas = resident_ctas(g, nsteps)) {
     for (int left = nsteps; left > 0;) {
       const int n = std::min(left, kResidentMaxSteps);
@@ -773,7 +789,7 @@ TWS_API int tws_destroy(tws_grid* g) {
     if (ev) cudaEventDestroy(ev);
   if (g->io_up) cudaStreamDestroy(g->io_up);
   if (g->io_down) cudaStreamDestroy(g->io_down);
-  if (g->mesh_user) mesh_release(g->device);
+  if (g->mesh_user) mesh_release(g->device, g->stream);
   if (g->slab) cudaFreeAsync(g->slab, g->stream);
   if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
   delete g;
@@ -1096,6 +1112,7 @@ TWS_API int tws_autotune(tws_grid* g, int trial_steps, int* chosen) {
     t.variant = best;
     t.resident = resident_best;
     if (mesh_tried) t.mesh = mesh_best ? MeshTrial::kWon : MeshTrial::kLost;
+    g_tuned_any.store(true, std::memory_order_release);
   }
   if (chosen) *chosen = choice;
   return TWS_OK;
