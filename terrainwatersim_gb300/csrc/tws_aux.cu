@@ -121,11 +121,52 @@ struct DepthSum {
   }
 };
 
-// VEC: rows start on 16-byte boundaries, four depths per load.
+// VEC: rows start on 16-byte boundaries, four depths per load.  A block takes its
+// rows one by one; narrow ones (`lanes` below the block's threads, a power of two with
+// a thread for each load of a row) several side by side and four of each thread's in
+// flight, for the same sum.
 template <bool VEC>
 __global__ void __launch_bounds__(kVolThreads)
-    volume_rows_kernel(const float* __restrict__ d, int W, int H, int pitch, double* partials) {
+    volume_rows_kernel(const float* __restrict__ d, int W, int H, int pitch, int lanes,
+                       double* partials) {
   DepthSum sum;
+  if (lanes < kVolThreads) {
+    constexpr int U = 4, N = VEC ? 4 : 1;
+    const int x = threadIdx.x % lanes * N, n = min(N, W - x);  // this thread's columns
+    const long long step = (long long)gridDim.x * (kVolThreads / lanes);
+    long long y = blockIdx.x + (long long)gridDim.x * (threadIdx.x / lanes);
+    for (; n > 0 && y < H; y += U * step) {
+      float v[U][N];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long r = y + u * step;
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[u][k] = 0.0f;
+        if (r >= H) continue;
+        const float* p = d + (size_t)r * pitch + x;
+        if constexpr (VEC) {
+          if (n == 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+            v[u][0] = q.x, v[u][1] = q.y, v[u][2] = q.z, v[u][3] = q.w;
+          } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              if (k < n) v[u][k] = __ldg(p + k);
+          }
+        } else {
+          v[u][0] = __ldg(p);
+        }
+      }
+      sum.reserve(U * N);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < N; ++k) sum.add(v[u][k]);
+    }
+    const double s = sum.block_total();
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    return;
+  }
   for (int y = blockIdx.x; y < H; y += gridDim.x) {
     const float* row = d + (size_t)y * pitch;
     int x0 = 0;
@@ -154,10 +195,21 @@ __global__ void __launch_bounds__(kVolThreads)
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
-using VolumeRowsFn = void (*)(const float*, int, int, int, double*);
+using VolumeRowsFn = void (*)(const float*, int, int, int, int, double*);
+bool volume_in_quads(const float* d, int pitch) {
+  return reinterpret_cast<uintptr_t>(d) % 16 == 0 && pitch % 4 == 0;
+}
 VolumeRowsFn volume_rows_fn(const float* d, int pitch) {
-  return reinterpret_cast<uintptr_t>(d) % 16 == 0 && pitch % 4 == 0 ? volume_rows_kernel<true>
-                                                                    : volume_rows_kernel<false>;
+  return volume_in_quads(d, pitch) ? volume_rows_kernel<true> : volume_rows_kernel<false>;
+}
+// The threads that a row takes: the block's, or fewer where blocks have several narrow
+// rows each (tws_volume, us, side by side and one by one: 8 x 300000 39 and 287, 256 x
+// 100000 125 and 149, but 500 x 20000 76 and 64, 512 x 4096 39 and 28).
+int volume_lanes(const float* d, int W, int H, int pitch, int blocks) {
+  const int loads = volume_in_quads(d, pitch) ? (W + 3) / 4 : W;
+  int lanes = 1;
+  while (lanes < loads && lanes < kVolThreads) lanes *= 2;
+  return H > blocks && lanes <= kVolThreads / 4 ? lanes : kVolThreads;
 }
 
 __global__ void __launch_bounds__(kVolThreads)
@@ -401,7 +453,8 @@ int volume_partials_needed() { return kVolMaxBlocks; }
 cudaError_t launch_volume(const float* d, int W, int H, int pitch, double cell_area,
                           double* partials, int max_partials, double* out, cudaStream_t st) {
   const int nb = std::max(1, std::min({H, kVolMaxBlocks, max_partials}));
-  volume_rows_fn(d, pitch)<<<nb, kVolThreads, 0, st>>>(d, W, H, pitch, partials);
+  volume_rows_fn(d, pitch)<<<nb, kVolThreads, 0, st>>>(d, W, H, pitch,
+                                                       volume_lanes(d, W, H, pitch, nb), partials);
   volume_final_kernel<<<1, kVolThreads, 0, st>>>(partials, nb, cell_area, out);
   count_launch(2);
   return cudaGetLastError();
@@ -662,7 +715,7 @@ extern "C" TWS_API int tws_volume_noalloc(const float* depth, int width, int hei
   cfg.blockDim = dim3(tws::kVolThreads);
   cfg.stream = st;
   cudaError_t e = cudaLaunchKernelEx(&cfg, tws::volume_rows_fn(depth, pitch), depth, width, height,
-                                     pitch, scratch);
+                                     pitch, tws::kVolThreads, scratch);
   if (e == cudaSuccess) {
     tws::count_launch(1);
     cfg.gridDim = dim3(1);
