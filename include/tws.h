@@ -352,10 +352,10 @@ TWS_API int tws_surface(tws_grid* grid, const tws_surface_out* out);
  * `mips` (level l is floor(W/2^l) x floor(H/2^l) RGBA32F texels; every level
  * must be at least 1 x 1).  Any pointer may be NULL (mips need terrain_rgba).
  * terrain_rgba and mips must be 16-byte aligned and flowmap_rg16f 4-byte
- * aligned (TWS_ERR_INVALID otherwise).  Whole-sector stores also need
- * terrain_rgba on a 32-byte and flowmap_rg16f on a 16-byte boundary and a width
- * that is a multiple of 4; otherwise texels go out one by one (without mips: one
- * cell per thread), with the same results.  Asynchronous on the
+ * aligned (TWS_ERR_INVALID otherwise).  The fast paths also need flowmap_rg16f on
+ * a 16-byte boundary and a width that is a multiple of 4 (the fastest, with mips,
+ * terrain_rgba on a 32-byte boundary); otherwise texels go out one by one (without
+ * mips: one cell per thread), with the same results.  Asynchronous on the
  * grid's stream. */
 TWS_API int tws_export_textures(tws_grid* grid, float* terrain_rgba, uint16_t* flowmap_rg16f,
                                 int mip_levels, float* mips);

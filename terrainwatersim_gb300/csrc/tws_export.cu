@@ -311,11 +311,14 @@ struct MipLevels {
   int n;                           // levels written, 1 .. kMipFused
 };
 
-// Q: level-1 texels per block side, 32 or 16 (blocks of 64 or 32 cells).  WHOLE: the
-// width is a multiple of 4, terrain_rgba lies on a 32-byte and the flow map on a
-// 16-byte boundary: a thread's four texels go out in whole sectors.  Else any
-// width and alignment, texel by texel.
-template <int Q, bool WHOLE>
+// How a thread's four texels go out: one by one (any width and alignment); side by
+// side (a width of whole quads, the flow map's four in one store); in whole sectors
+// (terrain_rgba on a 32-byte boundary besides).  4096^2 with one level, us: whole
+// sectors 101, side by side 115, one by one 136.
+enum { kTexels = 0, kQuads = 1, kSectors = 2 };
+
+// Q: level-1 texels per block side, 32 or 16 (blocks of 64 or 32 cells).
+template <int Q, int STORE>
 __global__ void __launch_bounds__(8 * Q)
     export_mips_kernel4(const float* __restrict__ b, const float* __restrict__ d,
                         const float2* __restrict__ v, int W, int H, int pitch,
@@ -345,9 +348,12 @@ __global__ void __launch_bounds__(8 * Q)
         t[r][1] = make_float4(b4.y, 0.3f, 0.3f, d4.y);
         t[r][2] = make_float4(b4.z, 0.3f, 0.3f, d4.z);
         t[r][3] = make_float4(b4.w, 0.3f, 0.3f, d4.w);
-        if constexpr (WHOLE) {
+        if constexpr (STORE == kSectors) {
           store_texels(rgba + out, t[r][0], t[r][1]);
           store_texels(rgba + out + 2, t[r][2], t[r][3]);
+        } else if constexpr (STORE == kQuads) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) rgba[out + k] = t[r][k];
         } else {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -358,7 +364,7 @@ __global__ void __launch_bounds__(8 * Q)
           const float4 v23 = *reinterpret_cast<const float4*>(v + i + 2);
           const __half2 h[4] = {__floats2half2_rn(v01.x, v01.y), __floats2half2_rn(v01.z, v01.w),
                                 __floats2half2_rn(v23.x, v23.y), __floats2half2_rn(v23.z, v23.w)};
-          if constexpr (WHOLE) {
+          if constexpr (STORE != kTexels) {
             uint4 packed;
             packed.x = *reinterpret_cast<const uint32_t*>(&h[0]);
             packed.y = *reinterpret_cast<const uint32_t*>(&h[1]);
@@ -475,9 +481,13 @@ cudaError_t launch_export(const float* b, const float* d, const float2* v, int W
       p += (size_t)w * h;
       ++fused.n;
     }
-    const bool whole = wide && aligned(terrain_rgba, 32);
-    auto fn = small ? (whole ? export_mips_kernel4<16, true> : export_mips_kernel4<16, false>)
-                    : (whole ? export_mips_kernel4<32, true> : export_mips_kernel4<32, false>);
+    const int store = !wide ? kTexels : aligned(terrain_rgba, 32) ? kSectors : kQuads;
+    auto fn = small ? (store == kSectors ? export_mips_kernel4<16, kSectors>
+                       : store == kQuads ? export_mips_kernel4<16, kQuads>
+                                         : export_mips_kernel4<16, kTexels>)
+                    : (store == kSectors ? export_mips_kernel4<32, kSectors>
+                       : store == kQuads ? export_mips_kernel4<32, kQuads>
+                                         : export_mips_kernel4<32, kTexels>);
     const int side = small ? 32 : 64;
     launch(fn, dim3((W + side - 1) / side, (H + side - 1) / side), dim3(small ? 128 : 256), s, b, d,
            v, W, H, pitch, reinterpret_cast<float4*>(terrain_rgba),
