@@ -1366,10 +1366,12 @@ int step_variant_for(int k, int /*flux_storage*/, int W, int H) {
   // One step on a smaller grid takes 32x16 tiles, twice as many CTAs (us per
   // launch, FP32, against 32x32): 256^2 4.1 (5.8), 512^2 5.1 (6.4), 1024^2 10.6
   // (11.1), 2048^2 39.5 (39.9).  What counts is the number of tiles: 8 x 500000, of
-  // as few cells as 2048^2 but four times the tiles, takes 109 (93).
+  // as few cells as 2048^2 but four times the tiles, takes 109 (93).  So does a
+  // height of which 32-row tiles waste more: 300000 x 8 30 (48).
   const long long tiles = (long long)((W + 31) / 32) * ((H + 31) / 32);
+  const bool flat = 4 * ((H + 15) / 16 * 16) <= 3 * ((H + 31) / 32 * 32);
   switch (k) {
-    case 1: return tiles < kSmallStepTiles ? 5 : 0;
+    case 1: return tiles < kSmallStepTiles || flat ? 5 : 0;
     case 2: return 16;
     case 3: return 18;
     case 4: return 20;

@@ -54,3 +54,13 @@ def test_default_as_the_plain_kernel(tws, W):
             out.append(g.download())
     for name, x, y in zip(("depth", "flux", "flow map"), *out):
         assert_bitexact(x, y, name)
+
+
+@pytest.mark.parametrize("W,H,tile_y", [(300000, 8, 16), (300000, 16, 16), (200000, 48, 16),
+                                        (200000, 24, 32), (200000, 64, 32)])
+def test_one_step_tile_of_flat_grids(tws, W, H, tile_y):
+    """16 rows a tile where 32 would waste a third more."""
+    with tws.Grid(W, H) as g:
+        g.set_steps_per_launch(1)
+        v = tws.variants()[g.current_variant()]
+    assert (v[0], v[1], v[2]) == (1, 32, tile_y)
