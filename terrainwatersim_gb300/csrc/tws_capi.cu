@@ -1771,14 +1771,16 @@ bool sweep_is_faster(const tws_batch* b, const std::vector<int>& steps) {
   const long long least =
       b->flux_storage == TWS_FLUX_F16 ? kBatchSweepF16Cells : kBatchSweepCells;
   long long cells = 0, strips = 0, tiles = 0;
+  for (size_t i = 0; i < steps.size(); ++i)
+    if (steps[i] >= kBatchSweepK) cells += (long long)b->grids[i]->W * b->grids[i]->H;
+  if (cells < least) return false;
   for (size_t i = 0; i < steps.size(); ++i) {
     if (steps[i] < kBatchSweepK) continue;
     const long long W = b->grids[i]->W, H = b->grids[i]->H;
-    cells += W * H;
     strips += (W + cols - 1) / cols * cols * H;
     tiles += (W + 31) / 32 * 32 * ((H + 31) / 32 * 32);
   }
-  if (cells < least || 20 * strips > 23 * tiles) return false;
+  if (20 * strips > 23 * tiles) return false;
 
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(b->stream, &cap) != cudaSuccess ||
@@ -1828,6 +1830,7 @@ int batch_advance(tws_batch* b, const std::vector<int>& steps) {
   // kernel.  Where three steps a launch leave one over, the last four go as two
   // and two.
   std::vector<int> left(n), two(n, 0), one(n, 0), launches(n);
+  bool any_left = false, any_two = false, any_one = false;
   for (int i = 0; i < n; ++i) {
     left[i] = steps[i] / k;
     const int rest = steps[i] % k;
@@ -1839,16 +1842,19 @@ int batch_advance(tws_batch* b, const std::vector<int>& steps) {
     } else {
       one[i] = rest;
     }
+    any_left |= left[i] > 0;
+    any_two |= two[i] > 0;
+    any_one |= one[i] > 0;
   }
-  for (;;) {
+  while (any_left) {
     for (int i = 0; i < n; ++i) launches[i] = std::min(left[i], per_chain);
-    if (*std::max_element(launches.begin(), launches.end()) <= 0) break;
     const int rc = run_chain(b, variant, launches);
     if (rc != TWS_OK) return rc;
-    for (int i = 0; i < n; ++i) left[i] -= launches[i];
+    any_left = false;
+    for (int i = 0; i < n; ++i) any_left |= (left[i] -= launches[i]) > 0;
   }
-  int rc = run_chain(b, batch_variant_default(), two);
-  if (rc == TWS_OK) rc = run_chain(b, kBatchOneStepVariant, one);
+  int rc = any_two ? run_chain(b, batch_variant_default(), two) : TWS_OK;
+  if (rc == TWS_OK && any_one) rc = run_chain(b, kBatchOneStepVariant, one);
   return rc;
 }
 
