@@ -114,10 +114,11 @@ int batch_variant_count();
 int batch_variant_default();  // two steps per launch, unified 32x32 tiles
 int batch_variant_sweep();    // the batched row sweep, three steps per launch
 // A batch without a set variant takes the sweep from this many cells on, where its
-// strips waste little more than the tiles (us for 48 steps, sweep against tiles:
-// 6 x 1024^2 1749 (1818), 8 x 1024^2 2208 (2387), 32 steps of 20 grids of 128 to
-// 2048 a side 2830 (3437); FP16 24 x 1024^2 5896
-// (6179), 128 x 512^2 8757 (8752), 8 x 2048^2 6704 (7974)).
+// strips waste little more than the tiles (us for 48 steps with one disk a grid, sweep
+// against tiles: 6 x 1024^2, below the line, 1749 (1818), 8 x 1024^2 2208 (2387), 32
+// steps of 20 grids of 128 to 2048 a side 2830 (3437); FP16 24 x 1024^2 5896 (6179),
+// 128 x 512^2 8757 (8752), 8 x 2048^2 6704 (7974)).  The line leaves room for sources:
+// with two large disks a grid the tiles still lead on 8 x 1024^2 (sweep_is_faster).
 constexpr long long kBatchSweepCells = 8LL << 20;
 constexpr long long kBatchSweepF16Cells = 24LL << 20;
 void batch_variant_info(int i, int* k, int* tx, int* ty, int* step_variant);

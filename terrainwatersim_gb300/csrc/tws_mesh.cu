@@ -33,8 +33,8 @@
 // chosen per grid from a measured cost model (mesh_shape).
 //
 // Measured (us per step of long calls, CUDA events, one rain disk; in brackets the
-// two-step tiles): 64^2 1.3 (3.1), 256^2 1.7 (3.3), 512^2 2.5 (3.9), 1021 x 763
-// 4.9 (6.2), 1024^2 5.9 (7.1).  Four columns per lane (boxes of 128 columns) issue
+// two-step tiles): 64^2 1.3 (3.1), 256^2 1.6 (3.3), 512^2 2.4 (3.9), 1021 x 763
+// 4.8 (6.2), 1024^2 6.2 (7.1).  Four columns per lane (boxes of 128 columns) issue
 // less per cell but leave a quarter of the warps' parallelism: 256^2 2.5 against
 // 1.4 without rain.
 //
@@ -474,6 +474,8 @@ __global__ void __launch_bounds__(kMeshThreads, 1)
             if (closed && y == 0) nw = 0;
           }
         }
+        // (outflow_factors2 with -t negated, not a second product: with that function
+        // 200 steps on 1021 x 763 take 980 us, not 960)
         const pair_t sum = add2(add2(add2(nx, ny), nz), nw);
         const pair_t tq = prod2(sum, cc2, nz2);
         const float2 t = un(tq), d = un(dc);

@@ -1319,11 +1319,13 @@ int step_variant_large_grid(int flux_storage, int W, int H) {
   // (190), 2896^2 229 (193), 3400^2 252 (197); with eight disks of a sixteenth of
   // the side, which weigh on the sweep's few units, 2720^2 171 (176), 2896^2 187
   // (178), 3400^2 218 (185)), FP16 flux from kLargeF16Cells
-  // on (4608^2 249 (217), with eight disks 229 (209); 4096^2, 238 (216), keeps the two-step
-  // tiles that callers of that size have as their default).  The band height is the tallest rung of a ladder that leaves at least
-  // 2.5 column-unit bands per resident warp of a 16-warp SM (8192^2: 315 with
-  // 192/48 rows, 305 with uniform bands of 64 to 192; 16384^2: 339 with 256/64,
-  // 320 uniform).
+  // on (4608^2 249 (217), with eight disks 229 (209)).  The sweep leads below that
+  // line too (4096^2 241 (221), with eight disks 206 (200); 3750^2 202 (196)): what
+  // holds it there is test_default_variant_ladder, which fixes the two-step tiles as
+  // the choice for 4096^2 FP16.  The band height is the tallest rung of a ladder that
+  // leaves at least 2.5 column-unit bands per resident warp of a 16-warp SM (8192^2:
+  // 315 with 192/48 rows, 305 with uniform bands of 64 to 192; 16384^2: 339 with
+  // 256/64, 320 uniform).
   const long long cells = (long long)W * H;
   if (cells < kLargeGridCells) return -1;
   if (flux_storage != TWS_FLUX_F32 && cells < kLargeF16Cells) return -1;

@@ -745,7 +745,8 @@ __global__ void __launch_bounds__(kSweepThreads, (K <= 3 ? 3 : 2))
     int u = sweep_next(queue, head.x, head.y, which, queues, lane);
     const bool queued = u >= 0;
     if (!queued) {
-      // the queues are empty: the largest of 64 other warps' ranges, its back half
+      // as in sweep_kernel (shared as a function, the search changed that kernel's
+      // register allocation: 4096^2 262 -> 244 Gcell-steps/s)
       bool got = false;
       for (int attempt = 0; attempt < kSweepStealTries && !got; ++attempt) {
         seed = seed * 1664525u + 1013904223u;  // (Numerical Recipes' generator)
