@@ -673,8 +673,24 @@ TWS_API int tws_params_reference(float steps_per_second, float flow_damping,
 
 }  // extern "C"
 
+// The mesh kernel's workspace, where it fits this grid (whatever its sources).
+void tws::take_mesh_workspace(tws_grid* g) {
+  if (g->mesh_user) return;
+  size_t inbox = 0;
+  for (int brushes = 0; brushes <= TWS_MAX_SOURCES; ++brushes) {
+    MeshShape shape;
+    if (mesh_shape(g->W, g->H, brushes, &shape)) inbox = std::max(inbox, mesh_inbox_bytes(shape));
+  }
+  if (inbox == 0) return;
+  if (mesh_hold(g->device, inbox, g->stream) != cudaSuccess) {
+    cudaGetLastError();  // the step kernels run without it
+  } else {
+    g->mesh_user = true;
+  }
+}
+
 int tws::create_grid(int width, int height, const tws_sim_params* params, int flux_storage,
-                     void* stream, tws_grid** out) {
+                     void* stream, bool mesh, tws_grid** out) {
   if (!out) return TWS_ERR_INVALID;
   *out = nullptr;
   // (height <= 2^19 keeps the tile rows of a one-CTA-per-tile launch within
@@ -738,34 +754,17 @@ int tws::create_grid(int width, int height, const tws_sim_params* params, int fl
   // padding cell of odd-width rows and relies on it staying zero): the front of
   // the allocation, in one fill.
   cudaMemsetAsync(g->slab, 0, at.zeroed, g->stream);
+  if (mesh) take_mesh_workspace(g);
   if (cudaStreamSynchronize(g->stream) != cudaSuccess) return bail(TWS_ERR_CUDA);
   *out = g;
   return TWS_OK;
-}
-
-// The mesh kernel's workspace, where it fits this grid (whatever its sources).
-void tws::take_mesh_workspace(tws_grid* g) {
-  if (g->mesh_user) return;
-  size_t inbox = 0;
-  for (int brushes = 0; brushes <= TWS_MAX_SOURCES; ++brushes) {
-    MeshShape shape;
-    if (mesh_shape(g->W, g->H, brushes, &shape)) inbox = std::max(inbox, mesh_inbox_bytes(shape));
-  }
-  if (inbox == 0) return;
-  if (mesh_hold(g->device, inbox, g->stream) != cudaSuccess) {
-    cudaGetLastError();  // the step kernels run without it
-  } else {
-    g->mesh_user = true;
-  }
 }
 
 extern "C" {
 
 TWS_API int tws_create(int width, int height, const tws_sim_params* params, int flux_storage,
                        void* stream, tws_grid** out) {
-  const int rc = create_grid(width, height, params, flux_storage, stream, out);
-  if (rc == TWS_OK) take_mesh_workspace(*out);
-  return rc;
+  return create_grid(width, height, params, flux_storage, stream, true, out);
 }
 
 TWS_API size_t tws_test_mesh_workspace(void) {

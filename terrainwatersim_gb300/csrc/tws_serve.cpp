@@ -71,7 +71,7 @@ bool valid_request(const tws_request& r) {
 // Create the grid of a request and queue its scene on the grid's stream.
 int make_grid(const tws_server_config& cfg, const tws_request& r, tws_grid** out) {
   tws_grid* g = nullptr;
-  int rc = tws::create_grid(r.width, r.height, &r.params, cfg.flux_storage, nullptr, &g);
+  int rc = tws::create_grid(r.width, r.height, &r.params, cfg.flux_storage, nullptr, false, &g);
   if (rc != TWS_OK) return rc;
   rc = tws_generate_scene(g, r.seed, r.height_scale, r.fill);
   if (rc == TWS_OK) rc = tws_set_sources(g, r.sources, r.nsources);
