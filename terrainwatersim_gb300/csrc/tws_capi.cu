@@ -455,8 +455,15 @@ void mesh_release(int device, cudaStream_t s) {
   std::lock_guard<std::mutex> lk(m->mu);
   if (--m->users > 0) return;
   mesh_free_inbox(m, device, s);
-  for (MeshStream& e : m->streams) cudaEventDestroy(e.last);
-  m->streams.clear();
+  // (a destroyed grid's launch may still run, and the next grid's must not beside it)
+  std::vector<MeshStream> busy;
+  for (MeshStream& e : m->streams) {
+    if (mesh_still_busy(e))
+      busy.push_back(e);
+    else
+      cudaEventDestroy(e.last);
+  }
+  m->streams.swap(busy);
 }
 
 // One launch of `n` steps, unless another stream's work is in its way or it is

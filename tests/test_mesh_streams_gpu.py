@@ -127,6 +127,37 @@ def test_last_grid_destroyed_with_work_queued(tws, oracle):
     assert event.query()
 
 
+def test_destroyed_grids_work_still_counts(tws, oracle):
+    """The last grid is gone, its launch is not: a new grid's steps go beside it as
+    tiles, and as the mesh kernel once it has run."""
+    import torch
+    stream = torch.cuda.Stream()
+    for W, H in ((200, 150), (300, 200)):  # (the kernels are loaded)
+        with tws.Grid(W, H, params(tws)) as warm:
+            warm.step(24)
+            warm.set_steps_per_launch(2)
+            warm.step(4)
+            warm.sync()
+    g = tws.Grid(300, 200, params(tws), stream=stream.cuda_stream)
+    g.upload(*state(300, 200))
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(SLEEP)
+    g.step(400)
+    g.close()
+    event = torch.cuda.Event()
+    event.record(stream)
+    with tws.Grid(200, 150, params(tws)) as g:
+        data = state(200, 150)
+        g.upload(*data)
+        n = launches(tws, g, 24)
+        g.sync()
+        assert not event.query()
+        assert n == 12
+        stream.synchronize()
+        assert launches(tws, g, 24) == 1
+        check(tws, oracle, g, data, 48)
+
+
 def test_many_streams_in_turn(tws, oracle):
     """More streams than entries stay, stepped in turn without waiting."""
     import torch
